@@ -41,6 +41,7 @@ def _sources():
     return [
         ("kernels_particles.cu", common_nv + ["--fmad=false"]),
         ("kernels_pcg.cu", common_nv),
+        ("kernels_pcg_resident.cu", common_nv),
         ("kernels_mixed.cu", common_nv),
         ("noalloc.cu", common_nv),
         ("kernels_adjoint.cu", common_nv + ["--fmad=false"]),

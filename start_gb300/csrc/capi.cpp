@@ -16,6 +16,7 @@
 #include <string>
 #include <vector>
 
+#include "pcg_resident.h"
 #include "spg_internal.h"
 
 using namespace spg;
@@ -99,7 +100,7 @@ struct spg_handle {
     // scalars go to a pinned record, read when the run ends.
     bool defer_solves = false;
     PcgScalars *solve_rec = nullptr;          // pinned, kSolveRecs records
-    uint8_t solve_kind[kSolveRecs] = {};      // 0: do_solve64, 1: do_solve_mixed_amg
+    uint8_t solve_kind[kSolveRecs] = {};      // 0: do_solve64, 1: do_solve_mixed_amg, 2: resident Jacobi PCG
     int n_solve_rec = 0;
     bool deferred_capped = false;             // a drained record had hit max_iter
     bool occ_fresh = false;                   // no particle has moved since the deposit listed the tets
@@ -114,6 +115,12 @@ struct spg_handle {
     PcgScalars *sc = nullptr;
     int pcg_blocks = 1;
     PcgGrid grid64, grid32;
+    // Jacobi PCG of a system that fits on the chip, one launch per solve
+    // (blocks == 0: it does not fit, or AMG is selected)
+    ResidentPlan resident;
+    double2 *res_zp = nullptr;        // two arrays of n_nodes pairs
+    double *res_partials = nullptr;
+    unsigned int *res_arrived = nullptr;
     // PCG iterations are replayed as a CUDA graph of kPcgChunk iterations
     // (3 kernels each); converged solves turn the remaining kernels into no-ops.
     cudaGraphExec_t pcg_graph = nullptr;
@@ -941,10 +948,11 @@ int finish_solve(spg_handle *h, int32_t iters, double rr, double bb, bool capped
     return record_solve(h, iters, rr, bb, capped);
 }
 
-// Launch count and profiled bytes of a while-graph solve (kind 0: do_solve64,
-// 1: do_solve_mixed_amg) that ran hs.iters iterations.
+// Launch count and profiled bytes of a device-controlled solve (kind 0: the
+// while graph of do_solve64, 1: of do_solve_mixed_amg, 2: the resident Jacobi
+// PCG, one launch) that ran hs.iters iterations.
 void account_while_solve(spg_handle *h, int kind, const PcgScalars &hs) {
-    h->launches += int64_t(hs.iters + 1) * (pcg_iter_launches(h) + 1);
+    h->launches += kind == 2 ? 1 : int64_t(hs.iters + 1) * (pcg_iter_launches(h) + 1);
     if (!h->prof) return;
     const double n = double(h->n_nodes), nnz = double(h->nnz_kept);
     h->pcg_iters_prof += hs.iters;
@@ -956,6 +964,31 @@ void account_while_solve(spg_handle *h, int kind, const PcgScalars &hs) {
         h->pcg_bytes += double(hs.iters) * (12.0 * nnz + 4.0 * (n + 1.0) + 72.0 * n);
 }
 
+int solver_timed_out(spg_handle *h) {
+    return fail(h, SPG_E_CUDA, "PCG: a barrier of the resident solver gave up");
+}
+
+// The resident Jacobi PCG of A x = b on the handle's stream.
+int launch_resident(spg_handle *h, const double *b, double *x) {
+    ResidentArgs a;
+    a.n = int(h->n_nodes);
+    a.slice_ptr = h->slice_ptr;
+    a.col = h->scol;
+    a.val = h->sval;
+    a.inv_diag = h->inv_diag;
+    a.b = b;
+    a.x = x;
+    a.zp[0] = h->res_zp;
+    a.zp[1] = h->res_zp + h->n_nodes;
+    a.partials = h->res_partials;
+    a.arrived = h->res_arrived;
+    a.sc = h->sc;
+    a.rtol2 = h->prm.cg_rtol * h->prm.cg_rtol;
+    a.max_iter = h->prm.cg_max_iter;
+    CK(launch_pcg_resident(h->resident, a, h->stream));
+    return SPG_OK;
+}
+
 // The statistics of the solves held back by the run (one synchronisation).
 int drain_solves(spg_handle *h) {
     if (h->n_solve_rec == 0) return SPG_OK;
@@ -964,6 +997,7 @@ int drain_solves(spg_handle *h) {
     h->n_solve_rec = 0;
     for (int k = 0; k < n; ++k) {
         const PcgScalars hs = h->solve_rec[k];
+        if (hs.converged == kPcgTimedOut) return solver_timed_out(h);
         account_while_solve(h, h->solve_kind[k], hs);
         if (record_solve(h, hs.iters, hs.rr, hs.bb, hs.converged == 2) == SPG_E_NOT_CONVERGED)
             h->deferred_capped = true;
@@ -1026,6 +1060,19 @@ void build_pcg_while(spg_handle *h, F iterate, cudaGraphExec_t *exec, bool *fail
 
 int do_solve64(spg_handle *h) {
     const int64_t n = h->n_nodes;
+    if (h->resident.blocks > 0) {
+        ev_begin(h, h->ev_pcg);
+        const int rc = launch_resident(h, h->b, h->phi);
+        if (rc) return rc;
+        if (h->defer_solves) return defer_solve(h, 2);
+        PcgScalars hs{};
+        CK(cudaMemcpyAsync(&hs, h->sc, sizeof(hs), cudaMemcpyDeviceToHost, h->stream));
+        CK(cudaStreamSynchronize(h->stream));
+        ev_end(h, h->ev_pcg);
+        if (hs.converged == kPcgTimedOut) return solver_timed_out(h);
+        account_while_solve(h, 2, hs);
+        return finish_solve(h, hs.iters, hs.rr, hs.bb, hs.converged == 2);
+    }
     PcgScalars init{};
     init.tol2 = (h->prm.cg_rtol * h->prm.cg_rtol);
     init.max_iter = h->prm.cg_max_iter;
@@ -1616,7 +1663,13 @@ int spg_create(const spg_mesh_desc *mesh, const spg_params *params, spg_handle *
     h->pcg_blocks = pcg_blocks(n);
     h->grid64 = pcg_grid64(n);
     h->grid32 = pcg_grid32(n);
+    if (!h->amg && !h->amg32) h->resident = resident_plan(n);
     CK(cudaGetLastError());
+    if (h->resident.blocks > 0) {
+        CK(dalloc(&h->res_zp, 2 * size_t(n)));
+        CK(dalloc(&h->res_partials, kResidentPartials));
+        CK(dalloc(&h->res_arrived, 1));
+    }
     CK(dalloc(&h->partials, 3 * size_t(h->pcg_blocks)));
     CK(dalloc(&h->sc, 1));
     CK(dalloc(&h->partials32, 3 * size_t(h->pcg_blocks)));
@@ -1665,7 +1718,7 @@ int spg_destroy(spg_handle *h) {
                     h->gE,       h->lam,      h->mu,       h->dJdg,    h->sums, h->hist.tet, h->hist.vx,
                     h->hist.vy,  h->hist.vz,  h->tri_scratch, h->ctr_scratch,
                     h->q,        h->partials, h->sc,       h->tri_count, h->ctr,      h->n_alive_dev, h->sort_scratch, h->walkq_n,
-                    h->io,       h->seg_rq,   h->seg_qn};
+                    h->io,       h->seg_rq,   h->seg_qn,   h->res_zp,  h->res_partials, h->res_arrived};
     for (void *ptr : ptrs) cudaFree(ptr);
     for (EventSeries *s : {&h->ev_step, &h->ev_dep, &h->ev_pcg, &h->ev_ef, &h->ev_sort}) ev_destroy(*s);
     for (void *ptr : h->amg_alloc) cudaFree(ptr);
@@ -2603,6 +2656,17 @@ void free_particle_set32(std::vector<DevParticles32> &v) {
 
 // Solves K x = b (b, x device vectors of n_nodes) with the FP64 PCG of spg_solve.
 int solve_into(spg_handle *h, double *b, double *x, int32_t *iters) {
+    if (h->resident.blocks > 0) {
+        const int rc = launch_resident(h, b, x);
+        if (rc) return rc;
+        PcgScalars hs{};
+        CK(cudaMemcpyAsync(&hs, h->sc, sizeof(hs), cudaMemcpyDeviceToHost, h->stream));
+        CK(cudaStreamSynchronize(h->stream));
+        if (iters) *iters = hs.iters;
+        if (hs.converged == kPcgTimedOut) return solver_timed_out(h);
+        if (hs.converged == 2) return fail(h, SPG_E_NOT_CONVERGED, "adjoint PCG did not converge");
+        return SPG_OK;
+    }
     PcgScalars init{};
     init.tol2 = h->prm.cg_rtol * h->prm.cg_rtol;
     init.max_iter = h->prm.cg_max_iter;

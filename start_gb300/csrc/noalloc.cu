@@ -18,6 +18,7 @@
 #include <mutex>
 #include <string>
 
+#include "pcg_resident.h"
 #include "spg_internal.h"
 
 namespace spg {
@@ -218,7 +219,13 @@ int na_fail(int code, const std::string &msg) {
 std::mutex g_na_mutex;
 double *g_na_ptr[64] = {nullptr};
 
-int na_scratch(double **out) {
+// Launch plan of the resident solver for the row count last solved on each device.
+struct NaPlan {
+    int64_t n = -1;
+    ResidentPlan plan;
+} g_na_plan[64];
+
+int na_scratch(double **out, int64_t n, ResidentPlan *plan) {
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return na_fail(SPG_E_NO_DEVICE, std::string("cudaGetDevice: ") + cudaGetErrorString(e));
@@ -231,7 +238,30 @@ int na_scratch(double **out) {
             return na_fail(SPG_E_CUDA, std::string("cudaGetSymbolAddress: ") + cudaGetErrorString(e));
         g_na_ptr[dev] = static_cast<double *>(ptr);
     }
+    if (g_na_plan[dev].n != n) {
+        g_na_plan[dev].plan = resident_plan(n);
+        g_na_plan[dev].n = n;
+    }
+    *plan = g_na_plan[dev].plan;
     *out = g_na_ptr[dev];
+    return SPG_OK;
+}
+
+// The outcome of a finished solve.
+int na_outcome(const PcgScalars &hs, int32_t *iters, double *relres) {
+    if (hs.flags)
+        return na_fail(SPG_E_INVALID,
+                       "spg_pcg_solve_noalloc: a row has no stored diagonal entry, or a zero or non-finite one");
+    if (hs.converged == kPcgTimedOut)
+        return na_fail(SPG_E_CUDA, "spg_pcg_solve_noalloc: a barrier of the resident solver gave up");
+    if (iters) *iters = hs.iters;
+    if (relres) *relres = hs.bb > 0.0 ? std::sqrt(hs.rr / hs.bb) : 0.0;
+    if (hs.converged == 2)
+        return na_fail(SPG_E_NOT_CONVERGED, "spg_pcg_solve_noalloc: PCG did not converge within max_iter");
+    if (hs.converged == kPcgBreakdown)
+        return na_fail(SPG_E_NOT_CONVERGED,
+                       "spg_pcg_solve_noalloc: CG breakdown (p.Ap <= 0 after " + std::to_string(hs.iters) +
+                           " iterations): the matrix is not SPD, or the data hold NaN");
     return SPG_OK;
 }
 
@@ -251,9 +281,37 @@ extern "C" int spg_pcg_solve_noalloc(int64_t n, const int32_t *row_ptr, const in
     if (!(rtol > 0.0) || max_iter < 1)
         return na_fail(SPG_E_INVALID, "spg_pcg_solve_noalloc: rtol must be > 0 and max_iter >= 1");
     double *base = nullptr;
-    int rc = na_scratch(&base);
+    ResidentPlan plan;
+    int rc = na_scratch(&base, n, &plan);
     if (rc) return rc;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
+    PcgScalars hs;
+    cudaError_t e;
+    if (plan.blocks > 0) {
+        // the whole solve in one launch; the working vectors' scratch holds its pairs and partial sums
+        ResidentArgs r;
+        r.n = int(n);
+        r.row_ptr = row_ptr;
+        r.col = col;
+        r.val = val;
+        r.b = b;
+        r.x = x;
+        r.zp[0] = reinterpret_cast<double2 *>(base);
+        r.zp[1] = reinterpret_cast<double2 *>(base + 2 * kNoAllocMaxRows);
+        r.partials = base + 4 * kNoAllocMaxRows;
+        r.arrived = reinterpret_cast<unsigned int *>(base + 4 * kNoAllocMaxRows + kResidentPartials);
+        r.sc = reinterpret_cast<PcgScalars *>(base + 5 * kNoAllocMaxRows + 3 * kNaMaxBlocks);
+        r.rtol2 = rtol * rtol;
+        r.max_iter = max_iter;
+        r.breakdown = kPcgBreakdown;
+        r.zero_on_zero_b = true;
+        e = launch_pcg_resident(plan, r, s);
+        if (e == cudaSuccess) e = cudaMemcpyAsync(&hs, r.sc, sizeof(hs), cudaMemcpyDeviceToHost, s);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+        if (e != cudaSuccess) return na_fail(SPG_E_CUDA, std::string("PCG: ") + cudaGetErrorString(e));
+        return na_outcome(hs, iters, relres);
+    }
+    // a device with too few SMs for one row per thread: separate kernels
     NaArgs a;
     a.n = n;
     a.row_ptr = row_ptr;
@@ -274,21 +332,18 @@ extern "C" int spg_pcg_solve_noalloc(int64_t n, const int32_t *row_ptr, const in
     std::memset(&init, 0, sizeof(init));
     init.tol2 = rtol * rtol;
     init.max_iter = max_iter;
-    cudaError_t e = cudaMemcpyAsync(a.sc, &init, sizeof(init), cudaMemcpyHostToDevice, s);
+    e = cudaMemcpyAsync(a.sc, &init, sizeof(init), cudaMemcpyHostToDevice, s);
     if (e != cudaSuccess) return na_fail(SPG_E_CUDA, std::string("scalar reset: ") + cudaGetErrorString(e));
     const int64_t want = (n + kNaThreads - 1) / kNaThreads;
     const unsigned blocks = unsigned(want < kNaMaxBlocks ? want : kNaMaxBlocks);
     k_na_setup<<<blocks, kNaThreads, 0, s>>>(a);
     k_na_rr<<<blocks, kNaThreads, 0, s>>>(a);
     k_na_zero_x<<<blocks, kNaThreads, 0, s>>>(a);
-    PcgScalars hs;
     for (;;) {
         e = cudaMemcpyAsync(&hs, a.sc, sizeof(hs), cudaMemcpyDeviceToHost, s);
         if (e == cudaSuccess) e = cudaStreamSynchronize(s);
         if (e != cudaSuccess) return na_fail(SPG_E_CUDA, std::string("PCG: ") + cudaGetErrorString(e));
-        if (hs.flags)
-            return na_fail(SPG_E_INVALID,
-                           "spg_pcg_solve_noalloc: a row has no stored diagonal entry, or a zero or non-finite one");
+        if (hs.flags) break;
         if (hs.converged) break;
         for (int k = 0; k < kNaChunk; ++k) {
             k_na_spmv_dot<<<blocks, kNaThreads, 0, s>>>(a);
@@ -298,13 +353,5 @@ extern "C" int spg_pcg_solve_noalloc(int64_t n, const int32_t *row_ptr, const in
         e = cudaGetLastError();
         if (e != cudaSuccess) return na_fail(SPG_E_CUDA, std::string("launch: ") + cudaGetErrorString(e));
     }
-    if (iters) *iters = hs.iters;
-    if (relres) *relres = hs.bb > 0.0 ? std::sqrt(hs.rr / hs.bb) : 0.0;
-    if (hs.converged == 2)
-        return na_fail(SPG_E_NOT_CONVERGED, "spg_pcg_solve_noalloc: PCG did not converge within max_iter");
-    if (hs.converged == 3)
-        return na_fail(SPG_E_NOT_CONVERGED,
-                       "spg_pcg_solve_noalloc: CG breakdown (p.Ap <= 0 after " + std::to_string(hs.iters) +
-                           " iterations): the matrix is not SPD, or the data hold NaN");
-    return SPG_OK;
+    return na_outcome(hs, iters, relres);
 }
