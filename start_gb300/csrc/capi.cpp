@@ -94,6 +94,7 @@ struct spg_handle {
     double *efield = nullptr;                 // 3 per tet
     uint32_t *tet_stamp = nullptr;            // per tet: epoch of its field (E, H)
     uint32_t field_epoch = 0;                 // epoch of the current potential's field
+    uint32_t field_seq = 0;                   // last stamp given out (epochs and FP64 step launches)
     bool field_full = true;                   // every tet's field is of field_epoch
     bool in_run = false;                      // inside spg_run: solves refresh the occupied tets only
     // Inside spg_run a while-graph solve does not wait for the host: its
@@ -163,10 +164,10 @@ struct spg_handle {
     int64_t cap = 0, np = 0, n_active = 0, init_lost = 0;
     unsigned int *tri_count = nullptr;
     DevCounters *ctr = nullptr;
-    WalkItem *walkq = nullptr;       // capacity cap (particles)
+    WalkItem *walkq = nullptr;       // mixed form's walk queue, capacity cap (particles)
     unsigned int *walkq_n = nullptr;
-    // segmented steps of the mixed form: at most seg_max steps per segment
-    // (1: one launch per step); resumed-particle list and per-round counters
+    // segmented steps: at most seg_max steps per segment (1: one launch per
+    // step); mixed form: resumed-particle list and per-round counters
     int seg_max = 32;
     int2 *seg_rq = nullptr;
     int64_t seg_rq_cap = 0;
@@ -577,7 +578,7 @@ int alloc_particles(spg_handle *h, int64_t n) {
             CK(dalloc(&P.idf, n));
         }
     }
-    CK(dalloc(&h->walkq, n));
+    if (h->mixed) CK(dalloc(&h->walkq, n));
     h->cap = n;
     return SPG_OK;
 }
@@ -633,7 +634,7 @@ int grow_particles(spg_handle *h, int64_t need) {
         h->P[0] = N[0];
         h->P[1] = N[1];
     }
-    CK(dalloc(&h->walkq, cap));
+    if (h->mixed) CK(dalloc(&h->walkq, cap));
     h->cap = cap;
     h->cur = 0;
     return SPG_OK;
@@ -853,7 +854,7 @@ int do_gather(spg_handle *h) {
     CK(cudaMemsetAsync(h->node_fix, 0, sizeof(unsigned long long) * h->n_nodes, h->stream));
     // the deposit also lists the occupied tets, for the field of the next solve
     CK(cudaMemsetAsync(h->occ_n, 0, sizeof(unsigned int), h->stream));
-    h->occ_epoch = h->field_epoch + 1;
+    h->occ_epoch = h->field_epoch;
     const OccList occ{h->occ_list, h->occ_n, h->occ_gen, ++h->occ_count};
     ev_begin(h, h->ev_dep);
     if (h->mixed)
@@ -897,9 +898,14 @@ FieldArgs field_args(const spg_handle *h) {
 // particles; the walks compute the others as particles enter them.
 int update_field(spg_handle *h, bool sparse) {
     ev_begin(h, h->ev_ef);
-    h->field_epoch++;
+    const bool listed = sparse && h->occ_epoch == h->field_epoch;  // the deposit before this solve listed the tets
+    if (h->field_seq >= 0xf0000000u) {  // stamps start over long before they wrap
+        CK(cudaMemsetAsync(h->tet_stamp, 0, sizeof(uint32_t) * size_t(h->n_tets), h->stream));
+        h->field_seq = 0;
+    }
+    h->field_epoch = ++h->field_seq;
     const FieldArgs f = field_args(h);
-    if (sparse && h->occ_epoch == h->field_epoch) {  // the deposit before this solve listed the tets
+    if (listed) {
         if (h->mixed)
             launch_field32_list(f, h->occ_list, h->occ_n, h->stream);
         else
@@ -923,7 +929,8 @@ int update_field(spg_handle *h, bool sparse) {
 
 // E = 0 everywhere (no solve yet).
 void zero_field(spg_handle *h) {
-    h->field_epoch++;
+    h->field_seq = h->field_seq >= 0xf0000000u ? 1 : h->field_seq + 1;  // every stamp is written
+    h->field_epoch = h->field_seq;
     h->field_full = true;
     launch_zero_field(field_args(h), h->n_tets, h->stream);
 }
@@ -1267,26 +1274,57 @@ void free_tracks(spg_handle *h) {
     h->track_k = h->track_cap = 0;
 }
 
+// Stamp of the next FP64 step launch: above every stamp set so far. With a
+// complete field no launch sets one, and the next number is not used up.
+int step_stamp(spg_handle *h, uint32_t &seq) {
+    if (!h->field_full && h->field_seq < 0xfffffff0u) {
+        seq = ++h->field_seq;
+        return SPG_OK;
+    }
+    if (!h->field_full) {  // out of numbers: a complete field needs none
+        h->field_epoch = h->field_seq = 1;
+        launch_field64_full(field_args(h), h->n_tets, h->stream);
+        CK(cudaGetLastError());
+        h->field_full = true;
+    }
+    seq = h->field_epoch + 1;
+    return SPG_OK;
+}
+
+// Steps h->step .. h->step + l - 1 of the FP64 form in one launch (nothing of
+// the time loop falls between them).
+int do_segment64(spg_handle *h, int l) {
+    h->occ_fresh = false;
+    uint32_t seq = 0;
+    const int rc = step_stamp(h, seq);
+    if (rc) return rc;
+    ev_begin(h, h->ev_step);
+    launch_segment64(h->P[h->cur], h->n_active, mesh_dev(h), step_const(h), l, h->tri_count, h->ctr, field_args(h), seq,
+                     h->stream);
+    ev_end(h, h->ev_step);
+    if (h->n_active > 0) h->launches += 1;
+    CK(cudaGetLastError());
+    if (h->prof)
+        h->step_bytes += double(l) * 152.0 * double(h->occupied ? h->occupied : std::min(h->n_tets, h->n_active));
+    h->step += l;
+    return SPG_OK;
+}
+
 int do_process(spg_handle *h) {
     h->occ_fresh = false;
     if (h->track_k > 0) {
         const int rc = record_tracks(h);
         if (rc) return rc;
     }
+    if (!h->mixed) return do_segment64(h, 1);
     StepConst c = step_const(h);
     ev_begin(h, h->ev_step);
-    if (h->mixed)
-        launch_step32(h->Q[h->cur], h->n_active, mesh_dev32(h), c, h->tri_count, h->walkq, h->walkq_n, h->ctr,
-                      field_args(h), h->stream);
-    else
-        launch_step64(h->P[h->cur], h->n_active, mesh_dev(h), c, h->tri_count, h->walkq, h->walkq_n, h->ctr,
-                      field_args(h), h->stream);
+    launch_step32(h->Q[h->cur], h->n_active, mesh_dev32(h), c, h->tri_count, h->walkq, h->walkq_n, h->ctr,
+                  field_args(h), h->stream);
     ev_end(h, h->ev_step);
     if (h->n_active > 0) h->launches += 2;  // step kernel + queued walks
     CK(cudaGetLastError());
-    if (h->prof)
-        h->step_bytes += (h->mixed ? 92.0 : 152.0) *
-                         double(h->occupied ? h->occupied : std::min(h->n_tets, h->n_active));
+    if (h->prof) h->step_bytes += 92.0 * double(h->occupied ? h->occupied : std::min(h->n_tets, h->n_active));
     h->step++;
     return SPG_OK;
 }
@@ -1323,13 +1361,13 @@ int do_segment32(spg_handle *h, int l) {
 }
 
 // l steps with nothing of the time loop between them: segments of at most
-// seg_max steps in the mixed form (without trajectory sampling, which records
-// every step), single steps otherwise.
+// seg_max steps (without trajectory sampling, which records every step),
+// single steps otherwise.
 int do_steps(spg_handle *h, int l) {
-    if (h->mixed && h->track_k == 0 && h->seg_max > 1 && l > 1) {
+    if (h->track_k == 0 && h->seg_max > 1 && l > 1) {
         while (l > 0) {
             const int m = std::min(l, h->seg_max);
-            const int rc = do_segment32(h, m);
+            const int rc = h->mixed ? do_segment32(h, m) : do_segment64(h, m);
             if (rc) return rc;
             l -= m;
         }
@@ -1553,6 +1591,14 @@ int spg_create(const spg_mesh_desc *mesh, const spg_params *params, spg_handle *
     CK(upload(reinterpret_cast<int32_t **>(&h->ftri), hm.ftri, s));
     CK(upload(reinterpret_cast<int32_t **>(&h->tet_nodes), hm.tet_nodes, s));
     CK(upload(&h->node_xyz, hm.node_xyz, s));
+    // Tets inside the modelling box: every node inside it by 1e-5 of its extent
+    // plus its largest coordinate, far above the rounding of a position.
+    double margin = 0.0;
+    for (int c = 0; c < 3; ++c)
+        margin = std::max(margin, 1e-5 * ((hm.bbox_hi[c] - hm.bbox_lo[c]) +
+                                          std::max(std::fabs(hm.bbox_lo[c]), std::fabs(hm.bbox_hi[c]))));
+    launch_interior_flags(h->rec, h->tet_nodes, h->node_xyz, h->n_tets, hm.bbox_lo, hm.bbox_hi, margin, s);
+    CK(cudaGetLastError());
     {
         std::vector<int64_t> sp;
         std::vector<int32_t> sc;
@@ -1602,13 +1648,8 @@ int spg_create(const spg_mesh_desc *mesh, const spg_params *params, spg_handle *
         std::vector<TetRec32> r32(hm.n_tets);
         std::vector<double> cen(3 * hm.n_tets);
         std::vector<float> cen_lo(3 * hm.n_tets);
-        // Interior tets: every vertex inside the modelling box by 1e-5 of its
-        // extent plus its largest coordinate, some hundred times the FP32
-        // rounding of a centroid-plus-local position and of the box bounds.
-        double margin = 0.0;
-        for (int c = 0; c < 3; ++c)
-            margin = std::max(margin, 1e-5 * ((hm.bbox_hi[c] - hm.bbox_lo[c]) +
-                                              std::max(std::fabs(hm.bbox_lo[c]), std::fabs(hm.bbox_hi[c]))));
+        // Interior tets: the margin is some hundred times the FP32 rounding of a
+        // centroid-plus-local position and of the box bounds.
         for (int64_t t = 0; t < hm.n_tets; ++t) {
             for (int c = 0; c < 3; ++c) {
                 double acc = 0.0;
@@ -2774,7 +2815,7 @@ int spg_grad_forward(spg_handle *h, int32_t nsteps, int32_t checkpoint_every, co
     h->grad_steps = nsteps;
     h->grad_every = checkpoint_every;
     h->grad_step0 = h->step;
-    for (int k = 0; k < nsteps; ++k) {
+    for (int k = 0; k < nsteps;) {
         if (k % checkpoint_every == 0) {
             const int w = k / checkpoint_every;
             rc = h->mixed ? copy_particles32(h, h->ckpt32[w], h->Q[h->cur], n)
@@ -2782,14 +2823,20 @@ int spg_grad_forward(spg_handle *h, int32_t nsteps, int32_t checkpoint_every, co
             if (rc) return rc;
         }
         StepConst c = step_const(h);
-        if (h->mixed)
+        int l = 1;
+        if (h->mixed) {
             launch_step32(h->Q[h->cur], h->n_active, mesh_dev32(h), c, h->tri_count, h->walkq, h->walkq_n, h->ctr,
                           field_args(h), h->stream, h->land);
-        else
-            launch_step64(h->P[h->cur], h->n_active, mesh_dev(h), c, h->tri_count, h->walkq, h->walkq_n, h->ctr,
-                          field_args(h), h->stream, h->land);
+        } else {  // to the next checkpoint in segments
+            l = std::min({nsteps - k, checkpoint_every - k % checkpoint_every, h->seg_max});
+            uint32_t seq = 0;
+            if ((rc = step_stamp(h, seq))) return rc;
+            launch_segment64(h->P[h->cur], h->n_active, mesh_dev(h), c, l, h->tri_count, h->ctr, field_args(h), seq,
+                             h->stream, h->land);
+        }
         CK(cudaGetLastError());
-        h->step++;
+        h->step += l;
+        k += l;
     }
     CK(cudaMemsetAsync(h->sums, 0, 2 * sizeof(double), h->stream));
     if (h->mixed)
@@ -2860,17 +2907,24 @@ int spg_grad_backward(spg_handle *h, double *dJ_dg, double *dJ_dx0, double *dJ_d
         rc = h->mixed ? copy_particles32(h, work32, h->ckpt32[w], n) : copy_particles(h, work, h->ckpt[w], n);
         if (rc) return rc;
         CK(cudaMemsetAsync(h->ctr_scratch, 0, sizeof(DevCounters), s));
-        for (int k = k0; k < k1; ++k) {
+        if (!h->mixed) CK(cudaMemsetAsync(h->hist.tet, 0xff, sizeof(int32_t) * size_t(k1 - k0) * n, s));  // -1: dead
+        for (int k = k0; k < k1;) {
             StepConst c = step_const(h);
             c.step = h->grad_step0 + k;
             if (h->mixed) {
                 launch_record32(work32, n, h->hist, k - k0, s);
                 launch_step32(work32, n, mesh_dev32(h), c, h->tri_scratch, h->walkq, h->walkq_n, h->ctr_scratch,
                               field_args(h), s);
+                ++k;
             } else {
-                launch_record(work, n, h->hist, k - k0, s);
-                launch_step64(work, n, mesh_dev(h), c, h->tri_scratch, h->walkq, h->walkq_n, h->ctr_scratch,
-                              field_args(h), s);
+                const int l = std::min(k1 - k, h->seg_max);
+                const int64_t o = int64_t(k - k0) * n;
+                const AdjHist hist{h->hist.tet + o, h->hist.vx + o, h->hist.vy + o, h->hist.vz + o};
+                uint32_t seq = 0;
+                if ((rc = step_stamp(h, seq))) return rc;
+                launch_segment64(work, n, mesh_dev(h), c, l, h->tri_scratch, h->ctr_scratch, field_args(h), seq, s,
+                                 nullptr, &hist, n);
+                k += l;
             }
         }
         StepConst c = step_const(h);

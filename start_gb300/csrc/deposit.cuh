@@ -231,11 +231,11 @@ __device__ __forceinline__ void deposit_tiles(const Src &src, int64_t n, const i
 
 // Blocks of `kernel` resident on the whole GPU at once (the deposit's one wave).
 template <class K>
-inline int resident_blocks(K kernel, int threads) {
+inline int resident_blocks(K kernel, int threads, size_t smem = 0) {
     int dev = 0, sms = 0, per_sm = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem);
     return std::max(1, sms * std::max(1, per_sm));
 }
 

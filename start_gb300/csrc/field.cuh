@@ -12,7 +12,7 @@ namespace spg {
 template <class F>
 __device__ __forceinline__ void refresh_tet(uint32_t *stamp, uint32_t epoch, int t, F compute) {
     const uint32_t old = __ldcg(stamp + t);
-    if (old == epoch) return;
+    if (old >= epoch) return;
     if (atomicCAS(stamp + t, old, epoch) == old) compute(t);
 }
 

@@ -16,7 +16,7 @@
 //     at step k<N: abar_va = J_Ck^T abar_v(k+1) + dt abar_x
 //     each step:   dJ/dE(t_k) += c abar_va,  abar_v(k) = abar_va
 // The tet sequence t_k and v_k come from recomputing each checkpoint window
-// forward (k_record + the production step kernels); the discrete tet
+// forward (the production step kernel, recording); the discrete tet
 // crossings and collision decisions are piecewise constant and carry no
 // gradient.
 #include <cmath>
@@ -30,16 +30,6 @@ namespace {
 
 constexpr unsigned kFull = 0xffffffffu;
 constexpr double kPi = 3.14159265358979323846;
-
-__global__ void k_record(const DevParticles p, int64_t n, AdjHist h, int k) {
-    const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const int64_t o = int64_t(k) * n + i;
-    h.tet[o] = (p.idf[i] & kDead) ? -1 : p.tet[i];
-    h.vx[o] = p.vx[i];
-    h.vy[o] = p.vy[i];
-    h.vz[o] = p.vz[i];
-}
 
 // dg/dr for each landed particle, g = exp(-|r - r_t|^2 / (2 sigma^2)), and the
 // sums of g and of the landed count (J = sum g / N_landed; the backward scales
@@ -336,9 +326,6 @@ inline unsigned grid_for(int64_t n, int b) { return unsigned((n + b - 1) / b); }
 
 }  // namespace
 
-void launch_record(const DevParticles &p, int64_t n, const AdjHist &h, int k, cudaStream_t s) {
-    if (n > 0) k_record<<<grid_for(n, 256), 256, 0, s>>>(p, n, h, k);
-}
 void launch_objective(const DevParticles &p, int64_t n, const LandRec *land, const double *target, double sigma,
                       double *gr, double *sums, cudaStream_t s) {
     if (n > 0)

@@ -76,7 +76,7 @@ __global__ void k_elements(const double *__restrict__ xyz, int32_t *__restrict__
         r.H[k] = 0.0;
     }
     r.ezero = 0u;
-    r.pad = 0u;
+    r.interior = 0u;
     vol[t] = det / 6.0;
 }
 

@@ -96,9 +96,17 @@ __device__ __forceinline__ bool same_value(double a, double b) {
 // That adds sum_k |M_ik| delta_k (times 1.01 for the truncation of M) to the
 // margin of lambda_i; lambda_0 = 1 - sum gets the sum of the three margins
 // plus 1e-6 for its own FP32 rounding.
-__device__ __forceinline__ bool inside_sure_scr(const TetScreen *__restrict__ scr, double px, double py, double pz) {
+struct ScreenRegs {
+    float4 q0, q1, q2;
+};
+
+__device__ __forceinline__ ScreenRegs load_screen(const TetScreen *__restrict__ scr) {
     const float4 *sp = reinterpret_cast<const float4 *>(scr);
-    const float4 q0 = __ldg(sp), q1 = __ldg(sp + 1), q2 = __ldg(sp + 2);
+    return ScreenRegs{__ldg(sp), __ldg(sp + 1), __ldg(sp + 2)};
+}
+
+__device__ __forceinline__ bool inside_sure(const ScreenRegs &scr, double px, double py, double pz) {
+    const float4 q0 = scr.q0, q1 = scr.q1, q2 = scr.q2;
     const float M[9] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w, q2.x};
     const float X0[3] = {q2.y, q2.z, q2.w};
     const float pf[3] = {hi_float(px), hi_float(py), hi_float(pz)};
@@ -128,17 +136,62 @@ struct WalkOut {
     double s;
 };
 
-// Straight walk of the segment p0 -> p1 starting in tet t (geometry g).
-// In each tet: if p1 is inside (all lambda >= 0) stop. Otherwise leave through
-// the face, other than the entry face, with lambda(p1) < 0 whose crossing
-// parameter s = l0/(l0 - l1) along the segment is smallest (lowest local face
-// index on ties). A face carrying a surface triangle stops the walk there
-// (when stop_surface); a boundary face without one is an exit.
-// FP64 is spent only where the decision needs it: in a tet entered by a
-// crossing the FP32 inside screen usually decides; lambda(p0) and the
-// divisions are formed only when two or more faces compete or s is returned
-// (the same expressions as the full evaluation, so the same values).
-__device__ __noinline__ WalkOut walk64(const MeshDev m, int t, double p0x, double p0y, double p0z, double p1x,
+// The walk's decision in one tet from the FP64 barycentrics (the oracle's):
+// kScreenInside, or the exit face.
+__device__ __noinline__ int exact_exit(const TetRec *__restrict__ rt, double p0x, double p0y, double p0z, double p1x,
+                                       double p1y, double p1z, int enter) {
+    double l1[4];
+    bary_rec(rt, p1x, p1y, p1z, l1);
+    int ncand = 0, best = -1;
+#pragma unroll
+    for (int f = 0; f < 4; ++f)
+        if (f != enter && l1[f] < 0.0) {
+            ++ncand;
+            best = f;
+        }
+    if (ncand == 0) return kScreenInside;
+    if (ncand > 1) {
+        double l0[4], sb = 0.0;
+        bary_rec(rt, p0x, p0y, p0z, l0);
+        best = -1;
+#pragma unroll
+        for (int f = 0; f < 4; ++f) {
+            if (f == enter || !(l1[f] < 0.0)) continue;
+            const double s = l0[f] / (l0[f] - l1[f]);
+            if (best < 0 || s < sb) {
+                best = f;
+                sb = s;
+            }
+        }
+    }
+    return best;
+}
+
+// Crossing parameter of face f along p0 -> p1.
+__device__ __noinline__ double exit_parameter(const TetRec *__restrict__ rt, double p0x, double p0y, double p0z,
+                                              double p1x, double p1y, double p1z, int f) {
+    double l0[4], l1[4];
+    bary_rec(rt, p0x, p0y, p0z, l0);
+    bary_rec(rt, p1x, p1y, p1z, l1);
+    const double a = f == 0 ? l0[0] : f == 1 ? l0[1] : f == 2 ? l0[2] : l0[3];
+    const double b = f == 0 ? l1[0] : f == 1 ? l1[1] : f == 2 ? l1[2] : l1[3];
+    return a / (a - b);
+}
+
+// Straight walk of the segment p0 -> p1 starting in tet t.
+// In each tet: if p1 is inside (no lambda < 0 but of the entry face) stop.
+// Otherwise leave through the face, other than the entry face, with
+// lambda(p1) < 0 whose crossing parameter s = l0/(l0 - l1) along the segment is
+// smallest (lowest local face index on ties). A face carrying a surface
+// triangle stops the walk there (when stop_surface); a boundary face without
+// one is an exit.
+// The decisions come from FP32 with bounds (screen_exit); the FP64 evaluation
+// runs where the bounds leave one open (about one decision in a thousand) and
+// for the crossing parameter that is returned. Deciding in FP64 the walks took
+// a third of the step's FP64 instructions: a lane that needs the second set of
+// barycentrics or a division (a dozen instructions and 1,470 cycles) costs its
+// whole warp.
+__device__ __forceinline__ WalkOut walk64(const MeshDev &m, int t, double p0x, double p0y, double p0z, double p1x,
                                        double p1y, double p1z, int max_cross, bool stop_surface) {
     WalkOut o;
     o.crossings = 0;
@@ -146,72 +199,39 @@ __device__ __noinline__ WalkOut walk64(const MeshDev m, int t, double p0x, doubl
     o.face = -1;
     o.s = 1.0;
     int enter = -1;
+    const double p0[3] = {p0x, p0y, p0z}, p1[3] = {p1x, p1y, p1z};
     for (;;) {
-        if (enter >= 0 && inside_sure_scr(m.screen + t, p1x, p1y, p1z)) {
-            o.tet = t;
-            o.status = W_INSIDE;
-            return o;
-        }
         const TetRec *rt = m.rec + t;
-        double l1[4];
-        bary_rec(rt, p1x, p1y, p1z, l1);
-        if (l1[0] >= 0.0 && l1[1] >= 0.0 && l1[2] >= 0.0 && l1[3] >= 0.0) {
-            o.tet = t;
+        int best;
+        {
+            const ScreenRegs scr = load_screen(m.screen + t);
+            const float4 q0 = scr.q0, q1 = scr.q1, q2 = scr.q2;
+            const float M[9] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w, q2.x};
+            const double2 e = __ldg(reinterpret_cast<const double2 *>(rt) + 4);
+            const double2 f = __ldg(reinterpret_cast<const double2 *>(rt) + 5);
+            const double x0[3] = {e.y, f.x, f.y};
+            best = screen_exit(M, x0, p0, p1, enter);
+        }
+        if (best == kScreenUndecided) best = exact_exit(rt, p0x, p0y, p0z, p1x, p1y, p1z, enter);
+        o.tet = t;
+        if (best == kScreenInside) {
             o.status = W_INSIDE;
             return o;
-        }
-        int ncand = 0, best = -1;
-#pragma unroll
-        for (int f = 0; f < 4; ++f)
-            if (f != enter && l1[f] < 0.0) {
-                ++ncand;
-                best = f;
-            }
-        if (ncand == 0) {
-            o.tet = t;
-            o.status = W_INSIDE;
-            return o;
-        }
-        double l0[4];
-        double sb = 0.0;
-        bool have_s = false;
-        if (ncand > 1) {
-            bary_rec(rt, p0x, p0y, p0z, l0);
-            best = -1;
-#pragma unroll
-            for (int f = 0; f < 4; ++f) {
-                if (f == enter || !(l1[f] < 0.0)) continue;
-                const double s = l0[f] / (l0[f] - l1[f]);
-                if (best < 0 || s < sb) {
-                    best = f;
-                    sb = s;
-                }
-            }
-            have_s = true;
         }
         const int tri = comp(__ldg(m.ftri + t), best);
         const int nb = comp(__ldg(m.nbr + t), best);
-        const bool surface = stop_surface && tri >= 0;
-        if ((surface || nb < 0) && !have_s) {
-            bary_rec(rt, p0x, p0y, p0z, l0);
-            sb = l0[best] / (l0[best] - l1[best]);
-        }
-        if (surface) {
-            o.tet = t;
+        if (stop_surface && tri >= 0) {
             o.status = W_SURFACE;
             o.tri = tri;
             o.face = best;
-            o.s = sb;
+            o.s = exit_parameter(rt, p0x, p0y, p0z, p1x, p1y, p1z, best);
             return o;
         }
         if (nb < 0) {
-            o.tet = t;
             o.status = W_EXIT;
-            o.s = sb;
             return o;
         }
         if (o.crossings == max_cross) {
-            o.tet = t;
             o.status = W_CAP;
             return o;
         }
@@ -223,7 +243,7 @@ __device__ __noinline__ WalkOut walk64(const MeshDev m, int t, double p0x, doubl
 
 // Collision probability exactly as the reference evaluates it:
 // HSModel.cpp:12-15, VHSModel.cpp:14-25 (and VSSModel.cpp, same formula).
-__device__ __noinline__ double probability64(const StepConst c, double vx, double vy, double vz) {
+__device__ __noinline__ double probability64(const StepConst &c, double vx, double vy, double vz) {
     const double vmod = sqrt(vx * vx + vy * vy + vz * vz);
     double sigma;
     if (c.model == SPG_COLL_HS) {
@@ -243,7 +263,7 @@ __device__ __noinline__ double probability64(const StepConst c, double vx, doubl
 // atan2(py, px) as their cosines and sines formed algebraically: the same
 // quantities, rounded differently, at a fraction of the FP64 instructions
 // (collisional runs are compared with the reference statistically).
-__device__ __noinline__ void scatter64(const StepConst c, double u1, double u2, double &vx, double &vy, double &vz) {
+__device__ __noinline__ void scatter64(const StepConst &c, double u1, double u2, double &vx, double &vy, double &vz) {
     double xi_cos;
     if (c.model == SPG_COLL_HS)
         xi_cos = -1.0 + 2.0 * u1;
@@ -288,7 +308,7 @@ __device__ __noinline__ void scatter64(const StepConst c, double u1, double u2, 
 //  * P is computed in FP64 only inside a band.
 // The test where the common case cannot decide it: a candidate, or P that
 // may exceed q (out of line, so the step loop carries none of it).
-__device__ __noinline__ bool collision_test64(const StepConst c, uint32_t id, uint64_t step, uint32_t byte, float v2,
+__device__ __noinline__ bool collision_test64(const StepConst &c, uint32_t id, uint64_t step, uint32_t byte, float v2,
                                               double vx, double vy, double vz) {
     constexpr float qf = float(kCandQ);
     const float pf = c.kp_f * exp2f(c.pexp_f * log2f(v2));
@@ -317,16 +337,21 @@ __device__ __noinline__ bool collision_test64(const StepConst c, uint32_t id, ui
     return P > kCandQ && u01_from(r.v[0], r.v[1]) < (P - kCandQ) / (1.0 - kCandQ);
 }
 
-__device__ __forceinline__ bool collide(const StepConst &c, uint32_t id, double &vx, double &vy, double &vz) {
-    const uint64_t step = uint64_t(c.step);
-    const uint32_t byte = candidate_byte(candidate_block(step, id, c.seed_lo, c.seed_hi), step);
-    const float fx = hi_float(vx), fy = hi_float(vy), fz = hi_float(vz);
-    const float v2 = fmaf(fz, fz, fmaf(fy, fy, fx * fx));
-    if (byte != 0u && v2 <= c.v2_cand_f) return false;
-    if (!collision_test64(c, id, step, byte, v2, vx, vy, vz)) return false;
-    const Philox4 r = collision_draw(step, 1u, id, c.seed_lo, c.seed_hi);
-    scatter64(c, u01_from(r.v[0], r.v[1]), u01_from(r.v[2], r.v[3]), vx, vy, vz);
-    return true;
+// The FP32 screens of collision_test64 that rule a collision out: for a
+// candidate (P certainly below q) u_acc certainly beyond 256 P; else P
+// certainly below q, or u_f certainly beyond its threshold (fast particles in
+// a dense gas, where P exceeds q in every step). False: not certain.
+__device__ __forceinline__ bool no_collision_sure(const StepConst &c, uint32_t id, uint64_t step, bool cand, float v2) {
+    constexpr float qf = float(kCandQ);
+    const float pf = c.kp_f * exp2f(c.pexp_f * log2f(v2));
+    const bool below = pf < qf * (1.0f - 1e-4f);
+    if (!cand && below) return true;
+    if (cand && !below) return false;
+    const uint32_t u = collision_draw(step, cand ? 3u : 4u, id, c.seed_lo, c.seed_hi).v[0] >> 8;
+    const float ulo = float(u) * 5.9604644775390625e-8f;  // 2^-24
+    if (cand) return ulo > pf * 256.0f * (1.0f + 1e-4f);
+    const float tf = (pf - qf) / (1.0f - qf), band = 3e-5f * pf + 2e-7f;
+    return pf > qf * (1.0f + 1e-4f) && ulo > tf + band;
 }
 
 __device__ __forceinline__ unsigned long long warp_sum(unsigned v) { return __reduce_add_sync(kFull, v); }
@@ -336,183 +361,495 @@ __device__ __forceinline__ bool finite_bits(double x) {
     return ((__double2hiint(x) >> 20) & 0x7ff) != 0x7ff;
 }
 
-// Append of this lane's item to the walk queue, called where the lane decides
-// to queue: the lanes converged there share one atomic (their slots follow
-// their lane order; the order of the queue does not matter).
-__device__ __forceinline__ void queue_walk(WalkItem *__restrict__ q, unsigned int *__restrict__ qn, int64_t i,
-                                           double x, double y, double z) {
-    const unsigned act = __activemask();
-    const int lane = threadIdx.x & 31;
-    const int leader = __ffs(act) - 1;
-    unsigned base = 0;
-    if (lane == leader) base = atomicAdd(qn, unsigned(__popc(act)));
-    base = __shfl_sync(act, base, leader);
-    WalkItem &w = q[base + __popc(act & ((1u << lane) - 1u))];
-    w.i = int32_t(i);
-    w.x0 = x;
-    w.y0 = y;
-    w.z0 = z;
-}
-
 // E per tet: E = -sum_i phi_i grad(lambda_i) = -sum_r (phi_{r+1} - phi_0) M_r
 // (VolumetricMesh::computeElectricFields, VolumetricMesh.cpp:382-411, with the
 // sign and scale of E = -grad(phi)), plus the push increment
 // H = ((q E / m) dt) / 2, the operations of Particle::electroMagneticPush.
-__device__ __forceinline__ void field_of_tet64(const FieldArgs &f, int64_t t) {
+struct Field64 {
+    double E[3], H[3];
+    uint32_t ezero;
+};
+
+__device__ __forceinline__ Field64 field_values64(const FieldArgs &f, int64_t t) {
     const int4 tn = __ldg(f.tet_nodes + t);
     const double f0 = f.phi[tn.x], f1 = f.phi[tn.y], f2 = f.phi[tn.z], f3 = f.phi[tn.w];
     const double d1 = f1 - f0, d2 = f2 - f0, d3 = f3 - f0;
-    TetRec &r = f.rec[t];
-    double E[3];
+    const TetRec &r = f.rec[t];
+    Field64 o;
 #pragma unroll
-    for (int k = 0; k < 3; ++k) E[k] = -((d1 * r.M[k] + d2 * r.M[3 + k]) + d3 * r.M[6 + k]);
+    for (int k = 0; k < 3; ++k) o.E[k] = -((d1 * r.M[k] + d2 * r.M[3 + k]) + d3 * r.M[6 + k]);
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
-        f.efield[3 * t + k] = E[k];
-        const double a = div_by_known(f.charge * E[k], f.mass, f.inv_mass);  // (q E) / m
-        r.H[k] = (a * f.dt) / 2.0;
+        const double a = div_by_known(f.charge * o.E[k], f.mass, f.inv_mass);  // (q E) / m
+        o.H[k] = (a * f.dt) / 2.0;
     }
-    r.ezero = (((__double_as_longlong(E[0]) | __double_as_longlong(E[1]) | __double_as_longlong(E[2])) << 1) == 0)
+    o.ezero = (((__double_as_longlong(o.E[0]) | __double_as_longlong(o.E[1]) | __double_as_longlong(o.E[2])) << 1) == 0)
                   ? 1u : 0u;  // all three +-0
+    return o;
 }
 
-// One particle step (ParticleDynamicsProcessor.cpp:161-200 order):
-// settled? -> |v| < vmin? -> outside bbox? -> E push (Boris, B = 0) -> move ->
-// gas collision -> surface crossing along the move segment.
-// The new position is written for every moving particle. A particle whose
-// end point is not certainly inside its tet is appended to the walk queue
-// with its start point; k_walk_queue64 then walks it in full warps (FP64
-// instructions issue per warp on GB300, so a walk taken by a few lanes of
-// every warp would cost the whole warp its FP64 throughput).
-__global__ void __launch_bounds__(256, 6) k_step64(DevParticles p, int64_t n, MeshDev m, StepConst c,
-                                                WalkItem *__restrict__ wq, unsigned int *__restrict__ wq_n,
-                                                DevCounters *ctr) {
-    const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    unsigned processed = 0, coll = 0, lost = 0;
-    if (i < n) {
-        // all of the particle's words in one round trip (the flags gate their use)
-        uint32_t idf = p.idf[i];
-        const int t = p.tet[i];
-        const double x = p.x[i], y = p.y[i], z = p.z[i];
-        double vx = p.vx[i], vy = p.vy[i], vz = p.vz[i];
-        if (!(idf & kDead)) {
-            processed = 1;
+__device__ __forceinline__ void store_field64(const FieldArgs &f, int64_t t, const Field64 &v) {
+    TetRec &r = f.rec[t];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        f.efield[3 * t + k] = v.E[k];
+        r.H[k] = v.H[k];
+    }
+    r.ezero = v.ezero;
+}
+
+__device__ __forceinline__ void field_of_tet64(const FieldArgs &f, int64_t t) {
+    store_field64(f, t, field_values64(f, t));
+}
+
+// ---------------------------------------------------------------- steps
+// Steps c.step .. c.step + L - 1 of every particle in one launch, in the order
+// of ParticleDynamicsProcessor.cpp:161-200: settled? -> |v| < vmin? -> outside
+// bbox? -> E push (Boris, B = 0) -> move -> gas collision -> surface crossing
+// along the move segment.
+//
+// A lane keeps its particle and the tet's push increment in registers and steps
+// it until a step needs what few lanes need: the exact walk (the end point is
+// not certainly inside the tet) or a collision that FP32 cannot rule out. An FP64
+// instruction costs its warp the pipe whatever its active lanes (1.7
+// thread-operations per clock and SM), so every warp schedules its lanes: such
+// a particle's state goes to the warp's pool in shared memory and the lane takes
+// a ready one from there. What is the same for all of them runs in full warps:
+// loading 32 new particles with their push increments and the Philox blocks of
+// the segment (prepare64), and the walks, or the scatterings, of 32 waiting
+// particles (run_pool64). Only the end of a warp's range runs with idle lanes.
+//
+// Against one launch per step with a second one for the walks, the state moves
+// once per segment instead of once per step and a scattering no longer costs
+// 32 lanes (at 4.6e-4 collisions per particle-step every 70th warp-step paid
+// one). The FP64 pipe bounds it, with the twelve operations of push and move:
+// 76 % active (pure FP64 additions reach 81 %), 158 FP64 instructions per warp
+// and ten steps against 171 with blocks that step in lockstep and 190 with the
+// walks decided in FP64. Per step and 1e7 ions on 6.0e6 tets 415 -> 328 us;
+// 1e6 ions on 7.5e5 tets 59 -> 36 us, 3e5 on 94,000 33 -> 14 us, 1e4 on 6,000
+// 21 -> 3.8 us (there the launches and one warp's serial FP64 latency).
+// The values are those of single steps in the same order for every particle,
+// so the segment length changes no result.
+//
+// A walk may enter a tet whose field is of an older potential. Stamps count up
+// with every launch that can write fields: epoch <= stamp < seq says the field
+// was computed by an earlier launch and is read; otherwise the lane forms it in
+// registers, and the lane whose compare-and-swap sets the stamp to seq also
+// stores it for later launches. No lane reads a field written in its launch.
+
+// Items of a warp's pool: those waiting for their walk at [0, np), those ready
+// to step at [kPool - nr, kPool), those with a collision to decide at
+// [kPool, kPool + ns) (while there is room; a scattering is over a hundred FP64
+// instructions, so they wait for a batch of their own instead of costing the
+// walks' batches theirs).
+// Words: position (waiting: at the step's start); waiting: end position, ready:
+// push increment; velocity; tet and id word; index, step and flags; bit j: step
+// j of the segment is a collision candidate.
+// np + nr <= 64 + idle lanes always holds: a step adds what it idles, taking a
+// ready item keeps it, and what adds up to 32 ready items (new particles, a
+// collision batch) runs only while np + nr <= 32 + idle lanes. So a step's
+// 32 - idle items fit kPool = 96.
+constexpr int kPool = 96, kSide = 24, kPoolWords = 12;
+constexpr int kRefill = 2;   // idle lanes that make a warp look for work (8: 343 us per step of 1e7, 4: 331, 2: 328)
+constexpr int kDrain = 16;   // idle lanes that make it run a part-filled batch when nothing else is left
+struct WarpPool {
+    double w[kPoolWords][kPool + kSide];
+    unsigned int cross, settled, lost, capped, coll;
+};
+// Waiting items: the walk; the collision test; a position that is no number.
+constexpr int kNeedWalk = 1, kNeedTest = 2, kNeedLost = 4;
+// Ready items: the field is not zero; the tet lies inside the modelling box; a
+// new particle (its place in its tet not yet shown, its arrays unchanged).
+constexpr int kPush = 1, kInterior = 2, kNew = 4;
+constexpr int kFlagBits = 3;
+
+struct Seg64 {
+    MeshDev m;
+    DevParticles p;
+    int64_t n;
+    unsigned int *tri_count;
+    DevCounters *ctr;
+    LandRec *land;     // nullable: landing records (adjoint)
+    AdjHist hist;      // tet nullptr: none; else tet and velocity at the start of every alive step
+    int64_t hist_n;    // particles of a history plane
+    int L;
+    uint32_t seq;
+};
+
+// Push increment and flags of a tet whose field an earlier launch wrote.
+struct Push64 {
+    double hx, hy, hz;
+    int flags;
+};
+
+__device__ __forceinline__ Push64 load_push(const TetRec *__restrict__ rec, int t) {
+    // the record's last 32 bytes, from L2: an L1 line may be older
+    const double2 *hp = reinterpret_cast<const double2 *>(rec + t) + 6;
+    const double2 a = __ldcg(hp), b = __ldcg(hp + 1);
+    const unsigned long long w = (unsigned long long)__double_as_longlong(b.y);
+    return Push64{a.x, a.y, b.x, ((w & 0xffffffffull) == 0ull ? kPush : 0) | ((w >> 32) != 0ull ? kInterior : 0)};
+}
+
+__device__ __forceinline__ void put_ready(WarpPool &P, int k, double x, double y, double z, const Push64 &h, double vx,
+                                          double vy, double vz, int tet, uint32_t idf, int i, int word, double cand) {
+    P.w[0][k] = x;
+    P.w[1][k] = y;
+    P.w[2][k] = z;
+    P.w[3][k] = h.hx;
+    P.w[4][k] = h.hy;
+    P.w[5][k] = h.hz;
+    P.w[6][k] = vx;
+    P.w[7][k] = vy;
+    P.w[8][k] = vz;
+    P.w[9][k] = __hiloint2double(int(idf), tet);
+    P.w[10][k] = __hiloint2double(word | h.flags, i);
+    P.w[11][k] = cand;
+}
+
+// New particles [base, base + 32) of the warp: the alive ones become ready
+// items. Returns the new count of ready items.
+__device__ __noinline__ int prepare64(const Seg64 &a, const StepConst &c, WarpPool &P, int64_t base, int nr) {
+    const int lane = threadIdx.x & 31;
+    const int64_t i = base + lane;
+    uint32_t idf = kDead;
+    if (i < a.n) idf = a.p.idf[i];
+    const bool alive = !(idf & kDead);
+    const unsigned go = __ballot_sync(kFull, alive);
+    if (alive) {
+        const int tet = a.p.tet[i];
+        const double x = a.p.x[i], y = a.p.y[i], z = a.p.z[i];
+        const double vx = a.p.vx[i], vy = a.p.vy[i], vz = a.p.vz[i];
+        const Push64 h = load_push(a.m.rec, tet);
+        unsigned long long cand = 0ull;
+        if (c.model != SPG_COLL_NONE) {
+            const int first = int(uint32_t(c.step) & 15u);
+            for (int g = 0; 16 * g < first + a.L; ++g) {
+                const unsigned long long m = candidate_mask(
+                    candidate_block(uint64_t(c.step) + 16ull * uint64_t(g), idf & kIdMask, c.seed_lo, c.seed_hi));
+                const int at = 16 * g - first;
+                cand |= at >= 0 ? m << at : m >> -at;
+            }
+        }
+        put_ready(P, kPool - 1 - nr - __popc(go & ((1u << lane) - 1u)), x, y, z, h, vx, vy, vz, tet, idf, int(i), kNew,
+                  __longlong_as_double((long long)cand));
+    }
+    __syncwarp();
+    return nr + __popc(go);
+}
+
+// The waiting items [first, first + take) of the warp's pool, one per lane:
+// collision, walk, landing. An item that goes on becomes a ready one, the
+// others are written to the particle arrays. Returns the new count of ready items.
+__device__ __noinline__ int run_pool64(const Seg64 &a, const StepConst &c, const FieldArgs &f, WarpPool &P, int first,
+                                       int take, int nr) {
+    const int lane = threadIdx.x & 31;
+    const bool mine = lane < take;
+    double x = 0.0, y = 0.0, z = 0.0, vx = 0.0, vy = 0.0, vz = 0.0, cand = 0.0;
+    int tet = 0, i = 0, j = 0;
+    uint32_t idf = 0;
+    bool on = false;
+    unsigned cross = 0;
+    int status = W_INSIDE;
+    bool hit = false;
+    Push64 h{};
+    if (mine) {
+        const int k = first + lane;
+        x = P.w[0][k];
+        y = P.w[1][k];
+        z = P.w[2][k];
+        double nx = P.w[3][k], ny = P.w[4][k], nz = P.w[5][k];
+        vx = P.w[6][k];
+        vy = P.w[7][k];
+        vz = P.w[8][k];
+        const double ti = P.w[9][k], ij = P.w[10][k];
+        cand = P.w[11][k];
+        tet = __double2loint(ti);
+        idf = uint32_t(__double2hiint(ti));
+        i = __double2loint(ij);
+        const int need = __double2hiint(ij);
+        j = need >> kFlagBits;
+        if (need & kNeedTest) {
+            const uint64_t step = uint64_t(c.step) + uint64_t(j);
+            const uint32_t id = idf & kIdMask;
+            const float fx = hi_float(vx), fy = hi_float(vy), fz = hi_float(vz);
+            const uint32_t is_cand = uint32_t((unsigned long long)__double_as_longlong(cand) >> j) & 1u;
+            hit = collision_test64(c, id, step, is_cand ^ 1u, fmaf(fz, fz, fmaf(fy, fy, fx * fx)), vx, vy, vz);
+            if (hit) {
+                const Philox4 r = collision_draw(step, 1u, id, c.seed_lo, c.seed_hi);
+                scatter64(c, u01_from(r.v[0], r.v[1]), u01_from(r.v[2], r.v[3]), vx, vy, vz);
+            }
+        }
+        bool have_field = false;
+        if (need & kNeedLost) {
+            idf |= kLost;
+            status = W_EXIT;
+            a.p.idf[i] = idf;
+            nx = x;
+            ny = y;
+            nz = z;
+        } else if (need & kNeedWalk) {
+            const WalkOut w = walk64(a.m, tet, x, y, z, nx, ny, nz, c.max_cross, true);
+            cross = unsigned(w.crossings);
+            status = w.status;
+            if (w.status == W_SURFACE) {
+                nx = x + w.s * (nx - x);
+                ny = y + w.s * (ny - y);
+                nz = z + w.s * (nz - z);
+                atomicAdd(a.tri_count + w.tri, 1u);
+                idf |= kSettled;
+                if (a.land) {
+                    a.land[i].step = int32_t(c.step + j);
+                    a.land[i].face = w.face;
+                    a.land[i].tet = w.tet;
+                    a.land[i].s = w.s;
+                }
+            } else if (w.status != W_INSIDE) {
+                idf |= kLost;
+            }
+            if (w.status != W_INSIDE) {
+                a.p.idf[i] = idf;
+            } else if (w.tet != tet) {
+                const uint32_t st = __ldcg(f.stamp + w.tet);
+                if (!(st >= f.epoch && st < a.seq)) {
+                    const Field64 v = field_values64(f, w.tet);
+                    h.hx = v.H[0];
+                    h.hy = v.H[1];
+                    h.hz = v.H[2];
+                    h.flags = (v.ezero == 0u ? kPush : 0) | (__ldcg(&a.m.rec[w.tet].interior) != 0u ? kInterior : 0);
+                    have_field = true;
+                    if (st < f.epoch && atomicCAS(f.stamp + w.tet, st, a.seq) == st) store_field64(f, w.tet, v);
+                }
+            }
+            tet = w.tet;
+        }
+        x = nx;
+        y = ny;
+        z = nz;
+        on = status == W_INSIDE && j + 1 < a.L;
+        if (!on) {
+            a.p.x[i] = x;
+            a.p.y[i] = y;
+            a.p.z[i] = z;
+            a.p.vx[i] = vx;
+            a.p.vy[i] = vy;
+            a.p.vz[i] = vz;
+            a.p.tet[i] = tet;
+        } else if (!have_field) {
+            h = load_push(a.m.rec, tet);
+        }
+    }
+    __syncwarp();
+    const unsigned go = __ballot_sync(kFull, on);
+    if (on)
+        put_ready(P, kPool - 1 - nr - __popc(go & ((1u << lane) - 1u)), x, y, z, h, vx, vy, vz, tet, idf, i,
+                  (j + 1) << kFlagBits, cand);
+    const unsigned n0 = __reduce_add_sync(kFull, cross), n4 = __popc(__ballot_sync(kFull, hit));
+    const unsigned n1 = __popc(__ballot_sync(kFull, status == W_SURFACE));
+    const unsigned n2 = __popc(__ballot_sync(kFull, status == W_EXIT || status == W_CAP));
+    const unsigned n3 = __popc(__ballot_sync(kFull, status == W_CAP));
+    if (lane == 0) {
+        P.cross += n0;
+        P.settled += n1;
+        P.lost += n2;
+        P.capped += n3;
+        P.coll += n4;
+    }
+    __syncwarp();
+    return nr + __popc(go);
+}
+
+template <bool HIST>
+__global__ void __launch_bounds__(128, 4) k_seg64(const __grid_constant__ Seg64 a, const __grid_constant__ StepConst c,
+                                                  const __grid_constant__ FieldArgs f) {
+    extern __shared__ __align__(16) unsigned char pool_bytes[];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const unsigned below = (1u << lane) - 1u;
+    WarpPool &P = reinterpret_cast<WarpPool *>(pool_bytes)[wid];
+    if (lane == 0) P.cross = P.settled = P.lost = P.capped = P.coll = 0u;
+    __syncwarp();
+    unsigned processed = 0;
+    int np = 0, nr = 0, ns = 0;
+    // new particles: 32 at a time, the warps of the grid in turn
+    const int64_t stride = int64_t(gridDim.x) * blockDim.x;
+    int64_t base = int64_t(blockIdx.x) * blockDim.x + 32 * wid;
+    bool have = false;
+    double x = 0.0, y = 0.0, z = 0.0, vx = 0.0, vy = 0.0, vz = 0.0, hx = 0.0, hy = 0.0, hz = 0.0;
+    int tet = 0, i = 0, j = 0, flags = 0;
+    uint32_t idf = 0;
+    unsigned long long cand = 0ull;
+    bool dirty = false;
+    for (;;) {
+        unsigned idle = __ballot_sync(kFull, !have);
+        if (__popc(idle) >= kRefill) {
+            if (nr < __popc(idle) && base < a.n && np + nr <= 32 + __popc(idle)) {
+                nr = prepare64(a, c, P, base, nr);
+                base += stride;
+            }
+            if (nr > 0) {
+                const int take = min(nr, __popc(idle));
+                const int k = kPool - nr + __popc(idle & below);
+                if (!have && __popc(idle & below) < take) {
+                    x = P.w[0][k];
+                    y = P.w[1][k];
+                    z = P.w[2][k];
+                    hx = P.w[3][k];
+                    hy = P.w[4][k];
+                    hz = P.w[5][k];
+                    vx = P.w[6][k];
+                    vy = P.w[7][k];
+                    vz = P.w[8][k];
+                    const double ti = P.w[9][k], ij = P.w[10][k];
+                    cand = (unsigned long long)__double_as_longlong(P.w[11][k]);
+                    tet = __double2loint(ti);
+                    idf = uint32_t(__double2hiint(ti));
+                    i = __double2loint(ij);
+                    flags = __double2hiint(ij);
+                    j = flags >> kFlagBits;
+                    dirty = !(flags & kNew);
+                    have = true;
+                }
+                nr -= take;
+                __syncwarp();
+                idle = __ballot_sync(kFull, !have);
+            }
+        }
+        const bool drain = base >= a.n && __popc(idle) >= kDrain;
+        if (np >= 32 || (np > 0 && drain)) {
+            const int take = min(np, 32);
+            np -= take;
+            nr = run_pool64(a, c, f, P, np, take, nr);
+            continue;
+        }
+        if ((ns == kSide || (ns > 0 && drain)) && np + nr <= 32 + __popc(idle)) {
+            nr = run_pool64(a, c, f, P, kPool, ns, nr);
+            ns = 0;
+            continue;
+        }
+        if (idle == kFull) {
+            if (nr > 0 || base < a.n) continue;
+            break;  // nothing waits and no new particle is left
+        }
+        // ---- one step of every lane that has a particle
+        int need = 0;
+        double nx = 0.0, ny = 0.0, nz = 0.0;
+        bool done = false;
+        if (have) {
+            if constexpr (HIST) {
+                const int64_t o = int64_t(j) * a.hist_n + i;
+                a.hist.tet[o] = tet;
+                a.hist.vx[o] = vx;
+                a.hist.vy[o] = vy;
+                a.hist.vz[o] = vz;
+            }
+            ++processed;
             // |v| < vmin: certainly false when some |v_k| >= 2 vmin (bit compare of
             // non-negative doubles); otherwise the exact FP64 test.
             const long long ax = __double_as_longlong(vx) & 0x7fffffffffffffffLL;
             const long long ay = __double_as_longlong(vy) & 0x7fffffffffffffffLL;
             const long long az = __double_as_longlong(vz) & 0x7fffffffffffffffLL;
-            bool slow = false;
+            bool stays = false;
             if (ax < c.two_vmin_bits && ay < c.two_vmin_bits && az < c.two_vmin_bits)
-                slow = sqrt(vx * vx + vy * vy + vz * vz) < c.vmin;
-            const long long kx = order_key(x), ky = order_key(y), kz = order_key(z);
-            const bool inside_box = kx >= c.lo_key[0] && kx <= c.hi_key[0] && ky >= c.lo_key[1] &&
-                                    ky <= c.hi_key[1] && kz >= c.lo_key[2] && kz <= c.hi_key[2];
-            if (!slow && inside_box) {
-                const TetRec *rp = m.rec + t;
-                if (!__ldg(&rp->ezero)) {
+                stays = sqrt(vx * vx + vy * vy + vz * vz) < c.vmin;
+            if ((flags & (kNew | kInterior)) != kInterior) {
+                // outside the modelling box; skipped where this launch has shown the
+                // particle to lie in its tet and the tet lies inside the box
+                const long long kx = order_key(x), ky = order_key(y), kz = order_key(z);
+                stays = stays || !(kx >= c.lo_key[0] && kx <= c.hi_key[0] && ky >= c.lo_key[1] && ky <= c.hi_key[1] &&
+                                   kz >= c.lo_key[2] && kz <= c.hi_key[2]);
+            }
+            if (stays) {  // nothing moves it any more
+                if constexpr (!HIST) {
+                    processed += unsigned(a.L - 1 - j);
+                    j = a.L - 1;
+                }
+            } else {
+                if (flags & kPush) {
                     // Particle::electroMagneticPush (Particle.cpp:196-234) with B = 0:
                     // v- = v + a dt/2, the rotation is the identity, v = v- + a dt/2.
-                    const double hx = __ldg(&rp->H[0]), hy = __ldg(&rp->H[1]), hz = __ldg(&rp->H[2]);
                     vx = (vx + hx) + hx;
                     vy = (vy + hy) + hy;
                     vz = (vz + hz) + hz;
                 }
+                dirty = true;
                 // Particle::updatePosition (Particle.cpp:157-165)
-                const double nx = x + vx * c.dt, ny = y + vy * c.dt, nz = z + vz * c.dt;
+                nx = x + vx * c.dt;
+                ny = y + vy * c.dt;
+                nz = z + vz * c.dt;
                 if (!(same_value(nx, x) && same_value(ny, y) && same_value(nz, z))) {
-                    const uint32_t id = idf & kIdMask;
-                    if (c.model != SPG_COLL_NONE) coll = collide(c, id, vx, vy, vz) ? 1u : 0u;
+                    if (c.model != SPG_COLL_NONE) {
+                        // no candidate and v^2 at most v2_cand_f (from the 20-bit components): no collision
+                        const bool is_cand = (cand >> j) & 1ull;
+                        const float fx = hi_float(vx), fy = hi_float(vy), fz = hi_float(vz);
+                        const float v2 = fmaf(fz, fz, fmaf(fy, fy, fx * fx));
+                        if ((is_cand || !(v2 <= c.v2_cand_f)) &&
+                            !no_collision_sure(c, idf & kIdMask, uint64_t(c.step) + uint64_t(j), is_cand, v2))
+                            need = kNeedTest;
+                    }
                     if (!(finite_bits(nx) && finite_bits(ny) && finite_bits(nz))) {
-                        idf |= kLost;
-                        lost = 1;
-                        p.idf[i] = idf;
+                        need |= kNeedLost;
                     } else {
-                        if (!inside_sure_scr(m.screen + t, nx, ny, nz)) queue_walk(wq, wq_n, i, x, y, z);
-                        p.x[i] = nx;
-                        p.y[i] = ny;
-                        p.z[i] = nz;
+                        if (!inside_sure(load_screen(a.m.screen + tet), nx, ny, nz)) need |= kNeedWalk;
+                        flags &= ~kNew;  // of the next step's position, walked or not
+                        if (!need) {
+                            x = nx;
+                            y = ny;
+                            z = nz;
+                        }
                     }
                 }
-                p.vx[i] = vx;
-                p.vy[i] = vy;
-                p.vz[i] = vz;
             }
+            if (!need) done = ++j == a.L;
+        }
+        const unsigned out = __ballot_sync(kFull, need != 0);
+        if (out) {
+            // collisions to the side while it has room, the rest to the waiting items
+            const unsigned test = __ballot_sync(kFull, (need & kNeedTest) != 0);
+            const int room = kSide - ns;
+            const bool side = (need & kNeedTest) && __popc(test & below) < room;
+            const unsigned main_out = __ballot_sync(kFull, need != 0 && !side);
+            if (need) {
+                const int k = side ? kPool + ns + __popc(test & below) : np + __popc(main_out & below);
+                P.w[0][k] = x;
+                P.w[1][k] = y;
+                P.w[2][k] = z;
+                P.w[3][k] = nx;
+                P.w[4][k] = ny;
+                P.w[5][k] = nz;
+                P.w[6][k] = vx;
+                P.w[7][k] = vy;
+                P.w[8][k] = vz;
+                P.w[9][k] = __hiloint2double(int(idf), tet);
+                P.w[10][k] = __hiloint2double((j << kFlagBits) | need, i);
+                P.w[11][k] = __longlong_as_double((long long)cand);
+                have = false;
+            }
+            np += __popc(main_out);
+            ns += min(__popc(test), room);
+            __syncwarp();
+        }
+        if (done) {
+            if (dirty) {
+                a.p.x[i] = x;
+                a.p.y[i] = y;
+                a.p.z[i] = z;
+                a.p.vx[i] = vx;
+                a.p.vy[i] = vy;
+                a.p.vz[i] = vz;
+                a.p.tet[i] = tet;
+            }
+            have = false;
         }
     }
-    // Block-level counter reduction, one atomic per counter per block (the
-    // walk kernel counts crossings, settled and capped particles).
-    __shared__ unsigned long long sh[8][3];
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    const unsigned long long a0 = warp_sum(processed), a1 = warp_sum(coll), a2 = warp_sum(lost);
+    // one atomic per counter and warp
+    const unsigned long long n0 = warp_sum(processed);
     if (lane == 0) {
-        sh[wid][0] = a0;
-        sh[wid][1] = a1;
-        sh[wid][2] = a2;
-    }
-    __syncthreads();
-    if (threadIdx.x < 3) {
-        unsigned long long s = 0;
-        const int nw = blockDim.x >> 5;
-        for (int w = 0; w < nw; ++w) s += sh[w][threadIdx.x];
-        if (s) {
-            unsigned long long *dst = threadIdx.x == 0   ? &ctr->processed
-                                      : threadIdx.x == 1 ? &ctr->collisions
-                                                         : &ctr->lost;
-            atomicAdd(dst, s);
-        }
-    }
-}
-
-// Exact FP64 walk of the queued particles (start point from the queue, end
-// point already in the position arrays), one particle per lane.
-// With land != nullptr, a particle that settles also records the step, the
-// exit face of its final tet and the hit fraction of the segment (adjoint).
-__global__ void __launch_bounds__(128) k_walk_queue64(DevParticles p, MeshDev m, int max_cross,
-                                                      const WalkItem *__restrict__ wq,
-                                                      const unsigned int *__restrict__ wq_n,
-                                                      unsigned int *__restrict__ tri_count, DevCounters *ctr,
-                                                      LandRec *__restrict__ land, int64_t step, const __grid_constant__ FieldArgs f) {
-    const unsigned nq = *wq_n;
-    unsigned cross = 0, settled = 0, lost = 0, capped = 0;
-    for (unsigned q = blockIdx.x * blockDim.x + threadIdx.x; q < nq; q += gridDim.x * blockDim.x) {
-        const WalkItem it = wq[q];
-        const int64_t i = it.i;
-        const int t = p.tet[i];
-        const double nx = p.x[i], ny = p.y[i], nz = p.z[i];
-        const WalkOut w = walk64(m, t, it.x0, it.y0, it.z0, nx, ny, nz, max_cross, true);
-        cross += unsigned(w.crossings);
-        uint32_t idf = p.idf[i];
-        if (w.status == W_SURFACE) {
-            p.x[i] = it.x0 + w.s * (nx - it.x0);
-            p.y[i] = it.y0 + w.s * (ny - it.y0);
-            p.z[i] = it.z0 + w.s * (nz - it.z0);
-            atomicAdd(tri_count + w.tri, 1u);
-            p.idf[i] = idf | kSettled;
-            settled++;
-            if (land) {
-                land[i].step = int32_t(step);
-                land[i].face = w.face;
-                land[i].tet = w.tet;
-                land[i].s = w.s;
-            }
-        } else if (w.status != W_INSIDE) {
-            p.idf[i] = idf | kLost;
-            lost++;
-            if (w.status == W_CAP) capped++;
-        }
-        if (w.tet != t) {
-            p.tet[i] = w.tet;
-            if (w.status == W_INSIDE) refresh_tet(f.stamp, f.epoch, w.tet, [&f](int tt) { field_of_tet64(f, tt); });
-        }
-    }
-    const unsigned long long a0 = __reduce_add_sync(kFull, cross), a1 = __reduce_add_sync(kFull, settled);
-    const unsigned long long a2 = __reduce_add_sync(kFull, lost), a3 = __reduce_add_sync(kFull, capped);
-    if ((threadIdx.x & 31) == 0) {
-        if (a0) atomicAdd(&ctr->crossings, a0);
-        if (a1) atomicAdd(&ctr->settled, a1);
-        if (a2) atomicAdd(&ctr->lost, a2);
-        if (a3) atomicAdd(&ctr->capped, a3);
+        const unsigned long long n1 = P.coll, n3 = P.cross, n4 = P.settled, n5 = P.capped, n6 = P.lost;
+        if (n0) atomicAdd(&a.ctr->processed, n0);
+        if (n1) atomicAdd(&a.ctr->collisions, n1);
+        if (n3) atomicAdd(&a.ctr->crossings, n3);
+        if (n4) atomicAdd(&a.ctr->settled, n4);
+        if (n5) atomicAdd(&a.ctr->capped, n5);
+        if (n6) atomicAdd(&a.ctr->lost, n6);
     }
 }
 
@@ -621,6 +958,22 @@ __global__ void k_refresh64(DevParticles p, int64_t n, const __grid_constant__ F
         refresh_tet(f.stamp, f.epoch, key, [&f](int t) { field_of_tet64(f, t); });
 }
 
+__global__ void k_interior_flags(TetRec *__restrict__ rec, const int4 *__restrict__ tet_nodes,
+                                 const double *__restrict__ xyz, int64_t n, double lx, double ly, double lz, double hx,
+                                 double hy, double hz) {
+    const int64_t t = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+    if (t >= n) return;
+    const int4 tn = tet_nodes[t];
+    const int nd[4] = {tn.x, tn.y, tn.z, tn.w};
+    bool in = true;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const double x = xyz[3 * int64_t(nd[k])], y = xyz[3 * int64_t(nd[k]) + 1], z = xyz[3 * int64_t(nd[k]) + 2];
+        in = in && x >= lx && x <= hx && y >= ly && y <= hy && z >= lz && z <= hz;
+    }
+    rec[t].interior = in ? 1u : 0u;
+}
+
 // E = 0 and H = 0 everywhere (before the first solve), stamped.
 __global__ void k_zero_field(const __grid_constant__ FieldArgs f, int64_t n) {
     const int64_t t = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
@@ -649,7 +1002,7 @@ __global__ void k_count_lost(const int32_t *__restrict__ tet, int64_t n, unsigne
 }
 
 // Point location: walk from the centroid of the voxel's seed tet to p.
-__global__ void k_locate(const double *__restrict__ pos, int64_t n, MeshDev m, const int32_t *__restrict__ vox_seed,
+__global__ void k_locate(const double *__restrict__ pos, int64_t n, const __grid_constant__ MeshDev m, const int32_t *__restrict__ vox_seed,
                          double ox, double oy, double oz, double ix, double iy, double iz, int dx, int dy, int dz,
                          int max_cross, int32_t *__restrict__ tet_out) {
     const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
@@ -678,8 +1031,8 @@ __global__ void k_locate(const double *__restrict__ pos, int64_t n, MeshDev m, c
 // link), so the copy overlaps the location walks: the same tet and state as
 // k_locate followed by k_init_particles (FP64 form) or k_to_local (mixed form,
 // cen != nullptr: FP32 position about the tet's centroid, FP32 velocity).
-__global__ void __launch_bounds__(128) k_upload(const double *__restrict__ pos, const double *__restrict__ vel, int64_t n, MeshDev m,
-                         const int32_t *__restrict__ vox_seed, double ox, double oy, double oz, double ix, double iy,
+__global__ void __launch_bounds__(128) k_upload(const double *__restrict__ pos, const double *__restrict__ vel, int64_t n,
+                         const __grid_constant__ MeshDev m, const int32_t *__restrict__ vox_seed, double ox, double oy, double oz, double ix, double iy,
                          double iz, int dx, int dy, int dz, int max_cross, DevParticles p, DevParticles32 q,
                          const double *__restrict__ cen, unsigned long long *lost) {
     // the block's xyz triples come in as one contiguous run per array (whole
@@ -918,13 +1271,35 @@ inline unsigned grid_for(int64_t n, int block) { return unsigned((n + block - 1)
 
 }  // namespace
 
-void launch_step64(const DevParticles &p, int64_t n, const MeshDev &m, const StepConst &c, unsigned int *tri_count,
-                   WalkItem *wq, unsigned int *wq_n, DevCounters *ctr, const FieldArgs &f, cudaStream_t s,
-                   LandRec *land) {
-    if (n <= 0) return;
-    cudaMemsetAsync(wq_n, 0, sizeof(unsigned int), s);
-    k_step64<<<grid_for(n, 256), 256, 0, s>>>(p, n, m, c, wq, wq_n, ctr);
-    k_walk_queue64<<<152 * 8, 128, 0, s>>>(p, m, c.max_cross, wq, wq_n, tri_count, ctr, land, c.step, f);
+void launch_segment64(const DevParticles &p, int64_t n, const MeshDev &m, const StepConst &c, int L,
+                      unsigned int *tri_count, DevCounters *ctr, const FieldArgs &f, uint32_t seq, cudaStream_t s,
+                      LandRec *land, const AdjHist *hist, int64_t hist_n) {
+    if (n <= 0 || L <= 0) return;
+    Seg64 a{};
+    a.m = m;
+    a.p = p;
+    a.n = n;
+    a.tri_count = tri_count;
+    a.ctr = ctr;
+    a.land = land;
+    if (hist) a.hist = *hist;
+    a.hist_n = hist_n;
+    a.L = L;
+    a.seq = seq;
+    // one wave: SMs x resident blocks (same on every device of this build);
+    // few particles spread over smaller blocks so that every SM has some
+    static int resident[2] = {0, 0};
+    int &r = resident[hist ? 1 : 0];
+    constexpr int kT = 128;
+    constexpr size_t smem = sizeof(WarpPool) * kT / 32;
+    static_assert(smem <= 48 * 1024, "a block's pools fit the default limit of dynamic shared memory");
+    if (r == 0) r = hist ? resident_blocks(k_seg64<true>, kT, smem) : resident_blocks(k_seg64<false>, kT, smem);
+    const int T = n >= int64_t(r) * kT ? kT : 32;
+    const unsigned grid = unsigned(std::min<int64_t>(grid_for(n, T), int64_t(r) * (kT / T)));
+    if (hist)
+        k_seg64<true><<<grid, T, smem * T / kT, s>>>(a, c, f);
+    else
+        k_seg64<false><<<grid, T, smem * T / kT, s>>>(a, c, f);
 }
 
 void launch_deposit64(const DevParticles &p, int64_t n, const MeshDev &m, int k, unsigned long long *node_fix,
@@ -956,6 +1331,14 @@ void launch_refresh64(const DevParticles &p, int64_t n, const FieldArgs &f, cuda
 
 void launch_zero_field(const FieldArgs &f, int64_t n_tets, cudaStream_t s) {
     if (n_tets > 0) k_zero_field<<<grid_for(n_tets, 256), 256, 0, s>>>(f, n_tets);
+}
+
+void launch_interior_flags(TetRec *rec, const int4 *tet_nodes, const double *node_xyz, int64_t n_tets,
+                           const double *lo, const double *hi, double margin, cudaStream_t s) {
+    if (n_tets > 0)
+        k_interior_flags<<<grid_for(n_tets, 256), 256, 0, s>>>(rec, tet_nodes, node_xyz, n_tets, lo[0] + margin,
+                                                              lo[1] + margin, lo[2] + margin, hi[0] - margin,
+                                                              hi[1] - margin, hi[2] - margin);
 }
 
 void launch_count_lost(const int32_t *tet, int64_t n, unsigned long long *out, cudaStream_t s) {

@@ -32,7 +32,7 @@ struct alignas(128) TetRec {
     double x0[3];
     double H[3];
     uint32_t ezero;
-    uint32_t pad;
+    uint32_t interior;  // the tet lies inside the modelling box with a margin (launch_interior_flags)
 };
 static_assert(sizeof(TetRec) == 128, "TetRec must be one 128-byte line");
 
@@ -150,11 +150,9 @@ struct MeshDev {
     int64_t n_tets, n_nodes;
 };
 
-// A particle whose move needs the exact tet walk: its index and start point.
-struct WalkItem {
-    int32_t i;
-    int32_t pad;
-    double x0, y0, z0;
+// Words of the mixed form's walk queue per particle (its items take 16 or 20 bytes).
+struct alignas(16) WalkItem {
+    int32_t w[8];
 };
 
 // Landing record of a settled particle (adjoint of the landing point): step
@@ -176,7 +174,6 @@ struct AdjHist {
 };
 
 // kernels_adjoint.cu
-void launch_record(const DevParticles &p, int64_t n, const AdjHist &h, int k, cudaStream_t s);
 void launch_objective(const DevParticles &p, int64_t n, const LandRec *land, const double *target, double sigma,
                       double *gr, double *sums, cudaStream_t s);
 // G (nullable): per-tet gradient of the recovered field (launch_field_gradient);
@@ -212,12 +209,16 @@ struct OccList {
     uint32_t gen;
 };
 // Kernel launchers (kernels_particles.cu).
-// Step kernel plus the exact walk of the queued particles (wq holds up to n
-// items); land (nullable) receives the landing records; a walk that brings a
-// particle into a tet with an older field computes that tet's field (f).
-void launch_step64(const DevParticles &p, int64_t n, const MeshDev &m, const StepConst &c,
-                   unsigned int *tri_count, WalkItem *wq, unsigned int *wq_n, DevCounters *ctr, const FieldArgs &f,
-                   cudaStream_t s, LandRec *land = nullptr);
+// Steps c.step .. c.step + L - 1 of the FP64 form in one launch. seq: a stamp
+// above every one set before (field writes of this launch); land (nullable)
+// receives the landing records; hist (nullable): tet and velocity at the start
+// of every step in which a particle is alive, step j at [j hist_n + i].
+void launch_segment64(const DevParticles &p, int64_t n, const MeshDev &m, const StepConst &c, int L,
+                      unsigned int *tri_count, DevCounters *ctr, const FieldArgs &f, uint32_t seq, cudaStream_t s,
+                      LandRec *land = nullptr, const AdjHist *hist = nullptr, int64_t hist_n = 0);
+// TetRec::interior of every tet: all four nodes inside [lo, hi] by margin.
+void launch_interior_flags(TetRec *rec, const int4 *tet_nodes, const double *node_xyz, int64_t n_tets,
+                           const double *lo, const double *hi, double margin, cudaStream_t s);
 // Fixed-point P1 deposit: node_fix[n] += round(lambda_n * 2^k) per alive
 // particle (lambda_0 takes the remainder so each particle adds exactly 2^k).
 // occ (list nullable) collects the tets holding particles.
@@ -274,16 +275,18 @@ static_assert(sizeof(TetRec32) == 64, "TetRec32 must be 64 bytes");
 // current potential. A full update computes every tet. After a solve inside
 // spg_run only the tets holding particles are computed (launch_refresh*),
 // and a walk that brings a particle into a tet whose field belongs to an
-// older potential (stamp[t] != epoch) computes that tet there: the first
-// lane to swap the stamp computes, the values are those of the full update,
-// and the next step (a later launch) reads them.
+// older potential (stamp[t] < epoch) computes that tet there: the first
+// lane to swap the stamp stores it, the values are those of the full update,
+// and later launches read them. The FP64 form stamps with a number of the
+// launch (above epoch), so that a lane can tell a field stored by an earlier
+// launch from one being stored beside it.
 struct FieldArgs {
     const int4 *tet_nodes;
     const double *phi;
     double *efield;    // 3 per tet
     TetRec *rec;       // FP64 map (read); H and ezero written in the FP64 form
     TetRec32 *rec32;   // mixed form: FP32 H and ezero written; nullptr in the FP64 form
-    uint32_t *stamp;   // per tet: epoch of its field
+    uint32_t *stamp;   // per tet: at least epoch once its field is of the current potential
     uint32_t epoch;
     double charge, mass, inv_mass, dt;
     double c32;        // mixed form: q dt / (2 m)
