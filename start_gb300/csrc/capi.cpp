@@ -220,7 +220,8 @@ struct spg_handle {
     LandRec *land = nullptr;
     double *gr = nullptr, *adj_x = nullptr, *adj_v = nullptr, *gE = nullptr, *lam = nullptr, *mu = nullptr,
            *dJdg = nullptr, *sums = nullptr;
-    AdjHist hist{};
+    HistRec *hist64 = nullptr;           // FP64 form
+    AdjHist hist{};                      // mixed form
     unsigned int *tri_scratch = nullptr;
     DevCounters *ctr_scratch = nullptr;
     std::vector<DevParticles32> ckpt32;  // the same for the FP32 form
@@ -1756,7 +1757,7 @@ int spg_destroy(spg_handle *h) {
                     h->rec32,    h->cen,      h->cen_lo,   h->sval32,   h->inv_diag32, h->e32,     h->r32,       h->z32,
                     h->p32,      h->q32,      h->partials32, h->sc32,
                     h->elim_rp,  h->elim_row, h->elim_col, h->elim_val, h->land, h->gr, h->adj_x, h->adj_v,
-                    h->gE,       h->lam,      h->mu,       h->dJdg,    h->sums, h->hist.tet, h->hist.vx,
+                    h->gE,       h->lam,      h->mu,       h->dJdg,    h->sums, h->hist64, h->hist.tet, h->hist.vx,
                     h->hist.vy,  h->hist.vz,  h->tri_scratch, h->ctr_scratch,
                     h->q,        h->partials, h->sc,       h->tri_count, h->ctr,      h->n_alive_dev, h->sort_scratch, h->walkq_n,
                     h->io,       h->seg_rq,   h->seg_qn,   h->res_zp,  h->res_partials, h->res_arrived};
@@ -2629,16 +2630,8 @@ int ensure(spg_handle *h, T **ptr, size_t count) {
 }
 
 int copy_particles(spg_handle *h, const DevParticles &dst, const DevParticles &src, int64_t n) {
-    if (n == 0) return SPG_OK;
-    cudaStream_t s = h->stream;
-    CK(cudaMemcpyAsync(dst.x, src.x, 8 * n, cudaMemcpyDeviceToDevice, s));
-    CK(cudaMemcpyAsync(dst.y, src.y, 8 * n, cudaMemcpyDeviceToDevice, s));
-    CK(cudaMemcpyAsync(dst.z, src.z, 8 * n, cudaMemcpyDeviceToDevice, s));
-    CK(cudaMemcpyAsync(dst.vx, src.vx, 8 * n, cudaMemcpyDeviceToDevice, s));
-    CK(cudaMemcpyAsync(dst.vy, src.vy, 8 * n, cudaMemcpyDeviceToDevice, s));
-    CK(cudaMemcpyAsync(dst.vz, src.vz, 8 * n, cudaMemcpyDeviceToDevice, s));
-    CK(cudaMemcpyAsync(dst.tet, src.tet, 4 * n, cudaMemcpyDeviceToDevice, s));
-    CK(cudaMemcpyAsync(dst.idf, src.idf, 4 * n, cudaMemcpyDeviceToDevice, s));
+    launch_copy_alive(src, dst, n, h->stream);
+    CK(cudaGetLastError());
     return SPG_OK;
 }
 
@@ -2663,15 +2656,8 @@ int alloc_dev_particles(spg_handle *h, DevParticles &P, int64_t n) {
 }
 
 int copy_particles32(spg_handle *h, const DevParticles32 &dst, const DevParticles32 &src, int64_t n) {
-    if (n == 0) return SPG_OK;
-    cudaStream_t s = h->stream;
-    for (int k = 0; k < 6; ++k) {
-        float *d = k == 0 ? dst.x : k == 1 ? dst.y : k == 2 ? dst.z : k == 3 ? dst.vx : k == 4 ? dst.vy : dst.vz;
-        const float *q = k == 0 ? src.x : k == 1 ? src.y : k == 2 ? src.z : k == 3 ? src.vx : k == 4 ? src.vy : src.vz;
-        CK(cudaMemcpyAsync(d, q, 4 * n, cudaMemcpyDeviceToDevice, s));
-    }
-    CK(cudaMemcpyAsync(dst.tet, src.tet, 4 * n, cudaMemcpyDeviceToDevice, s));
-    CK(cudaMemcpyAsync(dst.idf, src.idf, 4 * n, cudaMemcpyDeviceToDevice, s));
+    launch_copy_alive32(src, dst, n, h->stream);
+    CK(cudaGetLastError());
     return SPG_OK;
 }
 
@@ -2866,13 +2852,20 @@ int spg_grad_backward(spg_handle *h, double *dJ_dg, double *dJ_dx0, double *dJ_d
     h->occ_fresh = false;
     const int64_t hneed = int64_t(W) * std::max<int64_t>(n, 1);
     if (hneed > h->hist_cap) {
-        for (void *q : {(void *)h->hist.tet, (void *)h->hist.vx, (void *)h->hist.vy, (void *)h->hist.vz}) cudaFree(q);
+        for (void *q : {(void *)h->hist64, (void *)h->hist.tet, (void *)h->hist.vx, (void *)h->hist.vy,
+                        (void *)h->hist.vz})
+            cudaFree(q);
+        h->hist64 = nullptr;
         h->hist = AdjHist{};
         h->hist_cap = 0;
-        CK(dalloc(&h->hist.tet, hneed));
-        CK(dalloc(&h->hist.vx, hneed));
-        CK(dalloc(&h->hist.vy, hneed));
-        CK(dalloc(&h->hist.vz, hneed));
+        if (h->mixed) {
+            CK(dalloc(&h->hist.tet, hneed));
+            CK(dalloc(&h->hist.vx, hneed));
+            CK(dalloc(&h->hist.vy, hneed));
+            CK(dalloc(&h->hist.vz, hneed));
+        } else {
+            CK(dalloc(&h->hist64, hneed));
+        }
         h->hist_cap = hneed;
     }
     CK(cudaMemsetAsync(h->adj_x, 0, sizeof(double) * 3 * n, s));
@@ -2907,7 +2900,6 @@ int spg_grad_backward(spg_handle *h, double *dJ_dg, double *dJ_dx0, double *dJ_d
         rc = h->mixed ? copy_particles32(h, work32, h->ckpt32[w], n) : copy_particles(h, work, h->ckpt[w], n);
         if (rc) return rc;
         CK(cudaMemsetAsync(h->ctr_scratch, 0, sizeof(DevCounters), s));
-        if (!h->mixed) CK(cudaMemsetAsync(h->hist.tet, 0xff, sizeof(int32_t) * size_t(k1 - k0) * n, s));  // -1: dead
         for (int k = k0; k < k1;) {
             StepConst c = step_const(h);
             c.step = h->grad_step0 + k;
@@ -2918,12 +2910,10 @@ int spg_grad_backward(spg_handle *h, double *dJ_dg, double *dJ_dx0, double *dJ_d
                 ++k;
             } else {
                 const int l = std::min(k1 - k, h->seg_max);
-                const int64_t o = int64_t(k - k0) * n;
-                const AdjHist hist{h->hist.tet + o, h->hist.vx + o, h->hist.vy + o, h->hist.vz + o};
                 uint32_t seq = 0;
                 if ((rc = step_stamp(h, seq))) return rc;
                 launch_segment64(work, n, mesh_dev(h), c, l, h->tri_scratch, h->ctr_scratch, field_args(h), seq, s,
-                                 nullptr, &hist, n);
+                                 nullptr, h->hist64 + int64_t(k - k0) * n, n);
                 k += l;
             }
         }
@@ -2933,12 +2923,12 @@ int spg_grad_backward(spg_handle *h, double *dJ_dg, double *dJ_dx0, double *dJ_d
             launch_backward32(work32, n, mesh_dev32(h), h->hist, k0, k1, h->land, h->gr, h->grad_inv_n, h->adj_x,
                               h->adj_v, h->gE, c, s, G);
         else
-            launch_backward(work, n, h->hist, k0, k1, h->rec, h->land, h->gr, h->grad_inv_n, h->adj_x, h->adj_v,
+            launch_backward(work, n, h->hist64, k0, k1, h->rec, h->land, h->gr, h->grad_inv_n, h->adj_x, h->adj_v,
                             h->gE, c, s, G);
         CK(cudaGetLastError());
     }
     CK(cudaMemsetAsync(h->lam, 0, sizeof(double) * h->n_nodes, s));
-    launch_gE_to_nodes(h->tet_nodes, h->rec, h->gE, h->n_tets, h->lam, s);
+    launch_gE_to_nodes(h->tet_nodes, h->rec, h->gE, (h->prm.charge / h->prm.mass) * h->prm.dt, h->n_tets, h->lam, s);
     launch_adj_rhs(h->lam, h->is_dir, h->b, h->mu, h->n_nodes, s);
     CK(cudaGetLastError());
     int32_t it = 0;
@@ -2949,9 +2939,17 @@ int spg_grad_backward(spg_handle *h, double *dJ_dg, double *dJ_dx0, double *dJ_d
     CK(cudaGetLastError());
     CK(cudaMemcpyAsync(dJ_dg, h->dJdg, sizeof(double) * h->n_nodes, cudaMemcpyDeviceToHost, s));
     if (dJ_dx0 || dJ_dv0) {
-        double *dx = nullptr, *dv = nullptr;
-        if (dJ_dx0) CK(dalloc(&dx, 3 * n));
-        if (dJ_dv0) CK(dalloc(&dv, 3 * n));
+        // in id order through the window record, which nothing reads any more
+        double *own = nullptr, *dx = nullptr;
+        if (h->mixed ? h->hist_cap >= 6 * n : h->hist_cap >= 2 * n) {
+            dx = h->mixed ? h->hist.vx : reinterpret_cast<double *>(h->hist64);
+        } else {
+            CK(dalloc(&own, 6 * size_t(n)));
+            dx = own;
+        }
+        double *dv = dx + 3 * n;
+        if (!dJ_dx0) dx = nullptr;
+        if (!dJ_dv0) dv = nullptr;
         if (h->mixed)
             launch_gather_adj32(h->Q[h->cur], n, h->adj_x, h->adj_v, dx, dv, s);
         else
@@ -2959,8 +2957,7 @@ int spg_grad_backward(spg_handle *h, double *dJ_dg, double *dJ_dx0, double *dJ_d
         if (dJ_dx0) CK(cudaMemcpyAsync(dJ_dx0, dx, sizeof(double) * 3 * n, cudaMemcpyDeviceToHost, s));
         if (dJ_dv0) CK(cudaMemcpyAsync(dJ_dv0, dv, sizeof(double) * 3 * n, cudaMemcpyDeviceToHost, s));
         CK(cudaStreamSynchronize(s));
-        cudaFree(dx);
-        cudaFree(dv);
+        cudaFree(own);
     }
     CK(cudaStreamSynchronize(s));
     return SPG_OK;

@@ -21,7 +21,7 @@
 // gradient.
 #include <cmath>
 
-#include "philox.h"
+#include "collide64.cuh"
 #include "spg_internal.h"
 
 namespace spg {
@@ -29,7 +29,6 @@ namespace spg {
 namespace {
 
 constexpr unsigned kFull = 0xffffffffu;
-constexpr double kPi = 3.14159265358979323846;
 
 // dg/dr for each landed particle, g = exp(-|r - r_t|^2 / (2 sigma^2)), and the
 // sums of g and of the landed count (J = sum g / N_landed; the backward scales
@@ -69,49 +68,51 @@ __device__ __forceinline__ void face_normal(const TetRec &r, int f, double n[3])
     }
 }
 
-// Collision decision of step k for velocity va, exactly as the forward took
-// it (u0 < P with the reference's P), and the scattering direction.
-__device__ bool collided(const StepConst &c, uint32_t id, int64_t k, double vx, double vy, double vz, double nh[3]) {
-    const uint32_t byte = candidate_byte(candidate_block(uint64_t(k), id, c.seed_lo, c.seed_hi), uint64_t(k));
-    const double vmod = sqrt(vx * vx + vy * vy + vz * vz);
-    double sigma;
-    if (c.model == SPG_COLL_HS) {
-        sigma = c.sigma_hs;
-    } else {
-        const double base = c.two_kT / ((c.mr * vmod) * vmod);
-        sigma = kPi * (c.vhs_c1 * pow(base, c.expo));
-    }
-    const double P = ((sigma * vmod) * c.gas_n) * c.dt;
-    bool hit;
-    if (P <= kCandQ) {
-        hit = byte == 0u && u01_from_block(collision_draw(uint64_t(k), 3u, id, c.seed_lo, c.seed_hi)) < P * 256.0;
-    } else {
-        hit = byte == 0u ||
-              u01_from_block(collision_draw(uint64_t(k), 4u, id, c.seed_lo, c.seed_hi)) < (P - kCandQ) / (1.0 - kCandQ);
-    }
-    if (!hit) return false;
-    const Philox4 r = collision_draw(uint64_t(k), 1u, id, c.seed_lo, c.seed_hi);
+// abar_v through the collision of step `step` of pushed velocity v, its event
+// and random numbers held fixed: v' = m_cp v + m_ct |v| n, so
+// J^T a = m_cp a + m_ct v/|v| (n . a).
+__device__ __noinline__ void collision_adjoint(const StepConst &c, uint32_t id, uint64_t step, double vx, double vy,
+                                               double vz, double V[3]) {
+    const Philox4 r = collision_draw(step, 1u, id, c.seed_lo, c.seed_hi);
     const double u1 = u01_from(r.v[0], r.v[1]);
     const double u2 = u01_from(r.v[2], r.v[3]);
     const double xc = c.model == SPG_COLL_HS ? -1.0 + 2.0 * u1 : u1;
     const double xs = sqrt(1.0 - xc * xc);
     double sph, cph;  // the forward's azimuth, cospi / sinpi (2 u2)
     sincospi(2.0 * u2, &sph, &cph);
-    nh[0] = xs * cph;
-    nh[1] = xs * sph;
-    nh[2] = xc;
-    return true;
+    const double vm = sqrt(vx * vx + vy * vy + vz * vz);
+    const double na = (xs * cph * V[0] + xs * sph * V[1] + xc * V[2]) * c.mass_ct / vm;
+    V[0] = c.mass_cp * V[0] + na * vx;
+    V[1] = c.mass_cp * V[1] + na * vy;
+    V[2] = c.mass_cp * V[2] + na * vz;
+}
+
+// Upper bound of |v_k + 2 h_k| from the 20-bit components (hi_float truncates
+// toward zero, by at most 9.6e-7 of the value; 0 below 2^-126).
+__device__ __forceinline__ float reach(double v, double h) {
+    return fmaf(fabsf(hi_float(v)) + 2.0f * fabsf(hi_float(h)), 1.0f + 2e-6f, 1e-30f);
 }
 
 // Backward recursion over steps [k0, k1) of one checkpoint window, one
 // particle per thread; the adjoint state (abar_x, abar_v) carries between
 // windows in ax/av. Contributions to dJ/dE of consecutive steps in one tet
-// are summed in registers and added once.
-__global__ void __launch_bounds__(128) k_backward(const DevParticles p, int64_t n, const AdjHist h, int k0, int k1,
+// are summed in registers and added once (k_gE_to_nodes scales them).
+// FP64 issue bounds it (1.7 thread-operations per clock and SM), so a step takes
+// FP64 only for the recursion itself, three FMAs and three additions: the
+// slow-particle test is decided by the exponents, and a collision is ruled out
+// by the candidate bits (one Philox block per sixteen steps) with a bound of the
+// pushed speed; only a step that these leave open forms the pushed velocity and
+// decides as the forward did (collide64.cuh). With a square root, a Philox block
+// and the FP64 probability in every step the ten windows of 1e6 ions, 300 steps
+// took 11.5 ms; now 3.1 (FP64 pipe 80 % active; the rest of its instructions are
+// the tet changes and collisions of single lanes). The next step's record is
+// loaded before the current one is used.
+__global__ void __launch_bounds__(128) k_backward(const DevParticles p, int64_t n, const HistRec *__restrict__ h, int k0, int k1,
                                                   const TetRec *__restrict__ rec, const LandRec *__restrict__ land,
                                                   const double *__restrict__ gr, double gscale, double *__restrict__ ax,
-                                                  double *__restrict__ av, double *__restrict__ gE, StepConst c,
-                                                  double cq, const double *__restrict__ G) {
+                                                  double *__restrict__ av, double *__restrict__ gE,
+                                                  const __grid_constant__ StepConst c, double cq,
+                                                  const double *__restrict__ G) {
     const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const LandRec L = land[i];
@@ -123,27 +124,43 @@ __global__ void __launch_bounds__(128) k_backward(const DevParticles p, int64_t 
     double Vx = av[3 * i], Vy = av[3 * i + 1], Vz = av[3 * i + 2];
     int run = -1;
     double sx = 0.0, sy = 0.0, sz = 0.0;
-    for (int k = min(k1 - 1, N); k >= k0; --k) {
-        const int64_t o = int64_t(k - k0) * n + i;
-        const int t = h.tet[o];
-        if (t < 0) continue;
-        const double vx = h.vx[o], vy = h.vy[o], vz = h.vz[o];
-        if (sqrt(vx * vx + vy * vy + vz * vz) < c.vmin) continue;  // the step did not move it
-        const TetRec &R = rec[t];
-        double ax_ = vx, ay_ = vy, az_ = vz;
-        if (!R.ezero) {
-            ax_ = (vx + R.H[0]) + R.H[0];
-            ay_ = (vy + R.H[1]) + R.H[1];
-            az_ = (vz + R.H[2]) + R.H[2];
+    uint32_t cmask = 0u, cgroup = ~0u;  // candidate steps of the current sixteen-step group
+    int k = min(k1 - 1, N);
+    const double2 *hp2 = reinterpret_cast<const double2 *>(h + int64_t(k - k0) * n + i);
+    double2 a_next = __ldg(hp2), b_next = __ldg(hp2 + 1);
+    for (; k >= k0; --k) {
+        const int t = __double2loint(b_next.y);
+        double vx = a_next.x, vy = a_next.y, vz = b_next.x;
+        if (k > k0) {
+            hp2 -= 2 * n;
+            a_next = __ldg(hp2);
+            b_next = __ldg(hp2 + 1);
         }
+        // |v| < vmin: the step did not move it (certainly false when some |v_k| >= 2 vmin)
+        if ((__double_as_longlong(vx) & 0x7fffffffffffffffLL) < c.two_vmin_bits &&
+            (__double_as_longlong(vy) & 0x7fffffffffffffffLL) < c.two_vmin_bits &&
+            (__double_as_longlong(vz) & 0x7fffffffffffffffLL) < c.two_vmin_bits &&
+            sqrt(vx * vx + vy * vy + vz * vz) < c.vmin)
+            continue;
+        const double2 *hp = reinterpret_cast<const double2 *>(rec + t) + 6;
+        const double2 h0 = __ldg(hp), h1 = __ldg(hp + 1);
+        const bool push = uint32_t(__double2loint(h1.y)) == 0u;  // ezero
+        auto pushed = [&] {  // v_a
+            if (push) {
+                vx = (vx + h0.x) + h0.x;
+                vy = (vy + h0.y) + h0.y;
+                vz = (vz + h1.x) + h1.x;
+            }
+        };
         double bx, by, bz;  // abar_va
         if (k == N) {
+            pushed();
             const TetRec &RL = rec[L.tet];
             double nn[3];
             face_normal(RL, L.face, nn);
             const double gx = gr[3 * i] * gscale, gy = gr[3 * i + 1] * gscale, gz = gr[3 * i + 2] * gscale;
-            const double nv = nn[0] * ax_ + nn[1] * ay_ + nn[2] * az_;
-            const double vg = (ax_ * gx + ay_ * gy + az_ * gz) / nv;
+            const double nv = nn[0] * vx + nn[1] * vy + nn[2] * vz;
+            const double vg = (vx * gx + vy * gy + vz * gz) / nv;
             Ax = gx - nn[0] * vg;  // P^T g
             Ay = gy - nn[1] * vg;
             Az = gz - nn[2] * vg;
@@ -152,25 +169,38 @@ __global__ void __launch_bounds__(128) k_backward(const DevParticles p, int64_t 
             by = sdt * Ay;
             bz = sdt * Az;
         } else {
-            double nh[3];
-            if (c.model != SPG_COLL_NONE && collided(c, id, c.step + k, ax_, ay_, az_, nh)) {
-                // v' = m_cp v + m_ct |v| n:  J^T a = m_cp a + m_ct v/|v| (n . a)
-                const double vm = sqrt(ax_ * ax_ + ay_ * ay_ + az_ * az_);
-                const double na = (nh[0] * Vx + nh[1] * Vy + nh[2] * Vz) * c.mass_ct / vm;
-                Vx = c.mass_cp * Vx + na * ax_;
-                Vy = c.mass_cp * Vy + na * ay_;
-                Vz = c.mass_cp * Vz + na * az_;
+            if (c.model != SPG_COLL_NONE) {
+                const uint64_t step = uint64_t(c.step) + uint64_t(k);
+                if (uint32_t(step >> 4) != cgroup) {
+                    cgroup = uint32_t(step >> 4);
+                    cmask = candidate_mask(candidate_block(step, id, c.seed_lo, c.seed_hi));
+                }
+                const bool cand = (cmask >> (uint32_t(step) & 15u)) & 1u;
+                const float rx = reach(vx, h0.x), ry = reach(vy, h0.y), rz = reach(vz, h1.x);
+                if (cand || !(fmaf(rz, rz, fmaf(ry, ry, rx * rx)) * (1.0f + 1e-5f) <= c.v2_cand_f)) {
+                    pushed();
+                    const float fx = hi_float(vx), fy = hi_float(vy), fz = hi_float(vz);
+                    const float v2 = fmaf(fz, fz, fmaf(fy, fy, fx * fx));
+                    if ((cand || !(v2 <= c.v2_cand_f)) && !no_collision_sure(c, id, step, cand, v2) &&
+                        collision_test64(c, id, step, cand ? 0u : 1u, v2, vx, vy, vz)) {
+                        double V[3] = {Vx, Vy, Vz};
+                        collision_adjoint(c, id, step, vx, vy, vz, V);
+                        Vx = V[0];
+                        Vy = V[1];
+                        Vz = V[2];
+                    }
+                }
             }
-            bx = Vx + c.dt * Ax;
-            by = Vy + c.dt * Ay;
-            bz = Vz + c.dt * Az;
+            bx = fma(c.dt, Ax, Vx);
+            by = fma(c.dt, Ay, Vy);
+            bz = fma(c.dt, Az, Vz);
         }
         // v_a = v + c E is continuous in E, also where E = 0 skipped the push
         if (t != run) {
             if (run >= 0) {
-                atomicAdd(gE + 3 * run, cq * sx);
-                atomicAdd(gE + 3 * run + 1, cq * sy);
-                atomicAdd(gE + 3 * run + 2, cq * sz);
+                atomicAdd(gE + 3 * run, sx);
+                atomicAdd(gE + 3 * run + 1, sy);
+                atomicAdd(gE + 3 * run + 2, sz);
             }
             run = t;
             sx = sy = sz = 0.0;
@@ -181,7 +211,7 @@ __global__ void __launch_bounds__(128) k_backward(const DevParticles p, int64_t 
         Vx = bx;
         Vy = by;
         Vz = bz;
-        if (G && !R.ezero) {
+        if (G && push) {
             // the pushed velocity depends on the position through the recovered
             // field: abar_x += cq G^T abar_va, G[3 d + c] = dE_d / dx_c
             const double *g = G + 9 * int64_t(t);
@@ -191,9 +221,9 @@ __global__ void __launch_bounds__(128) k_backward(const DevParticles p, int64_t 
         }
     }
     if (run >= 0) {
-        atomicAdd(gE + 3 * run, cq * sx);
-        atomicAdd(gE + 3 * run + 1, cq * sy);
-        atomicAdd(gE + 3 * run + 2, cq * sz);
+        atomicAdd(gE + 3 * run, sx);
+        atomicAdd(gE + 3 * run + 1, sy);
+        atomicAdd(gE + 3 * run + 2, sz);
     }
     ax[3 * i] = Ax;
     ax[3 * i + 1] = Ay;
@@ -250,12 +280,13 @@ __global__ void k_tet_field_gradient(const int4 *__restrict__ tet_nodes, const T
     for (int q = 0; q < 9; ++q) G[9 * t + q] = g[q];
 }
 
-// dJ/dphi from dJ/dE: E = -sum_r (phi_{r+1} - phi_0) M_r.
+// dJ/dphi from dJ/dE = cq gE (gE: the sums of abar_va, cq = q dt / m):
+// E = -sum_r (phi_{r+1} - phi_0) M_r.
 __global__ void k_gE_to_nodes(const int4 *__restrict__ tet_nodes, const TetRec *__restrict__ rec,
-                              const double *__restrict__ gE, int64_t nt, double *__restrict__ lam) {
+                              const double *__restrict__ gE, double cq, int64_t nt, double *__restrict__ lam) {
     const int64_t t = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
     if (t >= nt) return;
-    const double a0 = gE[3 * t], a1 = gE[3 * t + 1], a2 = gE[3 * t + 2];
+    const double a0 = cq * gE[3 * t], a1 = cq * gE[3 * t + 1], a2 = cq * gE[3 * t + 2];
     if (a0 == 0.0 && a1 == 0.0 && a2 == 0.0) return;
     const int4 tn = tet_nodes[t];
     const TetRec &r = rec[t];
@@ -311,6 +342,23 @@ __global__ void k_set_dirichlet(const uint8_t *__restrict__ is_dir, const double
     phi[i] = g[i];
 }
 
+// A particle set's state from src to dst; of a dead particle only the id word,
+// which is all that marks it (a checkpoint window skips it).
+__global__ void k_copy_alive(const DevParticles src, DevParticles dst, int64_t n) {
+    const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const uint32_t idf = src.idf[i];
+    dst.idf[i] = idf;
+    if (idf & kDead) return;
+    dst.x[i] = src.x[i];
+    dst.y[i] = src.y[i];
+    dst.z[i] = src.z[i];
+    dst.vx[i] = src.vx[i];
+    dst.vy[i] = src.vy[i];
+    dst.vz[i] = src.vz[i];
+    dst.tet[i] = src.tet[i];
+}
+
 __global__ void k_gather_adj(const DevParticles p, int64_t n, const double *__restrict__ ax,
                              const double *__restrict__ av, double *dx, double *dv) {
     const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
@@ -326,22 +374,26 @@ inline unsigned grid_for(int64_t n, int b) { return unsigned((n + b - 1) / b); }
 
 }  // namespace
 
+void launch_copy_alive(const DevParticles &src, const DevParticles &dst, int64_t n, cudaStream_t s) {
+    if (n > 0) k_copy_alive<<<grid_for(n, 256), 256, 0, s>>>(src, dst, n);
+}
+
 void launch_objective(const DevParticles &p, int64_t n, const LandRec *land, const double *target, double sigma,
                       double *gr, double *sums, cudaStream_t s) {
     if (n > 0)
         k_objective<<<grid_for(n, 256), 256, 0, s>>>(p, n, land, target[0], target[1], target[2],
                                                       1.0 / (2.0 * sigma * sigma), gr, sums);
 }
-void launch_backward(const DevParticles &p, int64_t n, const AdjHist &h, int k0, int k1, const TetRec *rec,
+void launch_backward(const DevParticles &p, int64_t n, const HistRec *h, int k0, int k1, const TetRec *rec,
                      const LandRec *land, const double *gr, double gscale, double *ax, double *av, double *gE,
                      const StepConst &c, cudaStream_t s, const double *G) {
     if (n > 0)
         k_backward<<<grid_for(n, 128), 128, 0, s>>>(p, n, h, k0, k1, rec, land, gr, gscale, ax, av, gE, c,
                                                      c.charge / c.mass * c.dt, G);
 }
-void launch_gE_to_nodes(const int4 *tet_nodes, const TetRec *rec, const double *gE, int64_t nt, double *lam,
+void launch_gE_to_nodes(const int4 *tet_nodes, const TetRec *rec, const double *gE, double cq, int64_t nt, double *lam,
                         cudaStream_t s) {
-    k_gE_to_nodes<<<grid_for(nt, 256), 256, 0, s>>>(tet_nodes, rec, gE, nt, lam);
+    k_gE_to_nodes<<<grid_for(nt, 256), 256, 0, s>>>(tet_nodes, rec, gE, cq, nt, lam);
 }
 void launch_adj_rhs(const double *lam, const uint8_t *is_dir, double *b, double *x, int64_t nn, cudaStream_t s) {
     k_adj_rhs<<<grid_for(nn, 256), 256, 0, s>>>(lam, is_dir, b, x, nn);

@@ -894,9 +894,10 @@ __global__ void k_record32(DevParticles32 p, int64_t n, AdjHist h, int k) {
     if (i >= n) return;
     const int64_t o = int64_t(k) * n + i;
     h.tet[o] = (p.idf[i] & kDead) ? -1 : p.tet[i];
-    h.vx[o] = double(p.vx[i]);
-    h.vy[o] = double(p.vy[i]);
-    h.vz[o] = double(p.vz[i]);
+    // FP32 velocities in the record's arrays (a conversion issues on the FP64 pipe)
+    reinterpret_cast<float *>(h.vx)[o] = p.vx[i];
+    reinterpret_cast<float *>(h.vy)[o] = p.vy[i];
+    reinterpret_cast<float *>(h.vz)[o] = p.vz[i];
 }
 
 // dg/dr of each landed particle (r = centroid + local position, in FP64) and
@@ -949,11 +950,14 @@ __global__ void __launch_bounds__(128) k_backward32(MixedArgs a, AdjHist h, int 
     const double mcp = double(c.mass_cp_f), mct = double(c.mass_ct_f);
     int run = -1;
     double sx = 0.0, sy = 0.0, sz = 0.0;
+    const float *hvx = reinterpret_cast<const float *>(h.vx), *hvy = reinterpret_cast<const float *>(h.vy),
+                *hvz = reinterpret_cast<const float *>(h.vz);
+    uint32_t cmask = 0u, cgroup = ~0u;  // candidate steps of the current sixteen-step group
     for (int k = min(k1 - 1, N); k >= k0; --k) {
         const int64_t o = int64_t(k - k0) * n + i;
         const int t = h.tet[o];
         if (t < 0) continue;
-        float vx = float(h.vx[o]), vy = float(h.vy[o]), vz = float(h.vz[o]);
+        float vx = hvx[o], vy = hvy[o], vz = hvz[o];
         if (fmaf(vz, vz, fmaf(vy, vy, vx * vx)) < vmin * vmin) continue;  // the step did not move it
         const TetRec32 &R = a.rec[t];
         if (!(R.ezero & kRecEzero)) {
@@ -961,9 +965,9 @@ __global__ void __launch_bounds__(128) k_backward32(MixedArgs a, AdjHist h, int 
             vy = (vy + R.H[1]) + R.H[1];
             vz = (vz + R.H[2]) + R.H[2];
         }
-        const double wx = vx, wy = vy, wz = vz;  // pushed velocity, as the forward had it
         double bx, by, bz;
         if (k == N) {
+            const double wx = vx, wy = vy, wz = vz;  // pushed velocity, as the forward had it
             const double *M = a.rec64[L.tet].M;  // exit-face normal from the FP64 map
             double nn[3];
             for (int q = 0; q < 3; ++q)
@@ -981,8 +985,14 @@ __global__ void __launch_bounds__(128) k_backward32(MixedArgs a, AdjHist h, int 
         } else {
             float xc, xs, cp, sp;
             const uint64_t sk = uint64_t(c.step + k);
+            if (c.model != SPG_COLL_NONE && uint32_t(sk >> 4) != cgroup) {
+                cgroup = uint32_t(sk >> 4);
+                cmask = candidate_mask(candidate_block(sk, id, c.seed_lo, c.seed_hi));
+            }
             if (c.model != SPG_COLL_NONE &&
-                collision_event32(c, id, sk, is_candidate(c, id, sk), speed2(vx, vy, vz), xc, xs, cp, sp)) {
+                collision_event32(c, id, sk, (cmask >> (uint32_t(sk) & 15u)) & 1u, speed2(vx, vy, vz), xc, xs, cp,
+                                  sp)) {
+                const double wx = vx, wy = vy, wz = vz;
                 // v' = m_cp v + m_ct |v| n:  J^T a = m_cp a + m_ct v/|v| (n . a)
                 const double vm = sqrt(wx * wx + wy * wy + wz * wz);
                 const double na = (double(xs * cp) * Vx + double(xs * sp) * Vy + double(xc) * Vz) * mct / vm;
@@ -996,9 +1006,9 @@ __global__ void __launch_bounds__(128) k_backward32(MixedArgs a, AdjHist h, int 
         }
         if (t != run) {
             if (run >= 0) {
-                atomicAdd(gE + 3 * run, cq * sx);
-                atomicAdd(gE + 3 * run + 1, cq * sy);
-                atomicAdd(gE + 3 * run + 2, cq * sz);
+                atomicAdd(gE + 3 * run, sx);
+                atomicAdd(gE + 3 * run + 1, sy);
+                atomicAdd(gE + 3 * run + 2, sz);
             }
             run = t;
             sx = sy = sz = 0.0;
@@ -1019,9 +1029,9 @@ __global__ void __launch_bounds__(128) k_backward32(MixedArgs a, AdjHist h, int 
         }
     }
     if (run >= 0) {
-        atomicAdd(gE + 3 * run, cq * sx);
-        atomicAdd(gE + 3 * run + 1, cq * sy);
-        atomicAdd(gE + 3 * run + 2, cq * sz);
+        atomicAdd(gE + 3 * run, sx);
+        atomicAdd(gE + 3 * run + 1, sy);
+        atomicAdd(gE + 3 * run + 2, sz);
     }
     ax[3 * i] = Ax;
     ax[3 * i + 1] = Ay;
@@ -1029,6 +1039,22 @@ __global__ void __launch_bounds__(128) k_backward32(MixedArgs a, AdjHist h, int 
     av[3 * i] = Vx;
     av[3 * i + 1] = Vy;
     av[3 * i + 2] = Vz;
+}
+
+// A particle set's state from src to dst; of a dead particle only the id word.
+__global__ void k_copy_alive32(DevParticles32 src, DevParticles32 dst, int64_t n) {
+    const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const uint32_t idf = src.idf[i];
+    dst.idf[i] = idf;
+    if (idf & kDead) return;
+    dst.x[i] = src.x[i];
+    dst.y[i] = src.y[i];
+    dst.z[i] = src.z[i];
+    dst.vx[i] = src.vx[i];
+    dst.vy[i] = src.vy[i];
+    dst.vz[i] = src.vz[i];
+    dst.tet[i] = src.tet[i];
 }
 
 __global__ void k_gather_adj32(DevParticles32 p, int64_t n, const double *__restrict__ ax,
@@ -1126,6 +1152,10 @@ void launch_deposit32(const DevParticles32 &p, int64_t n, const MeshDev32 &m, in
     const DepSrc32 src{p, m.rec, k, 1LL << k};
     const unsigned grid = unsigned(std::min<int64_t>(grid_for(n, kDepThreads), blocks));
     k_deposit32<<<grid, kDepThreads, 0, s>>>(src, n, m.tet_nodes, node_fix, occ);
+}
+
+void launch_copy_alive32(const DevParticles32 &src, const DevParticles32 &dst, int64_t n, cudaStream_t s) {
+    if (n > 0) k_copy_alive32<<<grid_for(n, 256), 256, 0, s>>>(src, dst, n);
 }
 
 void launch_record32(const DevParticles32 &p, int64_t n, const AdjHist &h, int k, cudaStream_t s) {

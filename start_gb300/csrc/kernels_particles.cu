@@ -18,6 +18,7 @@
 #include <cstdio>
 
 #include "philox.h"
+#include "collide64.cuh"
 #include "deposit.cuh"
 #include "field.cuh"
 #include "exact_div.h"
@@ -29,7 +30,6 @@ namespace spg {
 
 namespace {
 
-constexpr double kPi = 3.14159265358979323846;
 constexpr unsigned kFull = 0xffffffffu;
 
 enum WalkStatus { W_INSIDE = 0, W_SURFACE = 1, W_EXIT = 2, W_CAP = 3 };
@@ -241,21 +241,6 @@ __device__ __forceinline__ WalkOut walk64(const MeshDev &m, int t, double p0x, d
     }
 }
 
-// Collision probability exactly as the reference evaluates it:
-// HSModel.cpp:12-15, VHSModel.cpp:14-25 (and VSSModel.cpp, same formula).
-__device__ __noinline__ double probability64(const StepConst &c, double vx, double vy, double vz) {
-    const double vmod = sqrt(vx * vx + vy * vy + vz * vz);
-    double sigma;
-    if (c.model == SPG_COLL_HS) {
-        sigma = c.sigma_hs;
-    } else {
-        const double base = c.two_kT / ((c.mr * vmod) * vmod);
-        const double d2 = c.vhs_c1 * pow(base, c.expo);
-        sigma = kPi * d2;
-    }
-    return ((sigma * vmod) * c.gas_n) * c.dt;
-}
-
 // Post-collision velocity (HSModel.cpp:24-39, VHSModel.cpp:31-46,
 // VSSModel.cpp:32-48): stationary target; v' = m_p/(m_p+m_t) v + |m_t/(m_p+m_t) v| n.
 // The azimuth phi = 2 pi u2 enters as cospi(2 u2), sinpi(2 u2) (no argument
@@ -294,64 +279,6 @@ __device__ __noinline__ void scatter64(const StepConst &c, double u1, double u2,
     vx = ex + cmx;
     vy = ey + cmy;
     vz = ez + cmz;
-}
-
-// Gas collision decision (the candidate-byte test of philox.h) and
-// scattering, bit-exact with the FP64 test and decided mostly in FP32:
-//  * a step that is no candidate (255 of 256) with v^2 at most c.v2_cand_f,
-//    computed from the 20-bit components (below the true v^2), has P below
-//    q: no collision, no FP64 instruction;
-//  * otherwise P_f = kp (v^2)^pexp from the 20-bit components (relative
-//    error below 2e-5) decides P against q outside the band q (1 -+ 1e-4),
-//    a candidate's u_acc against 256 P outside 256 P_f (1 -+ 1e-4), and
-//    u_f against (P - q) / (1 - q) outside a band of 3e-5 P_f + 2e-7;
-//  * P is computed in FP64 only inside a band.
-// The test where the common case cannot decide it: a candidate, or P that
-// may exceed q (out of line, so the step loop carries none of it).
-__device__ __noinline__ bool collision_test64(const StepConst &c, uint32_t id, uint64_t step, uint32_t byte, float v2,
-                                              double vx, double vy, double vz) {
-    constexpr float qf = float(kCandQ);
-    const float pf = c.kp_f * exp2f(c.pexp_f * log2f(v2));
-    if (byte == 0u) {
-        // a candidate: P > q collides; P <= q collides iff u_acc < 256 P
-        if (pf > qf * (1.0f + 1e-4f)) return true;
-        const Philox4 r = collision_draw(step, 3u, id, c.seed_lo, c.seed_hi);
-        if (pf < qf * (1.0f - 1e-4f)) {
-            const float ulo = float(r.v[0] >> 8) * 5.9604644775390625e-8f;  // 2^-24
-            const float uhi = ulo + 5.9604644775390625e-8f;
-            const float a = pf * 256.0f;
-            if (uhi < a * (1.0f - 1e-4f)) return true;
-            if (ulo > a * (1.0f + 1e-4f)) return false;
-        }
-        const double P = probability64(c, vx, vy, vz);
-        return P > kCandQ || u01_from(r.v[0], r.v[1]) < P * 256.0;
-    }
-    if (pf < qf * (1.0f - 1e-4f)) return false;
-    const Philox4 r = collision_draw(step, 4u, id, c.seed_lo, c.seed_hi);
-    const float ulo = float(r.v[0] >> 8) * 5.9604644775390625e-8f;  // 2^-24
-    const float uhi = ulo + 5.9604644775390625e-8f;
-    const float tf = (pf - qf) / (1.0f - qf), band = 3e-5f * pf + 2e-7f;
-    if (pf > qf * (1.0f + 1e-4f) && uhi < tf - band) return true;
-    if (pf > qf * (1.0f + 1e-4f) && ulo > tf + band) return false;
-    const double P = probability64(c, vx, vy, vz);
-    return P > kCandQ && u01_from(r.v[0], r.v[1]) < (P - kCandQ) / (1.0 - kCandQ);
-}
-
-// The FP32 screens of collision_test64 that rule a collision out: for a
-// candidate (P certainly below q) u_acc certainly beyond 256 P; else P
-// certainly below q, or u_f certainly beyond its threshold (fast particles in
-// a dense gas, where P exceeds q in every step). False: not certain.
-__device__ __forceinline__ bool no_collision_sure(const StepConst &c, uint32_t id, uint64_t step, bool cand, float v2) {
-    constexpr float qf = float(kCandQ);
-    const float pf = c.kp_f * exp2f(c.pexp_f * log2f(v2));
-    const bool below = pf < qf * (1.0f - 1e-4f);
-    if (!cand && below) return true;
-    if (cand && !below) return false;
-    const uint32_t u = collision_draw(step, cand ? 3u : 4u, id, c.seed_lo, c.seed_hi).v[0] >> 8;
-    const float ulo = float(u) * 5.9604644775390625e-8f;  // 2^-24
-    if (cand) return ulo > pf * 256.0f * (1.0f + 1e-4f);
-    const float tf = (pf - qf) / (1.0f - qf), band = 3e-5f * pf + 2e-7f;
-    return pf > qf * (1.0f + 1e-4f) && ulo > tf + band;
 }
 
 __device__ __forceinline__ unsigned long long warp_sum(unsigned v) { return __reduce_add_sync(kFull, v); }
@@ -470,7 +397,7 @@ struct Seg64 {
     unsigned int *tri_count;
     DevCounters *ctr;
     LandRec *land;     // nullable: landing records (adjoint)
-    AdjHist hist;      // tet nullptr: none; else tet and velocity at the start of every alive step
+    HistRec *hist;     // nullable: tet and velocity at the start of every alive step
     int64_t hist_n;    // particles of a history plane
     int L;
     uint32_t seq;
@@ -735,11 +662,9 @@ __global__ void __launch_bounds__(128, 4) k_seg64(const __grid_constant__ Seg64 
         bool done = false;
         if (have) {
             if constexpr (HIST) {
-                const int64_t o = int64_t(j) * a.hist_n + i;
-                a.hist.tet[o] = tet;
-                a.hist.vx[o] = vx;
-                a.hist.vy[o] = vy;
-                a.hist.vz[o] = vz;
+                double2 *o = reinterpret_cast<double2 *>(a.hist + int64_t(j) * a.hist_n + i);
+                o[0] = make_double2(vx, vy);
+                o[1] = make_double2(vz, __hiloint2double(0, tet));
             }
             ++processed;
             // |v| < vmin: certainly false when some |v_k| >= 2 vmin (bit compare of
@@ -1273,7 +1198,7 @@ inline unsigned grid_for(int64_t n, int block) { return unsigned((n + block - 1)
 
 void launch_segment64(const DevParticles &p, int64_t n, const MeshDev &m, const StepConst &c, int L,
                       unsigned int *tri_count, DevCounters *ctr, const FieldArgs &f, uint32_t seq, cudaStream_t s,
-                      LandRec *land, const AdjHist *hist, int64_t hist_n) {
+                      LandRec *land, HistRec *hist, int64_t hist_n) {
     if (n <= 0 || L <= 0) return;
     Seg64 a{};
     a.m = m;
@@ -1282,7 +1207,7 @@ void launch_segment64(const DevParticles &p, int64_t n, const MeshDev &m, const 
     a.tri_count = tri_count;
     a.ctr = ctr;
     a.land = land;
-    if (hist) a.hist = *hist;
+    a.hist = hist;
     a.hist_n = hist_n;
     a.L = L;
     a.seq = seq;

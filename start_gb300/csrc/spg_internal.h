@@ -166,20 +166,31 @@ struct LandRec {
     double s;
 };
 
-// Per-step record of a checkpoint window (adjoint recompute): tet (-1 when
-// the particle is dead) and velocity at the start of each step, [k][i].
+// Per-step record of a checkpoint window (adjoint recompute), [k][i]: tet and
+// velocity at the start of each step. FP64 form: one sector per particle and
+// step, written by the step kernel while the particle is alive (no entry
+// afterwards: the backward pass reads a landed particle's steps up to its
+// landing only).
+struct alignas(32) HistRec {
+    double vx, vy, vz;
+    int32_t tet, pad;
+};
+// Mixed form: separate arrays, the velocities as FP32 words; tet -1 when the
+// particle is dead.
 struct AdjHist {
     int32_t *tet;
     double *vx, *vy, *vz;
 };
 
 // kernels_adjoint.cu
+// Checkpoint of a particle set (dead particles: their id word only).
+void launch_copy_alive(const DevParticles &src, const DevParticles &dst, int64_t n, cudaStream_t s);
 void launch_objective(const DevParticles &p, int64_t n, const LandRec *land, const double *target, double sigma,
                       double *gr, double *sums, cudaStream_t s);
 // G (nullable): per-tet gradient of the recovered field (launch_field_gradient);
 // with it the position adjoint also carries the push's dependence on the
 // particle's position.
-void launch_backward(const DevParticles &p, int64_t n, const AdjHist &h, int k0, int k1, const TetRec *rec,
+void launch_backward(const DevParticles &p, int64_t n, const HistRec *h, int k0, int k1, const TetRec *rec,
                      const LandRec *land, const double *gr, double gscale, double *ax, double *av, double *gE,
                      const StepConst &c, cudaStream_t s, const double *G = nullptr);
 // G[9 t + 3 d + c] = dE_d/dx_c of the continuous field whose nodal values are
@@ -187,7 +198,8 @@ void launch_backward(const DevParticles &p, int64_t n, const AdjHist &h, int k0,
 // Wn (nn) are scratch.
 void launch_field_gradient(const int4 *tet_nodes, const TetRec *rec, const double *E, int64_t nt, int64_t nn,
                            double *En, double *Wn, double *G, cudaStream_t s);
-void launch_gE_to_nodes(const int4 *tet_nodes, const TetRec *rec, const double *gE, int64_t nt, double *lam,
+// lam (zeroed by the caller) += the transpose of E = -grad phi applied to cq gE, gE the backward pass's sums.
+void launch_gE_to_nodes(const int4 *tet_nodes, const TetRec *rec, const double *gE, double cq, int64_t nt, double *lam,
                         cudaStream_t s);
 void launch_adj_rhs(const double *lam, const uint8_t *is_dir, double *b, double *x, int64_t nn, cudaStream_t s);
 void launch_dirichlet_grad(const double *lam, const uint8_t *is_dir, const int32_t *er, const int32_t *ec,
@@ -211,11 +223,11 @@ struct OccList {
 // Kernel launchers (kernels_particles.cu).
 // Steps c.step .. c.step + L - 1 of the FP64 form in one launch. seq: a stamp
 // above every one set before (field writes of this launch); land (nullable)
-// receives the landing records; hist (nullable): tet and velocity at the start
-// of every step in which a particle is alive, step j at [j hist_n + i].
+// receives the landing records; hist (nullable): the record of every step in
+// which a particle is alive, step j at [j hist_n + i].
 void launch_segment64(const DevParticles &p, int64_t n, const MeshDev &m, const StepConst &c, int L,
                       unsigned int *tri_count, DevCounters *ctr, const FieldArgs &f, uint32_t seq, cudaStream_t s,
-                      LandRec *land = nullptr, const AdjHist *hist = nullptr, int64_t hist_n = 0);
+                      LandRec *land = nullptr, HistRec *hist = nullptr, int64_t hist_n = 0);
 // TetRec::interior of every tet: all four nodes inside [lo, hi] by margin.
 void launch_interior_flags(TetRec *rec, const int4 *tet_nodes, const double *node_xyz, int64_t n_tets,
                            const double *lo, const double *hi, double margin, cudaStream_t s);
@@ -336,6 +348,7 @@ int launch_segment32(const DevParticles32 &p, int64_t n, const MeshDev32 &m, con
                      const FieldArgs &f, cudaStream_t s);
 
 // adjoint of the FP32 form (kernels_mixed.cu)
+void launch_copy_alive32(const DevParticles32 &src, const DevParticles32 &dst, int64_t n, cudaStream_t s);
 void launch_record32(const DevParticles32 &p, int64_t n, const AdjHist &h, int k, cudaStream_t s);
 void launch_objective32(const DevParticles32 &p, int64_t n, const MeshDev32 &m, const LandRec *land,
                         const double *target, double sigma, double *gr, double *sums, cudaStream_t s);
