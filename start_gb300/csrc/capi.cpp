@@ -16,6 +16,9 @@
 #include <string>
 #include <vector>
 
+#include <sys/mman.h>
+#include <unistd.h>
+
 #include "pcg_resident.h"
 #include "spg_internal.h"
 
@@ -303,6 +306,23 @@ void *device_writable(const void *p) {
     if (a.type == cudaMemoryTypeHost && a.devicePointer) return a.devicePointer;
     if (a.type == cudaMemoryTypeManaged) return const_cast<void *>(p);
     return nullptr;
+}
+
+// Maps the pages of a result array (its contents stay): a copy from the device
+// into pages never touched faults them in one by one over the C2C link, 38 ms
+// for 48 MB of fresh numpy arrays, and mapping them takes 1 ms. Not by touching
+// them: a read maps the zero page, and its replacement by the write that follows
+// is announced to the GPU page by page (18 ms). Called while the device still
+// computes what is to be copied; small results are not worth the call.
+void map_pages(void *p, size_t bytes) {
+    if (!p || bytes < (size_t(1) << 20)) return;
+#ifndef MADV_POPULATE_WRITE
+#define MADV_POPULATE_WRITE 23
+#endif
+    const uintptr_t page = uintptr_t(sysconf(_SC_PAGESIZE));
+    const uintptr_t a = reinterpret_cast<uintptr_t>(p) / page * page;
+    const uintptr_t e = (reinterpret_cast<uintptr_t>(p) + bytes + page - 1) / page * page;
+    madvise(reinterpret_cast<void *>(a), e - a, MADV_POPULATE_WRITE);  // a kernel without it: nothing happens
 }
 
 int io_stage(spg_handle *h, int64_t n, IoStage &st) {
@@ -2186,6 +2206,10 @@ int spg_get_particles(spg_handle *h, int64_t n, double *pos, double *vel, int32_
     else
         launch_gather_by_id(h->P[h->cur], n, st.slot, dpos, dvel, dtet, dfl, s);
     CK(cudaGetLastError());
+    map_pages(pos, sizeof(double) * 3 * size_t(n));
+    map_pages(vel, sizeof(double) * 3 * size_t(n));
+    map_pages(tet, sizeof(int32_t) * size_t(n));
+    map_pages(flags, sizeof(uint32_t) * size_t(n));
     if (pos) CK(cudaMemcpyAsync(pos, dpos, sizeof(double) * 3 * n, cudaMemcpyDeviceToHost, s));
     if (vel) CK(cudaMemcpyAsync(vel, dvel, sizeof(double) * 3 * n, cudaMemcpyDeviceToHost, s));
     if (tet) CK(cudaMemcpyAsync(tet, dtet, sizeof(int32_t) * n, cudaMemcpyDeviceToHost, s));
@@ -2406,6 +2430,7 @@ int spg_get_efield(spg_handle *h, double *E) {
         CK(cudaGetLastError());
         h->field_full = true;
     }
+    map_pages(E, sizeof(double) * 3 * size_t(h->n_tets));
     CK(cudaMemcpyAsync(E, h->efield, sizeof(double) * 3 * h->n_tets, cudaMemcpyDeviceToHost, h->stream));
     CK(cudaStreamSynchronize(h->stream));
     return SPG_OK;
@@ -2927,6 +2952,9 @@ int spg_grad_backward(spg_handle *h, double *dJ_dg, double *dJ_dx0, double *dJ_d
                             h->gE, c, s, G);
         CK(cudaGetLastError());
     }
+    // the results' pages while the GPU runs the windows
+    map_pages(dJ_dx0, sizeof(double) * 3 * size_t(n));
+    map_pages(dJ_dv0, sizeof(double) * 3 * size_t(n));
     CK(cudaMemsetAsync(h->lam, 0, sizeof(double) * h->n_nodes, s));
     launch_gE_to_nodes(h->tet_nodes, h->rec, h->gE, (h->prm.charge / h->prm.mass) * h->prm.dt, h->n_tets, h->lam, s);
     launch_adj_rhs(h->lam, h->is_dir, h->b, h->mu, h->n_nodes, s);
