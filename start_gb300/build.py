@@ -51,6 +51,7 @@ def _sources():
         ("kernels_fem.cu", common_nv + ["--fmad=false"]),
         ("mesh_prep.cpp", common_cc + ["-fopenmp"]),
         ("amg_setup.cpp", common_cc + ["-O3", "-fopenmp"]),
+        ("sell_build.cpp", common_cc + ["-O3", "-fopenmp"]),
         ("capi.cpp", common_cc),
     ]
 

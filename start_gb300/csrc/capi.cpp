@@ -75,6 +75,8 @@ struct spg_handle {
     int64_t *slice_ptr = nullptr;
     int32_t *scol = nullptr;
     double *sval = nullptr;
+    int64_t *stag = nullptr;   // banded slices (band_sell32)
+    int32_t *sref = nullptr;
     int64_t sell_entries = 0;
     int64_t nnz_kept = 0;  // stiffness entries in the device format (exact zeros off the diagonal dropped)
     double *val = nullptr, *inv_diag = nullptr, *dir_value = nullptr, *lift = nullptr, *dual_vol = nullptr;
@@ -421,14 +423,20 @@ int upload_amg(spg_handle *h, const AmgHost &ah, const T *sval0, AmgDevT<T> &a) 
         std::vector<double> sv;
         const double avg = M.n ? double(M.ci.size()) / double(M.n) : 0.0;
         D.g = 0;
-        // FP64: one thread per row up to 48 entries per row, then lanes with
-        // about 12 entries each (each FP64 shuffle add of a lane group costs a
-        // full warp instruction at the FP64 rate); FP32: lanes from 12
-        // entries per row, about 4 entries per lane
-        if (sizeof(T) == 8 ? avg > 48.0 : avg > 12.0) {
-            const double per_lane = sizeof(T) == 8 ? 12.0 : 4.0;
+        // FP32: lanes from 12 entries per row, about 4 entries per lane. FP64
+        // shuffle adds cost a full warp instruction at the FP64 rate each, so
+        // large levels run one thread per row up to 48 entries and above that the
+        // fewest lanes that still fill the chip (27,117 rows of 166 entries: 8);
+        // a level of at most 8,192 rows is bound by latency and takes lanes as
+        // in FP32 (residual and restriction of 3,425 rows of 28 entries: 5.3 and
+        // 7.4 us with one thread per row, 3.1 and 2.4 with 8 lanes; of 15,365
+        // rows 6.2 against 8.0).
+        constexpr bool wide = sizeof(T) == 8;
+        const bool small = !wide || M.n <= 8192;
+        if (avg > (small ? 12.0 : 48.0)) {
             D.g = 4;
-            while (D.g < 32 && per_lane * D.g < avg) D.g *= 2;
+            while (D.g < 32 && (small ? 4.0 : 12.0) * D.g < avg) D.g *= 2;
+            while (!small && D.g > 4 && M.n * (D.g / 2) >= 131072) D.g /= 2;
             sp = M.rp;
             sc = M.ci;
             sv = M.v;
@@ -472,6 +480,9 @@ int upload_amg(spg_handle *h, const AmgHost &ah, const T *sval0, AmgDevT<T> &a) 
             D.A.slice_ptr = h->slice_ptr;
             D.A.scol = h->scol;
             D.A.sval = sval0;
+            D.A.stag = h->stag;
+            D.A.sref = h->sref;
+            D.A.g = h->stag ? kSellBanded : 0;
         } else if ((rc = up_mat(H.A, D.A))) {
             return rc;
         }
@@ -481,37 +492,17 @@ int upload_amg(spg_handle *h, const AmgHost &ah, const T *sval0, AmgDevT<T> &a) 
             CK(upload(&dv, conv(H.dinv), s));
             keep(dv);
             D.dinv = dv;
-            if ((rc = vec(&D.x[1], D.n)) || (rc = vec(&D.r, D.n)) || (rc = vec(&D.d, D.n))) return rc;
-            // degree 1 (damped Jacobi over [lam/4, lam]) on every level: on the
+            if ((rc = vec(&D.x[1], D.n)) || (rc = vec(&D.r, D.n))) return rc;
+            // the degree-1 polynomial over [lam/4, lam] on every level: on the
             // 1.03e6-node cube it needs 21 cold iterations against 22 with degree 2
             // on level 0, at 22 % fewer matrix entries per V-cycle
-            D.degree = 1;
-            const double hi = H.lam, lo = D.degree == 2 ? H.lam / 30.0 : H.lam / 4.0;
-            const double theta = 0.5 * (hi + lo), delta = 0.5 * (hi - lo);
-            const double sigma = theta / delta, rho0 = 1.0 / sigma, rho1 = 1.0 / (2.0 * sigma - rho0);
-            D.inv_theta = 1.0 / theta;
-            D.cheb_a = rho1 * rho0;
-            D.cheb_b = 2.0 * rho1 / delta;
+            D.inv_theta = 1.0 / (0.5 * (H.lam + H.lam / 4.0));
             const double nnzA = double(H.A.ci.size()), n = double(D.n);
             const double nnzP = double(H.P.ci.size()), nc = double(H.P.m);
-            if (D.degree == 2) {
-                // cheb0 4 n; three Chebyshev steps (nnz + 6 n each); residual
-                // (nnz + 3 n); restriction (nnz(P) + n + nc); prolongation
-                // (nnz(P) + 2 n + nc); vector words
-                h->amg_bytes += wv * (4.0 * n + 18.0 * n + 3.0 * n + 3.0 * n + 2.0 * nc) + wm * (4.0 * nnzA + 2.0 * nnzP);
-                h->amg_launches += 7;
-            } else if (sizeof(T) == 4) {
-                // residual from x0 = D^-1 b / theta (nnz + 3 n); restriction (nnz(P) +
-                // n + nc); prolongation onto x0 (nnz(P) + 3 n + nc); Jacobi step (nnz + 4 n)
-                h->amg_bytes += wv * (3.0 * n + n + 3.0 * n + 4.0 * n + 2.0 * nc) + wm * (2.0 * nnzA + 2.0 * nnzP);
-                h->amg_launches += 4;
-            } else {
-                // x0 = D^-1 b / theta (3 n); residual (nnz + 3 n); restriction (nnz(P) +
-                // n + nc); prolongation (nnz(P) + 2 n + nc); Jacobi step (nnz + 4 n)
-                h->amg_bytes += wv * (3.0 * n + 3.0 * n + n + 2.0 * n + 4.0 * n + 2.0 * nc) +
-                                wm * (2.0 * nnzA + 2.0 * nnzP);
-                h->amg_launches += 5;
-            }
+            // residual (nnz + 3 n); restriction with the next x0 (nnz(P) + n + 3 nc);
+            // prolongation (nnz(P) + 2 n + nc); Jacobi step (nnz + 4 n)
+            h->amg_bytes += wv * (3.0 * n + n + 2.0 * n + 4.0 * n + 4.0 * nc) + wm * (2.0 * nnzA + 2.0 * nnzP);
+            h->amg_launches += 4;
         }
         if (l > 0 && (rc = vec(&D.b, D.n))) return rc;
         if (l > 0 && (rc = vec(&D.x[0], D.n))) return rc;
@@ -551,24 +542,23 @@ int setup_amg(spg_handle *h, const HostMesh &hm) {
 // PCG setup and one iteration with the handle's preconditioner.
 void pcg_setup_any(spg_handle *h, const PcgDev &d, const double *b) {
     if (h->amg32)
-        launch_pcg_setup_amg_mixed(d, h->amgd32, b, h->r32, h->z32, h->stream);
+        launch_pcg_residual_amg(d, h->amgd32, b, h->r32, h->z32, h->stream);
     else if (h->amg)
-        launch_pcg_setup_amg(d, h->amgd, b, h->stream);
+        launch_pcg_residual_amg(d, h->amgd, b, h->stream);
     else
         launch_pcg_setup(d, b, h->stream);
 }
 void pcg_iteration_any(spg_handle *h, PcgDev &d) {
     if (h->amg32)
-        launch_pcg_iteration_amg_mixed(d, h->amgd32, h->r32, h->z32, h->stream);
+        launch_pcg_iteration_amg(d, h->amgd32, h->r32, h->z32, h->stream);
     else if (h->amg)
         launch_pcg_iteration_amg(d, h->amgd, h->stream);
     else
         launch_pcg_iteration(d, h->stream);
 }
-// (with the FP32 V-cycle the last level-0 step and r.z are one kernel where level 0 allows it)
-int pcg_rz_fused(const spg_handle *h) { return h->amg32 && amg_last_step_fusable(h->amgd32) ? 1 : 0; }
+// (a V-cycle of several levels runs its last level-0 step and r.z as one kernel)
 int pcg_iter_launches(const spg_handle *h) {
-    return (h->amg || h->amg32) ? 4 + h->amg_launches - pcg_rz_fused(h) : 3;
+    return (h->amg || h->amg32) ? 4 + h->amg_launches - (h->amg_launches > 1 ? 1 : 0) : 3;
 }
 int pcg_chunk(const spg_handle *h) { return (h->amg || h->amg32) ? 2 : kPcgChunk; }
 
@@ -763,6 +753,8 @@ PcgDev pcg_dev(spg_handle *h) {
     d.slice_ptr = h->slice_ptr;
     d.scol = h->scol;
     d.sval = h->sval;
+    d.stag = h->stag;
+    d.sref = h->sref;
     d.x = h->phi;
     d.r = h->r;
     d.z = h->z;
@@ -1108,7 +1100,7 @@ int do_solve64(spg_handle *h) {
     PcgDev d = pcg_dev(h);
     ev_begin(h, h->ev_pcg);
     pcg_setup_any(h, d, h->b);
-    h->launches += h->amg ? 2 + h->amg_launches : 1;
+    h->launches += 1;
     PcgScalars hs{};
     if (!h->pcg64_while && !h->pcg64_while_failed)
         build_pcg_while(h, [&] { pcg_iteration_any(h, d); }, &h->pcg64_while, &h->pcg64_while_failed);
@@ -1159,18 +1151,11 @@ int do_solve_mixed_amg(spg_handle *h) {
     CK(cudaMemcpyAsync(h->sc, &init, sizeof(init), cudaMemcpyHostToDevice, h->stream));
     PcgDev d = pcg_dev(h);
     ev_begin(h, h->ev_pcg);
-    const bool rotated = pcg_rotated_ok(h->amgd32);
-    if (!h->pcg_while && !h->pcg_while_failed && rotated)
-        build_pcg_while(h, [&] { launch_pcg_rotated_iteration_amg_mixed(d, h->amgd32, h->r32, h->z32, h->stream); },
-                        &h->pcg_while, &h->pcg_while_failed);
-    if (h->pcg_while) {
-        // r only; the first iteration of the graph begins with the V-cycle
-        launch_pcg_residual_amg_mixed(d, h->b, h->r32, h->stream);
-        h->launches += 1;
-    } else {
-        launch_pcg_setup_amg_mixed(d, h->amgd32, h->b, h->r32, h->z32, h->stream);
-        h->launches += 2 + h->amg_launches - pcg_rz_fused(h);
-    }
+    // (one level is a dense inverse: one or two iterations, less than a while-graph's start)
+    if (!h->pcg_while && !h->pcg_while_failed && h->amgd32.levels > 1)
+        build_pcg_while(h, [&] { pcg_iteration_any(h, d); }, &h->pcg_while, &h->pcg_while_failed);
+    pcg_setup_any(h, d, h->b);
+    h->launches += 1;
     if (h->pcg_while) {
         CK(cudaGraphLaunch(h->pcg_while, h->stream));
         if (h->defer_solves) return defer_solve(h, 1);
@@ -1185,7 +1170,7 @@ int do_solve_mixed_amg(spg_handle *h) {
     if (!h->pcg32_graph) {
         cudaGraph_t g = nullptr;
         CK(cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
-        for (int k = 0; k < chunk; ++k) launch_pcg_iteration_amg_mixed(d, h->amgd32, h->r32, h->z32, h->stream);
+        for (int k = 0; k < chunk; ++k) pcg_iteration_any(h, d);
         CK(cudaStreamEndCapture(h->stream, &g));
         CK(cudaGraphInstantiate(&h->pcg32_graph, g, 0));
         cudaGraphDestroy(g);
@@ -1625,6 +1610,13 @@ int spg_create(const spg_mesh_desc *mesh, const spg_params *params, spg_handle *
         std::vector<int32_t> sc;
         std::vector<double> sv;
         build_sell32(hm.n_nodes, hm.row_ptr.data(), hm.col.data(), hm.val.data(), sp, sc, sv);
+        std::vector<int64_t> tag;
+        std::vector<int32_t> ref;
+        // Banded slices change the order in which a row's products are added. The
+        // FP32 Jacobi iterations of the mixed form amplify that to 6e-10 of phi at
+        // rtol 1e-10, so only the AMG forms, whose FP64 recurrences do not, use them.
+        const bool amg = h->prm.preconditioner == SPG_PRECOND_AMG || h->prm.preconditioner == SPG_PRECOND_AMG_F32;
+        const bool banded = amg && 2 * band_sell32(hm.n_nodes, sp, sc, sv, tag, ref) > int64_t(sp.size()) - 1;
         h->sell_entries = int64_t(sv.size());
         h->nnz_kept = 0;
         for (int64_t r = 0; r < hm.n_nodes; ++r)
@@ -1633,6 +1625,10 @@ int spg_create(const spg_mesh_desc *mesh, const spg_params *params, spg_handle *
         CK(upload(&h->slice_ptr, sp, s));
         CK(upload(&h->scol, sc, s));
         CK(upload(&h->sval, sv, s));
+        if (banded) {
+            CK(upload(&h->stag, tag, s));
+            CK(upload(&h->sref, ref, s));
+        }
         if (h->mixed || h->prm.preconditioner == SPG_PRECOND_AMG_F32) {
             std::vector<float> sv32(sv.begin(), sv.end());
             CK(upload(&h->sval32, sv32, s));
@@ -1774,6 +1770,7 @@ int spg_destroy(spg_handle *h) {
                     h->node_q,   h->rho,      h->phi,      h->phi_prev,  h->phi_prev2,      h->b,         h->r,        h->z,         h->p,
                     h->phi_vac,  h->id_slot,  h->io_counter, h->grad_G, h->grad_En,
                     h->node_fix, h->efield,   h->tet_stamp, h->occ_list, h->occ_n, h->occ_gen,   h->slice_ptr, h->scol,   h->sval,
+                    h->stag,     h->sref,
                     h->rec32,    h->cen,      h->cen_lo,   h->sval32,   h->inv_diag32, h->e32,     h->r32,       h->z32,
                     h->p32,      h->q32,      h->partials32, h->sc32,
                     h->elim_rp,  h->elim_row, h->elim_col, h->elim_val, h->land, h->gr, h->adj_x, h->adj_v,

@@ -1,10 +1,9 @@
 // V-cycle of the smoothed-aggregation AMG preconditioner (hierarchy from
-// amg_setup.cpp). Per level: Jacobi-Chebyshev pre-smoothing from a zero
-// guess, residual, restriction R = P^T, the coarser level, prolongation, and
-// post-smoothing with the same polynomial (degree 1, damped Jacobi, or
-// degree 2, per level); the coarsest level multiplies by its dense inverse.
-// Pre- and post-smoother are the same polynomial in D^-1 A, so the V-cycle
-// is a symmetric positive definite operator and CG stays CG.
+// amg_setup.cpp). Per level: a damped Jacobi step from a zero guess, residual,
+// restriction R = P^T, the coarser level, prolongation, and the same Jacobi
+// step again; the coarsest level multiplies by its dense inverse. Pre- and
+// post-smoother are the same, so the V-cycle is a symmetric positive definite
+// operator and CG stays CG.
 // Operators with short rows are stored SELL-32 with one thread per row (level
 // 0 shares the solver's matrix); long rows (coarse operators, restriction)
 // CSR with 4-32 lanes per row. No atomics, so z = M^-1 r is deterministic.
@@ -17,64 +16,125 @@ namespace spg {
 namespace {
 
 constexpr int kT = 256;
+constexpr int kBanded = kSellBanded;
 
 // converged: 1 or 2 (plain PCG), or 3 (inner cap of the mixed form)
-// (Every V-cycle kernel starts here: pdl_sync orders it after its predecessor.)
+// (Every V-cycle kernel comes here before it reads a vector: pdl_wait orders it
+// after its predecessor.)
 __device__ __forceinline__ bool done(const PcgScalars *sc) {
     pdl_sync();
     return sc && *(volatile const int *)&sc->converged;
 }
 
-// Row `row` of M x, xf(c) = x[c]. G = 0: SELL-32, the calling thread owns
-// the row. G > 0: CSR, the G lanes of a group (lane = lane index within the
-// group) stride over the row's entries and a butterfly over the group leaves
-// the sum in every lane of the group.
-template <class T, int G, class X>
-__device__ __forceinline__ T mat_row_f(const DevSellT<T> &M, X xf, int64_t row, int lane) {
-    if constexpr (G == 0) {
-        return spmv_row_sell_f<T>(M.slice_ptr, M.scol, M.sval, xf, row);
-    } else {
-        const int64_t k0 = __ldg(M.slice_ptr + row), k1 = __ldg(M.slice_ptr + row + 1);
-        T a0 = T(0), a1 = T(0);
-        int64_t k = k0 + lane;
-        for (; k + 3 * G < k1; k += 4 * G) {  // four entries per lane in flight
-            const int32_t c0 = __ldg(M.scol + k), c1 = __ldg(M.scol + k + G);
-            const int32_t c2 = __ldg(M.scol + k + 2 * G), c3 = __ldg(M.scol + k + 3 * G);
-            const T v0 = __ldg(M.sval + k), v1 = __ldg(M.sval + k + G);
-            const T v2 = __ldg(M.sval + k + 2 * G), v3 = __ldg(M.sval + k + 3 * G);
-            const T x0 = xf(c0), x1 = xf(c1), x2 = xf(c2), x3 = xf(c3);
-            a0 = fma(v0, x0, a0);
-            a1 = fma(v1, x1, a1);
-            a0 = fma(v2, x2, a0);
-            a1 = fma(v3, x3, a1);
-        }
-        // the last (at most three) entries of this lane: their column and value
-        // loads issued together, then the gathers, then the sums
-        int32_t cr[3];
-        T vr[3], xr[3];
+// Row `row` of M x, xf(c) = x[c], in two parts: RowHead holds what does not
+// depend on x (the row's extents and its first entries) and is loaded before
+// the kernel waits for its predecessor, so that a kernel whose grid is already
+// on the chip spends its first two memory latencies while the predecessor
+// ends. The small levels are bound by those latencies: one PCG iteration with
+// the FP32 V-cycle took 41.4 us at 9,261 nodes, 75 at 132,651 and 235 at
+// 1.03e6, and takes 32.7, 62.7 and 191 with the heads, the stored x0
+// (k_restrict) and the banded level 0 (sell.cuh); with the FP64 V-cycle 50.6,
+// 113 and 330 before, 40.5, 101 and 305 now (level 0 bound by FP64 issue: 8
+// fused multiply-adds a row take 16.5 us at the measured rate).
+// G = 0 or kBanded: SELL-32, the calling thread owns the row. G > 0: CSR, the
+// G lanes of a group (lane = lane index within the group) stride over the
+// row's entries, four per lane in flight, and a butterfly over the group leaves
+// the sum in every lane of the group. Every lane of a warp joins the
+// butterflies; rows past n read nothing.
+template <class T, int G>
+struct RowHead {
+    int64_t k, k1;  // this lane's first entry, the row's end
+    int32_t c[4];
+    T v[4];
+    __device__ __forceinline__ void fetch(const DevSellT<T> &M) {
 #pragma unroll
-        for (int u = 0; u < 3; ++u) {
+        for (int u = 0; u < 4; ++u) {
             const int64_t kk = k + int64_t(u) * G;
-            cr[u] = kk < k1 ? __ldg(M.scol + kk) : -1;
-            vr[u] = kk < k1 ? __ldg(M.sval + kk) : T(0);
+            c[u] = kk < k1 ? __ldg(M.scol + kk) : -1;
+            v[u] = kk < k1 ? __ldg(M.sval + kk) : T(0);
         }
+    }
+    __device__ __forceinline__ RowHead(const DevSellT<T> &M, int64_t row, int lane, int64_t n) {
+        k = k1 = 0;
+        if (row < n) {
+            k = __ldg(M.slice_ptr + row) + lane;
+            k1 = __ldg(M.slice_ptr + row + 1);
+        }
+        fetch(M);
+    }
+    template <class X>
+    __device__ __forceinline__ T finish(const DevSellT<T> &M, X xf, int64_t, int64_t) {
+        T a0 = T(0), a1 = T(0);
+        while (true) {
+            T x[4];
+            const bool full = c[3] >= 0;  // four entries; else the lane's last ones
 #pragma unroll
-        for (int u = 0; u < 3; ++u) xr[u] = cr[u] >= 0 ? xf(cr[u]) : T(0);
+            for (int u = 0; u < 4; ++u) x[u] = c[u] >= 0 ? xf(c[u]) : T(0);
+            if (!full) {
 #pragma unroll
-        for (int u = 0; u < 3; ++u)
-            if (cr[u] >= 0) a0 = fma(vr[u], xr[u], a0);
+                for (int u = 0; u < 3; ++u)
+                    if (c[u] >= 0) a0 = fma(v[u], x[u], a0);
+                break;
+            }
+            a0 = fma(v[0], x[0], a0);
+            a1 = fma(v[1], x[1], a1);
+            a0 = fma(v[2], x[2], a0);
+            a1 = fma(v[3], x[3], a1);
+            k += 4 * G;
+            fetch(M);
+        }
         T s = a0 + a1;
 #pragma unroll
         for (int off = G / 2; off > 0; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off, G);
         return s;
     }
-}
+};
+
+template <bool Band>
+struct SellRow32 {
+    SellHead<float, Band> h;
+    __device__ __forceinline__ SellRow32(const DevSellT<float> &M, int64_t row, int, int64_t n) {
+        if (row < n) h.load(sell_of(M), row);
+    }
+    template <class X>
+    __device__ __forceinline__ float finish(const DevSellT<float> &M, X xf, int64_t row, int64_t n) {
+        return row < n ? h.finish(sell_of(M), xf, row) : 0.0f;
+    }
+};
+template <bool Band>
+struct SellRow64 {
+    __device__ __forceinline__ SellRow64(const DevSellT<double> &, int64_t, int, int64_t) {}
+    template <class X>
+    __device__ __forceinline__ double finish(const DevSellT<double> &M, X xf, int64_t row, int64_t n) {
+        if (row >= n) return 0.0;
+        if constexpr (Band)
+            return sell_row_band(sell_of(M), xf, row);
+        else
+            return sell_row_plain(sell_of(M), xf, row);
+    }
+};
+template <>
+struct RowHead<float, 0> : SellRow32<false> {
+    using SellRow32<false>::SellRow32;
+};
+template <>
+struct RowHead<float, kBanded> : SellRow32<true> {
+    using SellRow32<true>::SellRow32;
+};
+template <>
+struct RowHead<double, 0> : SellRow64<false> {
+    using SellRow64<false>::SellRow64;
+};
+template <>
+struct RowHead<double, kBanded> : SellRow64<true> {
+    using SellRow64<true>::SellRow64;
+};
 
 // Thread -> (row, lane within the row's group); `own`: this thread writes the row.
 template <int G>
 __device__ __forceinline__ void row_of(int64_t n, int64_t &row, int &lane, bool &own) {
     const int64_t t = int64_t(blockIdx.x) * kT + threadIdx.x;
-    if constexpr (G == 0) {
+    if constexpr (G <= 0) {
         row = t;
         lane = 0;
     } else {
@@ -84,116 +144,24 @@ __device__ __forceinline__ void row_of(int64_t n, int64_t &row, int &lane, bool 
     own = row < n && lane == 0;
 }
 
-// Every lane of a warp joins the group shuffles; rows past n read nothing.
-template <class T, int G, class X>
-__device__ __forceinline__ T mat_row_safe_f(const DevSellT<T> &M, X xf, int64_t row, int lane, int64_t n) {
-    if constexpr (G == 0) {
-        return row < n ? mat_row_f<T, 0>(M, xf, row, 0) : T(0);
-    } else {
-        if (row >= n) {
-            T s = T(0);
-#pragma unroll
-            for (int off = G / 2; off > 0; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off, G);
-            return s;
-        }
-        return mat_row_f<T, G>(M, xf, row, lane);
-    }
-}
-
-template <class T, int G>
-__device__ __forceinline__ T mat_row_safe(const DevSellT<T> &M, const T *__restrict__ x, int64_t row, int lane,
-                                          int64_t n) {
-    return mat_row_safe_f<T, G>(M, [x](int32_t c) { return __ldg(x + c); }, row, lane, n);
-}
-
-// The first smoothing step from x = 0, x0 = D^-1 b / theta. The FP32
-// V-cycle forms it where it is read (k_resid_j, k_prolong_j) instead of
-// storing it; the FP64 V-cycle stores it (k_jacobi0), because forming it at
-// every gathered column would triple the FP64 work of the residual.
 template <class T>
-__device__ __forceinline__ T jacobi0(const AmgLevelDevT<T> &L, const T *__restrict__ b, int64_t i) {
-    return T(L.inv_theta) * (__ldg(L.dinv + i) * __ldg(b + i));
+__device__ __forceinline__ auto plain(const T *__restrict__ x) {
+    return [x](int32_t c) { return __ldg(x + c); };
 }
 
-// x = D^-1 b / theta (degree 1, FP64 V-cycle)
-template <class T>
-__global__ void __launch_bounds__(kT) k_jacobi0(const AmgLevelDevT<T> L, const T *__restrict__ b, T *__restrict__ x,
-                                                const PcgScalars *sc) {
-    if (done(sc)) return;
-    const int64_t i = int64_t(blockIdx.x) * kT + threadIdx.x;
-    if (i < L.n) x[i] = jacobi0(L, b, i);
-}
-
-// x = d = D^-1 b / theta (first Chebyshev step from x = 0)
-template <class T>
-__global__ void __launch_bounds__(kT) k_cheb0(const AmgLevelDevT<T> L, const T *__restrict__ b, T *__restrict__ x,
-                                              const PcgScalars *sc) {
-    if (done(sc)) return;
-    const int64_t i = int64_t(blockIdx.x) * kT + threadIdx.x;
-    if (i >= L.n) return;
-    const T v = T(L.inv_theta) * (L.dinv[i] * b[i]);
-    x[i] = v;
-    L.d[i] = v;
-}
-
-// r = b - A x_in; d = ca d + cb D^-1 r; x_out = x_in + d
-template <class T, int G>
-__global__ void __launch_bounds__(kT) k_cheb_step(const AmgLevelDevT<T> L, const T *__restrict__ b,
-                                                  const T *__restrict__ xin, T *__restrict__ xout, double ca,
-                                                  double cb, const PcgScalars *sc) {
-    if (done(sc)) return;
-    int64_t i;
-    int lane;
-    bool own;
-    row_of<G>(L.n, i, lane, own);
-    const T ax = mat_row_safe<T, G>(L.A, xin, i, lane, L.n);
-    if (!own) return;
-    const T r = b[i] - ax;
-    const T d = T(ca) * L.d[i] + T(cb) * (L.dinv[i] * r);
-    L.d[i] = d;
-    xout[i] = xin[i] + d;
-}
-
+// r = b - A x_in
 template <class T, int G>
 __global__ void __launch_bounds__(kT) k_resid(const AmgLevelDevT<T> L, const T *__restrict__ b,
                                               const T *__restrict__ xin, const PcgScalars *sc) {
-    if (done(sc)) return;
     int64_t i;
     int lane;
     bool own;
     row_of<G>(L.n, i, lane, own);
-    const T ax = mat_row_safe<T, G>(L.A, xin, i, lane, L.n);
-    if (own) L.r[i] = b[i] - ax;
-}
-
-// Degree 1: r = b - A x0 with x0 = D^-1 b / theta formed at each column.
-template <class T, int G>
-__global__ void __launch_bounds__(kT) k_resid_j(const AmgLevelDevT<T> L, const T *__restrict__ b,
-                                                const PcgScalars *sc) {
+    pdl_trigger();
+    RowHead<T, G> row(L.A, i, lane, L.n);
     if (done(sc)) return;
-    int64_t i;
-    int lane;
-    bool own;
-    row_of<G>(L.n, i, lane, own);
-    const T *dinv = L.dinv;
-    const T it = T(L.inv_theta);
-    const T ax = mat_row_safe_f<T, G>(
-        L.A, [dinv, b, it](int32_t c) { return it * (__ldg(dinv + c) * __ldg(b + c)); }, i, lane, L.n);
+    const T ax = row.finish(L.A, plain(xin), i, L.n);
     if (own) L.r[i] = b[i] - ax;
-}
-
-// Degree 1: x_out = x0 + P x_coarse (x0 as in k_resid_j)
-template <class T, int G>
-__global__ void __launch_bounds__(kT) k_prolong_j(const AmgLevelDevT<T> L, const T *__restrict__ b,
-                                                  const T *__restrict__ xc, T *__restrict__ xout,
-                                                  const PcgScalars *sc) {
-    if (done(sc)) return;
-    int64_t i;
-    int lane;
-    bool own;
-    row_of<G>(L.P.n, i, lane, own);
-    const T v = mat_row_safe<T, G>(L.P, xc, i, lane, L.P.n);
-    if (own) xout[i] = jacobi0(L, b, i) + v;
 }
 
 // Degree 1 post-smoothing: x_out = x_in + D^-1 (b - A x_in) / theta
@@ -201,40 +169,56 @@ template <class T, int G>
 __global__ void __launch_bounds__(kT) k_jacobi_step(const AmgLevelDevT<T> L, const T *__restrict__ b,
                                                     const T *__restrict__ xin, T *__restrict__ xout,
                                                     const PcgScalars *sc) {
-    if (done(sc)) return;
     int64_t i;
     int lane;
     bool own;
     row_of<G>(L.n, i, lane, own);
-    const T ax = mat_row_safe<T, G>(L.A, xin, i, lane, L.n);
+    pdl_trigger();
+    RowHead<T, G> row(L.A, i, lane, L.n);
+    if (done(sc)) return;
+    const T ax = row.finish(L.A, plain(xin), i, L.n);
     if (!own) return;
     const T r = b[i] - ax;
     xout[i] = xin[i] + T(L.inv_theta) * (L.dinv[i] * r);
 }
 
-// b_next = R r
+// b_next = R r, and the next level's first smoothing step from x = 0 with it,
+// x0 = D^-1 b / theta (x0 null: the next level is the coarsest, which has
+// none). Level 0's x0 is written by the kernel that writes its b, the PCG's
+// residual: so the residual and the prolongation of every level gather and
+// read one stored vector, where forming x0 at each gathered column takes two
+// (residual of 39,764 rows of 258 entries: 18.4 us so, 13.0 us from the stored
+// vector), and no kernel is launched for it alone.
 template <class T, int G>
 __global__ void __launch_bounds__(kT) k_restrict(const DevSellT<T> R, const T *__restrict__ r, T *__restrict__ bnext,
+                                                 const T *__restrict__ dinv, T inv_theta, T *__restrict__ x0,
                                                  const PcgScalars *sc) {
-    if (done(sc)) return;
     int64_t i;
     int lane;
     bool own;
     row_of<G>(R.n, i, lane, own);
-    const T v = mat_row_safe<T, G>(R, r, i, lane, R.n);
-    if (own) bnext[i] = v;
+    pdl_trigger();
+    RowHead<T, G> row(R, i, lane, R.n);
+    const T di = own && x0 ? __ldg(dinv + i) : T(0);
+    if (done(sc)) return;
+    const T v = row.finish(R, plain(r), i, R.n);
+    if (!own) return;
+    bnext[i] = v;
+    if (x0) x0[i] = inv_theta * (di * v);
 }
 
 // x_out = x_in + P x_coarse
 template <class T, int G>
 __global__ void __launch_bounds__(kT) k_prolong(const DevSellT<T> P, const T *__restrict__ xin,
                                                 const T *__restrict__ xc, T *__restrict__ xout, const PcgScalars *sc) {
-    if (done(sc)) return;
     int64_t i;
     int lane;
     bool own;
     row_of<G>(P.n, i, lane, own);
-    const T v = mat_row_safe<T, G>(P, xc, i, lane, P.n);
+    pdl_trigger();
+    RowHead<T, G> row(P, i, lane, P.n);
+    if (done(sc)) return;
+    const T v = row.finish(P, plain(xc), i, P.n);
     if (own) xout[i] = xin[i] + v;
 }
 
@@ -260,6 +244,7 @@ inline unsigned blocks_for(int64_t n, int g = 0) {
 
 #define SPG_AMG_DISPATCH(g, KERNEL, GRIDN, ...)                                             \
     switch (g) {                                                                            \
+    case kBanded: launch_pdl(KERNEL<T, kBanded>, blocks_for(GRIDN, 0), kT, s, __VA_ARGS__); break; \
     case 4: launch_pdl(KERNEL<T, 4>, blocks_for(GRIDN, 4), kT, s, __VA_ARGS__); break;     \
     case 8: launch_pdl(KERNEL<T, 8>, blocks_for(GRIDN, 8), kT, s, __VA_ARGS__); break;     \
     case 16: launch_pdl(KERNEL<T, 16>, blocks_for(GRIDN, 16), kT, s, __VA_ARGS__); break;  \
@@ -267,8 +252,9 @@ inline unsigned blocks_for(int64_t n, int g = 0) {
     default: launch_pdl(KERNEL<T, 0>, blocks_for(GRIDN, 0), kT, s, __VA_ARGS__); break;    \
     }
 
-// skip_last: level 0's last Jacobi step (x1 = L.x[1] -> z) is left to the
-// caller, which fuses it with the PCG's r.z (FP32 degree-1 level 0 only).
+// xa holds x0 = D^-1 b / theta on entry (not on the coarsest level) and the
+// result on return. skip_last: level 0's last Jacobi step (L.x[1] -> z) is
+// left to the caller, which fuses it with the PCG's r.z.
 template <class T>
 void vcycle_level(const AmgDevT<T> &a, int l, const T *b, T *xa, const PcgScalars *sc, cudaStream_t s,
                   bool skip_last = false) {
@@ -280,48 +266,23 @@ void vcycle_level(const AmgDevT<T> &a, int l, const T *b, T *xa, const PcgScalar
     T *xb = L.x[1];
     const int ga = L.A.g;
     const AmgLevelDevT<T> &N = a.lev[l + 1];
-    if (L.degree == 1 && sizeof(T) == 4) {  // x0 = D^-1 b / theta; residual; coarse correction; damped Jacobi
-        SPG_AMG_DISPATCH(ga, k_resid_j, L.n, L, b, sc)
-        SPG_AMG_DISPATCH(L.R.g, k_restrict, L.R.n, L.R, L.r, N.b, sc)
-        vcycle_level<T>(a, l + 1, N.b, N.x[0], sc, s);
-        SPG_AMG_DISPATCH(L.P.g, k_prolong_j, L.P.n, L, b, N.x[0], xb, sc)
-        if (skip_last) return;
-        SPG_AMG_DISPATCH(ga, k_jacobi_step, L.n, L, b, xb, xa, sc)
-        return;
-    }
-    if (L.degree == 1) {
-        launch_pdl(k_jacobi0<T>, blocks_for(L.n), kT, s, L, b, xa, sc);
-        SPG_AMG_DISPATCH(ga, k_resid, L.n, L, b, xa, sc)
-        SPG_AMG_DISPATCH(L.R.g, k_restrict, L.R.n, L.R, L.r, N.b, sc)
-        vcycle_level<T>(a, l + 1, N.b, N.x[0], sc, s);
-        SPG_AMG_DISPATCH(L.P.g, k_prolong, L.P.n, L.P, xa, N.x[0], xb, sc)
-        SPG_AMG_DISPATCH(ga, k_jacobi_step, L.n, L, b, xb, xa, sc)
-        return;
-    }
-    launch_pdl(k_cheb0<T>, blocks_for(L.n), kT, s, L, b, xa, sc);
-    SPG_AMG_DISPATCH(ga, k_cheb_step, L.n, L, b, xa, xb, L.cheb_a, L.cheb_b, sc)
-    SPG_AMG_DISPATCH(ga, k_resid, L.n, L, b, xb, sc)
-    SPG_AMG_DISPATCH(L.R.g, k_restrict, L.R.n, L.R, L.r, N.b, sc)
+    T *x0 = l + 2 < a.levels ? N.x[0] : nullptr;  // the coarsest level has no smoothing
+    SPG_AMG_DISPATCH(ga, k_resid, L.n, L, b, xa, sc)
+    SPG_AMG_DISPATCH(L.R.g, k_restrict, L.R.n, L.R, L.r, N.b, N.dinv, T(N.inv_theta), x0, sc)
     vcycle_level<T>(a, l + 1, N.b, N.x[0], sc, s);
-    SPG_AMG_DISPATCH(L.P.g, k_prolong, L.P.n, L.P, xb, N.x[0], xa, sc)
-    SPG_AMG_DISPATCH(ga, k_cheb_step, L.n, L, b, xa, xb, 0.0, L.inv_theta, sc)
-    SPG_AMG_DISPATCH(ga, k_cheb_step, L.n, L, b, xb, xa, L.cheb_a, L.cheb_b, sc)
+    SPG_AMG_DISPATCH(L.P.g, k_prolong, L.P.n, L.P, xa, N.x[0], xb, sc)
+    if (skip_last) return;
+    SPG_AMG_DISPATCH(ga, k_jacobi_step, L.n, L, b, xb, xa, sc)
 }
 
 }  // namespace
 
 void launch_amg_vcycle(const AmgDev &a, const double *r, double *z, const PcgScalars *sc, cudaStream_t s) {
-    vcycle_level<double>(a, 0, r, z, sc, s);
+    vcycle_level<double>(a, 0, r, z, sc, s, a.levels > 1);
 }
 
 void launch_amg_vcycle(const AmgDev32 &a, const float *r, float *z, const PcgScalars *sc, cudaStream_t s) {
-    vcycle_level<float>(a, 0, r, z, sc, s);
-}
-
-bool amg_last_step_fusable(const AmgDev32 &a) { return a.levels > 1 && a.lev[0].degree == 1 && a.lev[0].A.g == 0; }
-
-void launch_amg_vcycle_but_last(const AmgDev32 &a, const float *r, float *z, const PcgScalars *sc, cudaStream_t s) {
-    vcycle_level<float>(a, 0, r, z, sc, s, true);
+    vcycle_level<float>(a, 0, r, z, sc, s, a.levels > 1);
 }
 
 }  // namespace spg

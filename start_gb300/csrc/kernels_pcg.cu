@@ -28,35 +28,45 @@ __device__ __forceinline__ double warp_sum(double v) {
     return v;
 }
 
-// Block sum of two values into partials[2*blockIdx.x + {0,1}]; returns true in
-// thread 0 of the last block to finish, whose totals are then in tot[0..1].
+// Sums of N values (1 or 2) over the grid: block sums to
+// partials[2 * blockIdx.x + {0, 1}]; true in thread 0 of the last block to
+// finish, whose totals are then in tot.
 // FP64 adds issue per warp at the FP64 rate, so the block sum runs in warp 0
 // only: the 256 per-thread values go through shared memory, lane l adds the
 // eight values l, l+32, ..., l+224 in that order and a five-level shuffle
-// tree finishes (a fixed order, so the sums are deterministic for a grid).
-__device__ __forceinline__ void block_sum2(double &a, double &b) {
-    __shared__ double sa[kThreads], sb[kThreads];
-    sa[threadIdx.x] = a;
-    sb[threadIdx.x] = b;
-    __syncthreads();
-    if (threadIdx.x < 32) {
-        double ta = sa[threadIdx.x], tb = sb[threadIdx.x];
+// tree finishes (a fixed order, so the sums are deterministic for a grid). A
+// second value is a chain of its own of the same length, so kernels with one
+// sum (N = 1) do not carry it.
+template <int N>
+__device__ __forceinline__ void block_sum(double (&a)[N]) {
+    __shared__ double sa[N][kThreads];
 #pragma unroll
-        for (int w = 1; w < kThreads / 32; ++w) {
-            ta += sa[threadIdx.x + 32 * w];
-            tb += sb[threadIdx.x + 32 * w];
-        }
-        a = warp_sum(ta);
-        b = warp_sum(tb);
+    for (int k = 0; k < N; ++k) sa[k][threadIdx.x] = a[k];
+    __syncthreads();
+    if (threadIdx.x < 32) {  // (the N chains interleaved)
+        double t[N];
+#pragma unroll
+        for (int k = 0; k < N; ++k) t[k] = sa[k][threadIdx.x];
+#pragma unroll
+        for (int w = 1; w < kThreads / 32; ++w)
+#pragma unroll
+            for (int k = 0; k < N; ++k) t[k] += sa[k][threadIdx.x + 32 * w];
+#pragma unroll
+        for (int off = 16; off > 0; off >>= 1)
+#pragma unroll
+            for (int k = 0; k < N; ++k) t[k] += __shfl_down_sync(kFull, t[k], off);
+#pragma unroll
+        for (int k = 0; k < N; ++k) a[k] = t[k];
     }
 }
 
-__device__ bool block_reduce2(double a, double b, double *partials, PcgScalars *sc, double tot[2]) {
+template <int N>
+__device__ bool block_reduce(double (&a)[N], double *partials, PcgScalars *sc, double (&tot)[N]) {
     __shared__ bool last;
-    block_sum2(a, b);
+    block_sum(a);
     if (threadIdx.x == 0) {
-        partials[2 * blockIdx.x] = a;
-        partials[2 * blockIdx.x + 1] = b;
+#pragma unroll
+        for (int k = 0; k < N; ++k) partials[2 * blockIdx.x + k] = a[k];
         __threadfence();
         const unsigned ticket = atomicInc(&sc->ticket, gridDim.x - 1);
         last = ticket == gridDim.x - 1;
@@ -65,21 +75,31 @@ __device__ bool block_reduce2(double a, double b, double *partials, PcgScalars *
     if (!last) return false;
     // last block: fixed-order sum of the partials
     __threadfence();
-    double ta = 0.0, tb = 0.0;
-    for (int k = threadIdx.x; k < int(gridDim.x); k += kThreads) {
-        ta += __ldcg(partials + 2 * k);
-        tb += __ldcg(partials + 2 * k + 1);
-    }
-    __syncthreads();  // the shared buffers of block_sum2 are reused
-    block_sum2(ta, tb);
-    if (threadIdx.x != 0) return false;
-    tot[0] = ta;
-    tot[1] = tb;
-    return true;
+#pragma unroll
+    for (int k = 0; k < N; ++k) tot[k] = 0.0;
+    for (int b = threadIdx.x; b < int(gridDim.x); b += kThreads)
+#pragma unroll
+        for (int k = 0; k < N; ++k) tot[k] += __ldcg(partials + 2 * b + k);
+    __syncthreads();  // the shared buffers of block_sum are reused
+    block_sum(tot);
+    return threadIdx.x == 0;
 }
 
+__device__ __forceinline__ bool block_reduce2(double a, double b, double *partials, PcgScalars *sc, double (&tot)[2]) {
+    double v[2] = {a, b};
+    return block_reduce<2>(v, partials, sc, tot);
+}
+__device__ __forceinline__ bool block_reduce1(double a, double *partials, PcgScalars *sc, double (&tot)[1]) {
+    double v[1] = {a};
+    return block_reduce<1>(v, partials, sc, tot);
+}
+
+__device__ __forceinline__ SellMat<double> sell_of(const PcgDev &d) {
+    return {d.slice_ptr, d.scol, d.sval, d.stag, d.sref};
+}
+template <bool Band>
 __device__ __forceinline__ double spmv_row(const PcgDev &d, const double *__restrict__ x, int64_t i) {
-    return spmv_row_sell<double>(d.slice_ptr, d.scol, d.sval, x, i);
+    return spmv_row_sell<Band>(sell_of(d), x, i);
 }
 
 __global__ void k_rhs(const double *__restrict__ node_q, double inv_eps0, const double *__restrict__ lift,
@@ -113,7 +133,7 @@ __global__ void __launch_bounds__(kThreads) k_setup(PcgDev d, const double *__re
     double rr = 0.0;
     for (int64_t i = int64_t(blockIdx.x) * kThreads + threadIdx.x; i < d.n; i += int64_t(gridDim.x) * kThreads) {
         const double bi = b[i];
-        const double ri = bi - spmv_row(d, d.x, i);
+        const double ri = bi - spmv_row<false>(d, d.x, i);
         const double zi = ri * d.inv_diag[i];
         d.r[i] = ri;
         d.z[i] = zi;
@@ -150,17 +170,20 @@ __global__ void __launch_bounds__(kThreads) k_setup(PcgDev d, const double *__re
 }
 
 // q = A p; pq = p.q; alpha = rz / pq
-__global__ void __launch_bounds__(kThreads) k_spmv_dot(PcgDev d) {
+template <bool Band>
+__global__ void __launch_bounds__(kThreads, 4) k_spmv_dot(PcgDev d) {
     pdl_sync();
     if (d.sc->converged) return;
     double pq = 0.0;
+#pragma unroll 1
     for (int64_t i = int64_t(blockIdx.x) * kThreads + threadIdx.x; i < d.n; i += int64_t(gridDim.x) * kThreads) {
-        const double qi = spmv_row(d, d.p, i);
+        const double pi = d.p[i];
+        const double qi = spmv_row<Band>(d, d.p, i);
         d.q[i] = qi;
-        pq += d.p[i] * qi;
+        pq += pi * qi;
     }
-    double tot[2];
-    if (block_reduce2(pq, 0.0, d.partials, d.sc, tot)) {
+    double tot[1];
+    if (block_reduce1(pq, d.partials, d.sc, tot)) {
         PcgScalars *sc = d.sc;
         sc->pq = tot[0];
         if (tot[0] > 0.0) {
@@ -213,20 +236,35 @@ __global__ void __launch_bounds__(kThreads) k_pupdate(PcgDev d) {
 }
 
 // ------------------------------------------------- PCG with the AMG V-cycle
-// M = false: the FP64 V-cycle reads r and writes z. M = true (mixed form):
+// T = double: the FP64 V-cycle reads r and writes z. T = float (mixed form):
 // the FP32 V-cycle reads r32 = float(r) and writes z32; x, r, p, q and all
 // sums stay FP64, so the solve still stops on the FP64 residual.
 
+// What the residual kernels write for the V-cycle: the FP32 copy of r (mixed
+// form) and level 0's first smoothing step x0 = D^-1 r / theta into z.
+template <class T>
+struct VcycleIn {
+    T *r;           // r32; unused in FP64
+    T *z;           // nullptr: one level only, no smoothing
+    const T *dinv;
+    T inv_theta;
+    __device__ __forceinline__ void put(int64_t i, double ri) const {
+        const T rt = T(ri);
+        if constexpr (sizeof(T) == 4) r[i] = rt;
+        if (z) z[i] = inv_theta * (__ldg(dinv + i) * rt);
+    }
+};
+
 // r = b - A x; bb = b.b, rr = r.r (z = M^-1 r follows as a V-cycle)
-template <bool M>
-__global__ void __launch_bounds__(kThreads) k_setup_amg(PcgDev d, const double *__restrict__ b, float *__restrict__ r32) {
+template <class T, bool Band>
+__global__ void __launch_bounds__(kThreads, 4) k_setup_amg(PcgDev d, const double *__restrict__ b, VcycleIn<T> v) {
     pdl_sync();
     double bb = 0.0, rr = 0.0;
     for (int64_t i = int64_t(blockIdx.x) * kThreads + threadIdx.x; i < d.n; i += int64_t(gridDim.x) * kThreads) {
         const double bi = b[i];
-        const double ri = bi - spmv_row(d, d.x, i);
+        const double ri = bi - spmv_row<Band>(d, d.x, i);
         d.r[i] = ri;
-        if constexpr (M) r32[i] = float(ri);
+        v.put(i, ri);
         bb += bi * bi;
         rr += ri * ri;
     }
@@ -245,21 +283,38 @@ __global__ void __launch_bounds__(kThreads) k_setup_amg(PcgDev d, const double *
 }
 
 // x += alpha p; r -= alpha q; rr = r.r and the stop test
-template <bool M>
-__global__ void __launch_bounds__(kThreads) k_update_amg(PcgDev d, float *__restrict__ r32) {
+template <class T>
+__global__ void __launch_bounds__(kThreads) k_update_amg(PcgDev d, VcycleIn<T> v) {
     pdl_sync();
     if (d.sc->converged) return;
     const double alpha = d.sc->alpha;
     double rr = 0.0;
-    for (int64_t i = int64_t(blockIdx.x) * kThreads + threadIdx.x; i < d.n; i += int64_t(gridDim.x) * kThreads) {
+    // pairs of elements: eight 16-byte loads' worth per thread in flight
+    const int64_t n2 = d.n >> 1;
+    for (int64_t i = int64_t(blockIdx.x) * kThreads + threadIdx.x; i < n2; i += int64_t(gridDim.x) * kThreads) {
+        double2 x = reinterpret_cast<double2 *>(d.x)[i], r = reinterpret_cast<double2 *>(d.r)[i];
+        const double2 p = reinterpret_cast<const double2 *>(d.p)[i], q = reinterpret_cast<const double2 *>(d.q)[i];
+        x.x += alpha * p.x;
+        x.y += alpha * p.y;
+        r.x -= alpha * q.x;
+        r.y -= alpha * q.y;
+        reinterpret_cast<double2 *>(d.x)[i] = x;
+        reinterpret_cast<double2 *>(d.r)[i] = r;
+        v.put(2 * i, r.x);
+        v.put(2 * i + 1, r.y);
+        rr += r.x * r.x;
+        rr += r.y * r.y;
+    }
+    if ((d.n & 1) && blockIdx.x == gridDim.x - 1 && threadIdx.x == kThreads - 1) {
+        const int64_t i = d.n - 1;
         d.x[i] += alpha * d.p[i];
         const double ri = d.r[i] - alpha * d.q[i];
         d.r[i] = ri;
-        if constexpr (M) r32[i] = float(ri);
+        v.put(i, ri);
         rr += ri * ri;
     }
-    double tot[2];
-    if (block_reduce2(rr, 0.0, d.partials, d.sc, tot)) {
+    double tot[1];
+    if (block_reduce1(rr, d.partials, d.sc, tot)) {
         PcgScalars *sc = d.sc;
         sc->iters += 1;
         sc->rr = tot[0];
@@ -270,54 +325,42 @@ __global__ void __launch_bounds__(kThreads) k_update_amg(PcgDev d, float *__rest
     }
 }
 
-// rz' = r.z (z from the V-cycle); first: p = z; else beta = rz'/rz
-template <bool M>
-__global__ void __launch_bounds__(kThreads) k_rz_amg(PcgDev d, const float *__restrict__ z32, int first) {
+// rz' = r.z with z = M^-1 r; first iteration (no update yet): p = z and beta =
+// 0, else beta = rz'/rz. Jacobi: z is the V-cycle's last level-0 step
+// z = x1 + D^-1 (r - A x1) / theta, x1 = L.x[1]; else z is read.
+template <class T, bool Jacobi, bool Band>
+__global__ void __launch_bounds__(kThreads, 4) k_rz_amg(PcgDev d, const AmgLevelDevT<T> L, const T *__restrict__ r32,
+                                                        T *__restrict__ z) {
     pdl_sync();
     if (d.sc->converged) return;
+    const bool first = d.sc->iters == 0;
+    const T *xin = L.x[1];
     double rz = 0.0;
+#pragma unroll 1
     for (int64_t i = int64_t(blockIdx.x) * kThreads + threadIdx.x; i < d.n; i += int64_t(gridDim.x) * kThreads) {
-        double zi;
-        if constexpr (M)
-            zi = double(z32[i]);
-        else
-            zi = d.z[i];
-        rz += d.r[i] * zi;
-        if (first) d.p[i] = zi;
-    }
-    double tot[2];
-    if (block_reduce2(rz, 0.0, d.partials, d.sc, tot)) {
-        PcgScalars *sc = d.sc;
-        if (!first) sc->beta = tot[0] / sc->rz;
-        sc->rz = tot[0];
-    }
-}
-
-// The V-cycle's last level-0 Jacobi step z32 = x1 + D^-1 (r32 - A x1) / theta
-// (k_jacobi_step's arithmetic) fused with k_rz_amg: rz' = r.z (FP64 r, z
-// promoted), first: p = z (and beta = 0); else beta = rz'/rz. First = 2: the
-// first iteration is the one with no update yet (sc->iters == 0).
-template <int FirstArg>
-__global__ void __launch_bounds__(kThreads) k_jacobi_rz(PcgDev d, const AmgLevelDevT<float> L,
-                                                        const float *__restrict__ r32, float *__restrict__ z32) {
-    pdl_sync();
-    if (d.sc->converged) return;
-    const bool First = FirstArg == 2 ? d.sc->iters == 0 : FirstArg == 1;
-    const float *xin = L.x[1];
-    double rz = 0.0;
-    for (int64_t i = int64_t(blockIdx.x) * kThreads + threadIdx.x; i < d.n; i += int64_t(gridDim.x) * kThreads) {
-        const float ax = spmv_row_sell<float>(L.A.slice_ptr, L.A.scol, L.A.sval, xin, i);
-        const float rr = r32[i] - ax;
-        const float zi = xin[i] + float(L.inv_theta) * (L.dinv[i] * rr);
-        z32[i] = zi;
+        const double ri = d.r[i];
+        T zi;
+        if constexpr (Jacobi) {
+            T rt;
+            if constexpr (sizeof(T) == 4)
+                rt = r32[i];
+            else
+                rt = ri;
+            const T x1 = xin[i], di = L.dinv[i];
+            const T ax = spmv_row_sell<Band>(sell_of(L.A), xin, i);
+            zi = x1 + T(L.inv_theta) * (di * (rt - ax));
+            z[i] = zi;
+        } else {
+            zi = z[i];
+        }
         const double zd = double(zi);
-        rz += d.r[i] * zd;
-        if (First) d.p[i] = zd;
+        rz += ri * zd;
+        if (first) d.p[i] = zd;
     }
-    double tot[2];
-    if (block_reduce2(rz, 0.0, d.partials, d.sc, tot)) {
+    double tot[1];
+    if (block_reduce1(rz, d.partials, d.sc, tot)) {
         PcgScalars *sc = d.sc;
-        sc->beta = First ? 0.0 : tot[0] / sc->rz;
+        sc->beta = first ? 0.0 : tot[0] / sc->rz;
         sc->rz = tot[0];
     }
 }
@@ -344,7 +387,7 @@ __global__ void __launch_bounds__(kThreads) k_pupdate_m(PcgDev d, const float *_
 // further accumulation is FP64.
 
 __device__ __forceinline__ float spmv_row32(const PcgDev32 &d, const float *__restrict__ x, int64_t i) {
-    return spmv_row_sell<float>(d.slice_ptr, d.scol, d.sval, x, i);
+    return spmv_row_sell<false>(SellMat<float>{d.slice_ptr, d.scol, d.sval, nullptr, nullptr}, x, i);
 }
 
 __device__ __forceinline__ float warp_sumf(float v) {
@@ -356,7 +399,7 @@ __device__ __forceinline__ float warp_sumf(float v) {
 // FP64 block reduction of FP32 per-thread partials: each warp sums in FP32
 // (the total lands in lane 0), only lane 0 passes it on, and everything from
 // there on is FP64.
-__device__ bool block_reduce2_w(float a, float b, double *partials, PcgScalars *sc, double tot[2]) {
+__device__ bool block_reduce2_w(float a, float b, double *partials, PcgScalars *sc, double (&tot)[2]) {
     a = warp_sumf(a);
     b = warp_sumf(b);
     const bool lead = (threadIdx.x & 31) == 0;
@@ -372,7 +415,7 @@ __global__ void __launch_bounds__(kThreads) k_refine_setup(PcgDev d, PcgDev32 f,
     __shared__ double s_rz[kThreads / 32];
     for (int64_t i = int64_t(blockIdx.x) * kThreads + threadIdx.x; i < d.n; i += int64_t(gridDim.x) * kThreads) {
         const double bi = b[i];
-        const double ri = bi - spmv_row(d, d.x, i);
+        const double ri = bi - spmv_row<false>(d, d.x, i);
         const float r32 = float(ri);
         const float z32 = r32 * f.inv_diag[i];
         f.r[i] = r32;
@@ -511,9 +554,13 @@ int wave(K kernel, int64_t n) {
 PcgGrid pcg_grid64(int64_t n) {
     PcgGrid g;
     g.setup = wave(k_setup, n);
-    g.spmv = wave(k_spmv_dot, n);
+    g.spmv = wave(k_spmv_dot<false>, n);
     g.update = wave(k_update, n);
     g.pupdate = wave(k_pupdate, n);
+    // (one grid for both types of the V-cycle: the FP64 kernels hold the fewer blocks)
+    g.setup_amg = wave(k_setup_amg<double, false>, n);
+    g.update_amg = wave(k_update_amg<double>, (n + 1) / 2);
+    g.rz = wave(k_rz_amg<double, true, false>, n);
     return g;
 }
 
@@ -534,130 +581,58 @@ void launch_pcg_setup(const PcgDev &d, const double *b, cudaStream_t s) {
     launch_pdl(k_setup, d.grid.setup, kThreads, s, d, b);
 }
 
-void launch_pcg_setup_amg(const PcgDev &d, const AmgDev &a, const double *b, cudaStream_t s) {
-    launch_pdl(k_setup_amg<false>, d.grid.setup, kThreads, s, d, b, nullptr);
-    launch_amg_vcycle(a, d.r, d.z, d.sc, s);
-    launch_pdl(k_rz_amg<false>, d.grid.update, kThreads, s, d, nullptr, 1);
+namespace {
+void launch_spmv_dot(const PcgDev &d, cudaStream_t s) {
+    launch_pdl(d.stag ? k_spmv_dot<true> : k_spmv_dot<false>, d.grid.spmv, kThreads, s, d);
 }
 
-void launch_pcg_iteration_amg(PcgDev &d, const AmgDev &a, cudaStream_t s) {
-    launch_pdl(k_spmv_dot, d.grid.spmv, kThreads, s, d);
-    launch_pdl(k_update_amg<false>, d.grid.update, kThreads, s, d, nullptr);
-    launch_amg_vcycle(a, d.r, d.z, d.sc, s);
-    launch_pdl(k_rz_amg<false>, d.grid.update, kThreads, s, d, nullptr, 0);
-    launch_pdl(k_pupdate, d.grid.pupdate, kThreads, s, d);
+template <class T>
+VcycleIn<T> vcycle_in(const AmgDevT<T> &a, T *r, T *z) {
+    return {r, a.levels > 1 ? z : nullptr, a.lev[0].dinv, T(a.lev[0].inv_theta)};
 }
-
-// z32 = M^-1 r32 and r.z: the V-cycle's last step fused with the sum where
-// level 0 allows it, else the whole V-cycle and k_rz_amg.
-static void vcycle_rz(PcgDev d, const AmgDev32 &a, float *r32, float *z32, int first, cudaStream_t s) {
-    if (amg_last_step_fusable(a)) {
-        launch_amg_vcycle_but_last(a, r32, z32, d.sc, s);
-        if (first)
-            launch_pdl(k_jacobi_rz<1>, d.grid.update, kThreads, s, d, a.lev[0], r32, z32);
-        else
-            launch_pdl(k_jacobi_rz<0>, d.grid.update, kThreads, s, d, a.lev[0], r32, z32);
-    } else {
-        launch_amg_vcycle(a, r32, z32, d.sc, s);
-        launch_pdl(k_rz_amg<true>, d.grid.update, kThreads, s, d, z32, first);
-    }
+template <class T>
+void residual_amg(const PcgDev &d, const AmgDevT<T> &a, const double *b, T *r, T *z, cudaStream_t s) {
+    launch_pdl(d.stag ? k_setup_amg<T, true> : k_setup_amg<T, false>, d.grid.setup_amg, kThreads, s, d, b,
+               vcycle_in(a, r, z));
 }
+template <class T>
+void iteration_amg(const PcgDev &d, const AmgDevT<T> &a, T *r, T *z, cudaStream_t s) {
+    launch_amg_vcycle(a, r, z, d.sc, s);
+    if (a.levels > 1)
+        launch_pdl(d.stag ? k_rz_amg<T, true, true> : k_rz_amg<T, true, false>, d.grid.rz, kThreads, s, d, a.lev[0], r,
+                   z);
+    else
+        launch_pdl(k_rz_amg<T, false, false>, d.grid.rz, kThreads, s, d, a.lev[0], r, z);
+    if constexpr (sizeof(T) == 4)
+        launch_pdl(k_pupdate_m, d.grid.pupdate, kThreads, s, d, z);
+    else
+        launch_pdl(k_pupdate, d.grid.pupdate, kThreads, s, d);
+    launch_spmv_dot(d, s);
+    launch_pdl(k_update_amg<T>, d.grid.update_amg, kThreads, s, d, vcycle_in(a, r, z));
+}
+}  // namespace
 
-void launch_pcg_setup_amg_mixed(const PcgDev &d, const AmgDev32 &a, const double *b, float *r32, float *z32,
-                                cudaStream_t s) {
-    launch_pdl(k_setup_amg<true>, d.grid.setup, kThreads, s, d, b, r32);
-    vcycle_rz(d, a, r32, z32, 1, s);
+void launch_pcg_residual_amg(const PcgDev &d, const AmgDev &a, const double *b, cudaStream_t s) {
+    residual_amg(d, a, b, d.r, d.z, s);
+}
+void launch_pcg_iteration_amg(PcgDev &d, const AmgDev &a, cudaStream_t s) { iteration_amg(d, a, d.r, d.z, s); }
+void launch_pcg_residual_amg(const PcgDev &d, const AmgDev32 &a, const double *b, float *r32, float *z32,
+                             cudaStream_t s) {
+    residual_amg(d, a, b, r32, z32, s);
+}
+void launch_pcg_iteration_amg(PcgDev &d, const AmgDev32 &a, float *r32, float *z32, cudaStream_t s) {
+    iteration_amg(d, a, r32, z32, s);
 }
 
 void launch_pcg_continue(cudaGraphConditionalHandle cond, const PcgScalars *sc, cudaStream_t s) {
     k_pcg_continue<<<1, 1, 0, s>>>(cond, sc);
 }
 
-bool pcg_rotated_ok(const AmgDev32 &a) { return amg_last_step_fusable(a); }
-
-void launch_pcg_residual_amg_mixed(const PcgDev &d, const double *b, float *r32, cudaStream_t s) {
-    launch_pdl(k_setup_amg<true>, d.grid.setup, kThreads, s, d, b, r32);
-}
-
-void launch_pcg_rotated_iteration_amg_mixed(PcgDev &d, const AmgDev32 &a, float *r32, float *z32, cudaStream_t s) {
-    launch_amg_vcycle_but_last(a, r32, z32, d.sc, s);
-    launch_pdl(k_jacobi_rz<2>, d.grid.update, kThreads, s, d, a.lev[0], r32, z32);
-    launch_pdl(k_pupdate_m, d.grid.pupdate, kThreads, s, d, z32);
-    launch_pdl(k_spmv_dot, d.grid.spmv, kThreads, s, d);
-    launch_pdl(k_update_amg<true>, d.grid.update, kThreads, s, d, r32);
-}
-
-void launch_pcg_iteration_amg_mixed(PcgDev &d, const AmgDev32 &a, float *r32, float *z32, cudaStream_t s) {
-    launch_pdl(k_spmv_dot, d.grid.spmv, kThreads, s, d);
-    launch_pdl(k_update_amg<true>, d.grid.update, kThreads, s, d, r32);
-    vcycle_rz(d, a, r32, z32, 0, s);
-    launch_pdl(k_pupdate_m, d.grid.pupdate, kThreads, s, d, z32);
-}
-
 void launch_pcg_iteration(PcgDev &d, cudaStream_t s) {
-    launch_pdl(k_spmv_dot, d.grid.spmv, kThreads, s, d);
+    launch_spmv_dot(d, s);
     launch_pdl(k_update, d.grid.update, kThreads, s, d);
     launch_pdl(k_pupdate, d.grid.pupdate, kThreads, s, d);
 }
-
-// Entries that are exactly zero off the diagonal are left out (the P1
-// stiffness of a Kuhn-split lattice is the 7-point stencil: 8 of its 15
-// structural couplings per row are exact zeros); a product with an exact
-// zero adds nothing to a sum, so A x is unchanged.
-template <class RP>
-void build_sell32_t(int64_t n, const RP *row_ptr, const int32_t *col, const double *val,
-                    std::vector<int64_t> &slice_ptr, std::vector<int32_t> &scol, std::vector<double> &sval) {
-    auto kept = [&](int64_t r, int64_t k) { return val[k] != 0.0 || col[k] == r; };
-    std::vector<int64_t> len(n, 0);
-    for (int64_t r = 0; r < n; ++r)
-        for (int64_t k = int64_t(row_ptr[r]); k < int64_t(row_ptr[r + 1]); ++k) len[r] += kept(r, k) ? 1 : 0;
-    const int64_t ns = (n + 31) / 32;
-    slice_ptr.assign(ns + 1, 0);
-    for (int64_t sl = 0; sl < ns; ++sl) {
-        int64_t w = 0;
-        for (int64_t r = sl * 32; r < std::min(n, sl * 32 + 32); ++r) w = std::max(w, len[r]);
-        slice_ptr[sl + 1] = slice_ptr[sl] + 32 * w;
-    }
-    scol.assign(slice_ptr[ns], 0);
-    sval.assign(slice_ptr[ns], 0.0);
-    for (int64_t sl = 0; sl < ns; ++sl) {
-        const int64_t w = (slice_ptr[sl + 1] - slice_ptr[sl]) / 32;
-        for (int64_t l = 0; l < 32; ++l) {
-            const int64_t r = sl * 32 + l;
-            int64_t j = 0;
-            int32_t first = 0;
-            if (r < n)
-                for (int64_t k = int64_t(row_ptr[r]); k < int64_t(row_ptr[r + 1]); ++k) {
-                    if (!kept(r, k)) continue;
-                    const int64_t o = slice_ptr[sl] + 32 * j + l;
-                    scol[o] = col[k];
-                    sval[o] = val[k];
-                    if (j == 0) first = col[k];
-                    ++j;
-                }
-            // padding: value 0 at a column the row already reads (or column
-            // 0), always inside x also for a rectangular matrix
-            for (; j < w; ++j) {
-                const int64_t o = slice_ptr[sl] + 32 * j + l;
-                scol[o] = first;
-                sval[o] = 0.0;
-            }
-        }
-    }
-}
-
-void build_sell32(int64_t n, const int32_t *row_ptr, const int32_t *col, const double *val,
-                  std::vector<int64_t> &slice_ptr, std::vector<int32_t> &scol, std::vector<double> &sval) {
-    build_sell32_t(n, row_ptr, col, val, slice_ptr, scol, sval);
-}
-void build_sell32(int64_t n, const int64_t *row_ptr, const int32_t *col, const double *val,
-                  std::vector<int64_t> &slice_ptr, std::vector<int32_t> &scol, std::vector<double> &sval) {
-    build_sell32_t(n, row_ptr, col, val, slice_ptr, scol, sval);
-}
-
-}  // namespace spg
-
-namespace spg {
 
 void launch_refine_setup(const PcgDev &d, const PcgDev32 &f, const double *b, cudaStream_t s) {
     launch_pdl(k_refine_setup, f.grid.setup, kThreads, s, d, f, b);

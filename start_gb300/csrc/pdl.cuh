@@ -7,6 +7,8 @@
 // keeps stream order. griddepcontrol.launch_dependents, issued first, lets
 // the successor be scheduled as soon as every block of this grid has
 // started. Both are no-ops for a kernel launched without the attribute.
+// A kernel may read before the wait what no kernel of the chain writes (the
+// matrices, written once when a handle is made and waited for there).
 #ifndef SPG_PDL_CUH
 #define SPG_PDL_CUH
 
@@ -16,9 +18,11 @@
 
 namespace spg {
 
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_sync() {
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    asm volatile("griddepcontrol.wait;" ::: "memory");
+    pdl_trigger();
+    pdl_wait();
 }
 
 template <class... KArgs, class... Args>

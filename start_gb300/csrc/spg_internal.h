@@ -10,6 +10,7 @@
 #include <cuda_runtime.h>
 
 #include "../../include/start_gpu.h"
+#include "sell_build.h"
 #include "screen.h"
 
 namespace spg {
@@ -379,6 +380,7 @@ struct PcgScalars {
 // kernel), capped by the rows; every kernel loops over rows grid-stride.
 struct PcgGrid {
     int setup = 1, spmv = 1, update = 1, pupdate = 1;
+    int setup_amg = 1, update_amg = 1, rz = 1;  // PCG with the V-cycle
 };
 struct PcgDev {
     int64_t n;
@@ -387,6 +389,8 @@ struct PcgDev {
     const int64_t *slice_ptr;  // SELL-32: n_slices + 1 offsets
     const int32_t *scol;
     const double *sval;
+    const int64_t *stag;       // banded slices (band_sell32); nullptr: too few
+    const int32_t *sref;
     double *x, *r, *z, *p, *p2, *q;
     double *partials;  // 3 doubles per block
     PcgScalars *sc;
@@ -415,12 +419,6 @@ void launch_refine_apply(double *x, const float *e, int64_t n, cudaStream_t s);
 // phi becomes the polynomial extrapolation of order `order` (0: unchanged,
 // 1: 2 phi - prev, 2: 3 phi - 3 prev + prev2).
 void launch_extrapolate(double *phi, double *prev, double *prev2, int64_t n, int order, cudaStream_t s);
-// CSR -> SELL-32 (slices of 32 rows, column-major, zero padding).
-void build_sell32(int64_t n, const int32_t *row_ptr, const int32_t *col, const double *val,
-                  std::vector<int64_t> &slice_ptr, std::vector<int32_t> &scol, std::vector<double> &sval);
-void build_sell32(int64_t n, const int64_t *row_ptr, const int32_t *col, const double *val,
-                  std::vector<int64_t> &slice_ptr, std::vector<int32_t> &scol, std::vector<double> &sval);
-
 // ---------------------------------------------------------------- sources
 // A particle source on the device (kernels_sources.cu): the spg_source with
 // its frame (e1, e2, normal) and energy constants formed on the host.
@@ -491,9 +489,10 @@ int amg_setup(int64_t n, const int32_t *row_ptr, const int32_t *col, const doubl
 
 constexpr int kAmgMaxLevels = 12;
 // A V-cycle operator on the device: SELL-32 with one thread per row (g = 0,
-// short rows), or CSR with g lanes per row (g = 4, 8, 16 or 32; the long rows
+// short rows; g = kSellBanded, mostly banded slices), or CSR with g lanes per row (g = 4, 8, 16 or 32; the long rows
 // of coarse operators and of the restriction). T: double (FP64 form) or
 // float (the inner solve of the mixed form).
+constexpr int kSellBanded = -1;
 template <class T>
 struct DevSellT {
     int64_t n = 0;
@@ -501,19 +500,20 @@ struct DevSellT {
     const int64_t *slice_ptr = nullptr;  // SELL: slice offsets; CSR: row offsets
     const int32_t *scol = nullptr;
     const T *sval = nullptr;
+    const int64_t *stag = nullptr;  // level 0: banded slices (band_sell32)
+    const int32_t *sref = nullptr;
 };
-// One level of the V-cycle on the device. Jacobi-Chebyshev smoothing on
-// D^-1 A: degree 2 over [lam/30, lam], or degree 1 (damped Jacobi,
-// 1/theta = 1.6/lam) over [lam/4, lam]; theta = (hi+lo)/2, delta = (hi-lo)/2.
+// One level of the V-cycle on the device. Damped Jacobi smoothing with
+// 1/theta = 1.6/lam, the degree-1 Chebyshev polynomial of D^-1 A over
+// [lam/4, lam].
 template <class T>
 struct AmgLevelDevT {
     int64_t n = 0;
-    int degree = 2;
     DevSellT<T> A, P, R;  // P: n x n_next, R: n_next x n
     const T *dinv = nullptr;
     T *x[2] = {nullptr, nullptr};  // iterate ping-pong
-    T *b = nullptr, *r = nullptr, *d = nullptr;
-    double inv_theta = 0.0, cheb_a = 0.0, cheb_b = 0.0;  // step 2: d = a d + b D^-1 r
+    T *b = nullptr, *r = nullptr;
+    double inv_theta = 0.0;
 };
 template <class T>
 struct AmgDevT {
@@ -526,33 +526,24 @@ using DevSell = DevSellT<double>;
 using AmgLevelDev = AmgLevelDevT<double>;
 using AmgDev = AmgDevT<double>;
 using AmgDev32 = AmgDevT<float>;
-// z = M^-1 r by one V-cycle (level 0 vectors: b = r, x[0] = z, x[1] scratch);
-// every kernel returns at once when sc->converged is set (sc->converged == 3,
-// the inner cap of the mixed form, also stops it).
+// One V-cycle on r but for level 0's last Jacobi step, which the PCG runs
+// fused with r.z: z holds x0 = D^-1 r / theta of level 0 on entry (written by
+// the kernel that writes r) and lev[0].x[1] the iterate of that last step on
+// return. With one level only (a system of at most AmgOptions::coarse_rows
+// rows) z = A^-1 r. Every kernel returns at once when sc->converged is set.
 void launch_amg_vcycle(const AmgDev &a, const double *r, double *z, const PcgScalars *sc, cudaStream_t s);
 void launch_amg_vcycle(const AmgDev32 &a, const float *r, float *z, const PcgScalars *sc, cudaStream_t s);
-// The FP32 V-cycle without level 0's last Jacobi step, which the mixed PCG
-// then runs fused with r.z (possible when level 0 is degree 1 in SELL-32).
-bool amg_last_step_fusable(const AmgDev32 &a);
-void launch_amg_vcycle_but_last(const AmgDev32 &a, const float *r, float *z, const PcgScalars *sc, cudaStream_t s);
-// PCG with the V-cycle: setup and one iteration (spmv_dot, update, V-cycle,
-// r.z and beta, p update).
-void launch_pcg_setup_amg(const PcgDev &d, const AmgDev &a, const double *b, cudaStream_t s);
+// PCG with the V-cycle, rotated so that a loop stops right after the stop
+// test: the residual and its norm, then iterations of V-cycle, r.z and beta
+// (p = z in the first), p update, SpMV and alpha, x and r update with the
+// stop test.
+void launch_pcg_residual_amg(const PcgDev &d, const AmgDev &a, const double *b, cudaStream_t s);
 void launch_pcg_iteration_amg(PcgDev &d, const AmgDev &a, cudaStream_t s);
-// The mixed form's PCG: FP64 SpMV, vectors and sums with the FP32 V-cycle as
-// the preconditioner (r32 = float(r) in, z32 out).
-void launch_pcg_setup_amg_mixed(const PcgDev &d, const AmgDev32 &a, const double *b, float *r32, float *z32,
-                                cudaStream_t s);
-void launch_pcg_iteration_amg_mixed(PcgDev &d, const AmgDev32 &a, float *r32, float *z32, cudaStream_t s);
-// The same PCG rotated for the while-graph, so that the loop stops right
-// after the update that converges: the setup only forms r (and r32); an
-// iteration is the V-cycle, r.z and beta (p = z in the first), the p update,
-// q = A p and the update of x and r with the stop test. Needs a level 0 that
-// fuses its last step with r.z (pcg_rotated_ok).
-bool pcg_rotated_ok(const AmgDev32 &a);
-void launch_pcg_residual_amg_mixed(const PcgDev &d, const double *b, float *r32, cudaStream_t s);
-void launch_pcg_rotated_iteration_amg_mixed(PcgDev &d, const AmgDev32 &a, float *r32, float *z32, cudaStream_t s);
-// Last node of a PCG while-graph body: the condition stays 1 until sc->converged.
+// The mixed form's: FP64 SpMV, vectors and sums with the FP32 V-cycle as the
+// preconditioner (r32 = float(r) in, z32 out).
+void launch_pcg_residual_amg(const PcgDev &d, const AmgDev32 &a, const double *b, float *r32, float *z32,
+                             cudaStream_t s);
+void launch_pcg_iteration_amg(PcgDev &d, const AmgDev32 &a, float *r32, float *z32, cudaStream_t s);
 void launch_pcg_continue(cudaGraphConditionalHandle cond, const PcgScalars *sc, cudaStream_t s);
 // b = node_q/eps0 - lift on free rows, g on Dirichlet rows
 void launch_pcg_rhs(const double *node_q, double inv_eps0, const double *lift, const uint8_t *is_dir,
