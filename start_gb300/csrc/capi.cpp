@@ -172,12 +172,8 @@ struct spg_handle {
     WalkItem *walkq = nullptr;       // mixed form's walk queue, capacity cap (particles)
     unsigned int *walkq_n = nullptr;
     // segmented steps: at most seg_max steps per segment (1: one launch per
-    // step); mixed form: resumed-particle list and per-round counters
+    // step)
     int seg_max = 32;
-    int2 *seg_rq = nullptr;
-    int64_t seg_rq_cap = 0;
-    unsigned int *seg_qn = nullptr;
-    int seg_qn_cap = 0;
     int64_t *n_alive_dev = nullptr;
     int32_t *sort_scratch = nullptr;
     // Staging for particles that cross the host boundary or come from a
@@ -1289,7 +1285,10 @@ int step_stamp(spg_handle *h, uint32_t &seq) {
     }
     if (!h->field_full) {  // out of numbers: a complete field needs none
         h->field_epoch = h->field_seq = 1;
-        launch_field64_full(field_args(h), h->n_tets, h->stream);
+        if (h->mixed)
+            launch_field32_full(field_args(h), h->n_tets, h->stream);
+        else
+            launch_field64_full(field_args(h), h->n_tets, h->stream);
         CK(cudaGetLastError());
         h->field_full = true;
     }
@@ -1316,49 +1315,29 @@ int do_segment64(spg_handle *h, int l) {
     return SPG_OK;
 }
 
+int do_segment32(spg_handle *h, int l);
+
 int do_process(spg_handle *h) {
     h->occ_fresh = false;
     if (h->track_k > 0) {
         const int rc = record_tracks(h);
         if (rc) return rc;
     }
-    if (!h->mixed) return do_segment64(h, 1);
-    StepConst c = step_const(h);
-    ev_begin(h, h->ev_step);
-    launch_step32(h->Q[h->cur], h->n_active, mesh_dev32(h), c, h->tri_count, h->walkq, h->walkq_n, h->ctr,
-                  field_args(h), h->stream);
-    ev_end(h, h->ev_step);
-    if (h->n_active > 0) h->launches += 2;  // step kernel + queued walks
-    CK(cudaGetLastError());
-    if (h->prof) h->step_bytes += 92.0 * double(h->occupied ? h->occupied : std::min(h->n_tets, h->n_active));
-    h->step++;
-    return SPG_OK;
+    return h->mixed ? do_segment32(h, 1) : do_segment64(h, 1);
 }
 
 // Steps h->step .. h->step + l - 1 of the mixed form as one segment (nothing
 // of the time loop falls between them).
 int do_segment32(spg_handle *h, int l) {
     h->occ_fresh = false;
-    if (h->seg_rq_cap < h->cap) {
-        cudaFree(h->seg_rq);
-        h->seg_rq = nullptr;
-        h->seg_rq_cap = 0;
-        CK(dalloc(&h->seg_rq, size_t(std::max<int64_t>(h->cap, 1))));
-        h->seg_rq_cap = h->cap;
-    }
-    if (h->seg_qn_cap < 2 * l + 1) {
-        cudaFree(h->seg_qn);
-        h->seg_qn = nullptr;
-        h->seg_qn_cap = 0;
-        CK(dalloc(&h->seg_qn, size_t(2 * h->seg_max + 1)));
-        h->seg_qn_cap = 2 * h->seg_max + 1;
-    }
-    StepConst c = step_const(h);
+    uint32_t seq = 0;
+    const int rc = step_stamp(h, seq);
+    if (rc) return rc;
     ev_begin(h, h->ev_step);
-    const int nl = launch_segment32(h->Q[h->cur], h->n_active, mesh_dev32(h), c, l, h->tri_count, h->walkq,
-                                    h->seg_rq, h->seg_qn, h->ctr, field_args(h), h->stream);
+    launch_segment32(h->Q[h->cur], h->n_active, mesh_dev32(h), step_const(h), l, h->tri_count, h->ctr, field_args(h), seq,
+                     h->stream);
     ev_end(h, h->ev_step);
-    h->launches += nl;
+    if (h->n_active > 0) h->launches += 1;
     CK(cudaGetLastError());
     if (h->prof)
         h->step_bytes += double(l) * 92.0 * double(h->occupied ? h->occupied : std::min(h->n_tets, h->n_active));
@@ -1777,7 +1756,7 @@ int spg_destroy(spg_handle *h) {
                     h->gE,       h->lam,      h->mu,       h->dJdg,    h->sums, h->hist64, h->hist.tet, h->hist.vx,
                     h->hist.vy,  h->hist.vz,  h->tri_scratch, h->ctr_scratch,
                     h->q,        h->partials, h->sc,       h->tri_count, h->ctr,      h->n_alive_dev, h->sort_scratch, h->walkq_n,
-                    h->io,       h->seg_rq,   h->seg_qn,   h->res_zp,  h->res_partials, h->res_arrived};
+                    h->io,       h->res_zp,  h->res_partials, h->res_arrived};
     for (void *ptr : ptrs) cudaFree(ptr);
     for (EventSeries *s : {&h->ev_step, &h->ev_dep, &h->ev_pcg, &h->ev_ef, &h->ev_sort}) ev_destroy(*s);
     for (void *ptr : h->amg_alloc) cudaFree(ptr);

@@ -22,6 +22,7 @@
 #include "philox.h"
 #include "deposit.cuh"
 #include "field.cuh"
+#include "segment.cuh"
 #include "sort_block.cuh"
 #include "spg_internal.h"
 
@@ -161,7 +162,7 @@ struct Walk32 {
 // re-based on every crossing (FP32 pair arithmetic). Same exit rule as the
 // FP64 walk (smallest crossing parameter among faces with lambda(p1) < 0,
 // entry face excluded).
-__device__ __noinline__ Walk32 walk32(const MixedArgs a, int t, float p0x, float p0y, float p0z, float p1x,
+__device__ __noinline__ Walk32 walk32(const MixedArgs &a, int t, float p0x, float p0y, float p0z, float p1x,
                                       float p1y, float p1z, int max_cross) {
     Walk32 o;
     o.crossings = 0;
@@ -420,29 +421,45 @@ __global__ void __launch_bounds__(256, 4) k_step32(MixedArgs a, StepConst c, Wal
 // across a tet would lose the field), then the FP32 push increment
 // H = float(E c) with c = q dt / (2 m) formed once on the host, so no FP64
 // division runs per tet. The FP64 record of the plain form is not touched.
-__device__ __forceinline__ void field_of_tet32(const FieldArgs &f, int64_t t) {
+struct Field32 {
+    double E[3];
+    float H[3];
+    bool zero;
+};
+
+__device__ __forceinline__ Field32 field_values32(const FieldArgs &f, int64_t t) {
     const int4 tn = __ldg(f.tet_nodes + t);
     const double f0 = f.phi[tn.x], f1 = f.phi[tn.y], f2 = f.phi[tn.z], f3 = f.phi[tn.w];
     const double d1 = f1 - f0, d2 = f2 - f0, d3 = f3 - f0;
     const TetRec &r = f.rec[t];
-    double E[3];
+    Field32 o;
     // Explicitly rounded products and sums: this file is built with FMA
     // contraction on, and E is the FP64 field the oracle computes unfused.
 #pragma unroll
-    for (int k = 0; k < 3; ++k)
-        E[k] = -__dadd_rn(__dadd_rn(__dmul_rn(d1, r.M[k]), __dmul_rn(d2, r.M[3 + k])), __dmul_rn(d3, r.M[6 + k]));
+    for (int k = 0; k < 3; ++k) {
+        o.E[k] = -__dadd_rn(__dadd_rn(__dmul_rn(d1, r.M[k]), __dmul_rn(d2, r.M[3 + k])), __dmul_rn(d3, r.M[6 + k]));
+        o.H[k] = float(o.E[k] * f.c32);
+    }
+    o.zero = o.E[0] == 0.0 && o.E[1] == 0.0 && o.E[2] == 0.0;
+    return o;
+}
+
+__device__ __forceinline__ void store_field32(const FieldArgs &f, int64_t t, const Field32 &v) {
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
-        f.efield[3 * t + k] = E[k];
-        f.rec32[t].H[k] = float(E[k] * f.c32);
+        f.efield[3 * t + k] = v.E[k];
+        f.rec32[t].H[k] = v.H[k];
     }
-    const bool null_field = E[0] == 0.0 && E[1] == 0.0 && E[2] == 0.0;
-    f.rec32[t].ezero = (f.rec32[t].ezero & kRecInterior) | (null_field ? kRecEzero : 0u);
+    f.rec32[t].ezero = (f.rec32[t].ezero & kRecInterior) | (v.zero ? kRecEzero : 0u);
+}
+
+__device__ __forceinline__ void field_of_tet32(const FieldArgs &f, int64_t t) {
+    store_field32(f, t, field_values32(f, t));
 }
 
 // With land != nullptr a particle that settles records the step, the exit
 // face, its tet and the hit fraction (adjoint).
-__global__ void __launch_bounds__(128) k_walk_queue32(MixedArgs a, int max_cross, const WalkItem32 *__restrict__ wq,
+__global__ void __launch_bounds__(128) k_walk_queue32(const __grid_constant__ MixedArgs a, int max_cross, const WalkItem32 *__restrict__ wq,
                                                       const unsigned int *__restrict__ wq_n,
                                                       unsigned int *__restrict__ tri_count, DevCounters *ctr,
                                                       LandRec *__restrict__ land, int64_t step,
@@ -491,234 +508,273 @@ __global__ void __launch_bounds__(128) k_walk_queue32(MixedArgs a, int max_cross
 
 // ---------------------------------------------------------------------------
 // Segmented step: every step between two events of the time loop (a solve,
-// a re-sort, the end of the call) in one pass over the particles. A particle
-// keeps its state and its tet's record in registers and leaves the pass at
-// the first step whose move needs the exact walk; it is queued with that
-// step's index, the walk kernel walks it, and a resume pass runs it on from
-// the next step. Each pass reads only fields that earlier launches wrote (a
-// walk computes the field of the tet it enters; the particle is stepped
-// there in the next launch), and every particle goes through the same FP32
-// operations in the same order as in single steps, so the result is
-// bit-identical to stepping one step per launch.
+// a re-sort, the end of the call) in one launch over the particles.
+//
+// A warp steps groups of 32 particles in registers, each lane with its tet's
+// map and push increment, until the segment's end or a step that needs what few
+// lanes need: the exact walk (the end point is not surely inside the tet) or a
+// collision test that the screen leaves open. Such a lane waits; when the group
+// is through, its waiting particles go to the warp's queue in shared memory.
+// Once 32 wait there they are the next group: their tests and walks run in a
+// full warp and they step on from where they left. So no particle passes
+// through memory between its load and its last store, and the branches of few
+// lanes cost a warp once per group instead of in 60 % of its steps.
+// A field that an earlier launch wrote (epoch <= stamp < seq, as in the FP64
+// form) is read, any other is formed in registers and stored by the lane that
+// swaps the stamp. Every particle goes through the same FP32 operations in the
+// same order as in single steps, so the result is bit-identical to stepping one
+// step per launch.
+//
+// Before, one launch took all particles to their first walk and up to L - 1
+// rounds of a walk and a resume launch took the ones that had left on. us per
+// step of a segment of ten: 1e7 ions on 6.0e6 tets 116 -> 73, 1e6 on 7.5e5 16.2
+// -> 8.1, 3e5 on 94,000 9.6 -> 3.8, 1e4 on 6,000 6.0 -> 1.9. It is bound by
+// instruction issue (69 % of the slots, 24 of 32 lanes; 130 MB read and 87
+// written per 4e6 ions and ten steps are a tenth of the memory's time). Blocks
+// per SM 8 / 7 / 6 / 5: 74 / 73 / 74 / 78 us at 1e7, 8.8 / 8.2 / 8.1 / 8.3 at
+// 1e6. Refilling idle lanes one by one, as the FP64 form does, costs FP32 steps
+// more instructions than the idle lanes (124 us at 1e7).
+constexpr int kMaxSegment = 64;         // steps per segment at most (the candidate mask's bits)
+constexpr int kWalkQ = 64, kTestQ = 32; // np <= 31 before a group and grows by at most 32
+constexpr int kTestRun = 24;            // tests without a walk that make a group of their own
+constexpr int kItemWords = 15;
 
-constexpr int kMaxSegment = 64;  // steps per segment at most
+struct WarpQueue {
+    float w[kItemWords][kWalkQ + kTestQ];
+};
+constexpr int kNeedWalk = 1, kNeedTest = 2, kNeedLost = 4;
+constexpr int kFlagBits = 3;
 
-struct SegItem32 {  // a move of step s0 + step that needs the walk
-    int32_t i, step;
-    float x0, y0, z0;
+struct Seg32 {
+    MixedArgs m;
+    unsigned int *tri_count;
+    DevCounters *ctr;
+    int L;
+    uint32_t seq;
 };
 
-struct SegQueues {
-    SegItem32 *wq;           // walk items of the current round (at most one per particle)
-    int2 *rq;                // resumed particles: {index, first step}
-    unsigned int *wq_n;      // [L + 1]: walk items of round r
-    unsigned int *rq_n;      // [L]: resumed particles of round r
-    int L;                   // steps of the segment (steps s0 .. s0 + L - 1)
-};
-
-__device__ __forceinline__ void queue_seg32(SegItem32 *__restrict__ q, unsigned int *__restrict__ qn, int64_t i,
-                                            int j, float x, float y, float z) {
-    const unsigned act = __activemask();
-    const int lane = threadIdx.x & 31;
-    const int leader = __ffs(act) - 1;
-    unsigned base = 0;
-    if (lane == leader) base = atomicAdd(qn, unsigned(__popc(act)));
-    base = __shfl_sync(act, base, leader);
-    SegItem32 &w = q[base + __popc(act & ((1u << lane) - 1u))];
-    w.i = int32_t(i);
-    w.step = j;
-    w.x0 = x;
-    w.y0 = y;
-    w.z0 = z;
-}
-
-// Steps j0 .. L - 1 of particle i (state w, alive) in registers: the
-// operations of k_step32 for each step. Leaves at the segment's end, when the
-// particle is lost, when it stays put for good (too slow or outside the
-// modelling box: nothing changes it any more) or with its move queued for
-// the walk (round r's items go to wq_n[r]).
-__device__ __forceinline__ void seg_steps32(const MixedArgs &a, const StepConst &c, int64_t i, const Words32 &w,
-                                            int j0, const SegQueues &sq, unsigned int *__restrict__ qn,
-                                            unsigned &processed, unsigned &coll, unsigned &lost) {
-    const float4 *rp = reinterpret_cast<const float4 *>(a.rec + w.t);
-    const float4 r0 = __ldg(rp), r1 = __ldg(rp + 1), r2 = __ldg(rp + 2), r3 = __ldg(rp + 3);
-    const Geo32 g{{r0.x, r0.y, r0.z, r0.w, r1.x, r1.y, r1.z, r1.w, r2.x}};
-    const uint32_t flags = __float_as_uint(r3.w);
-    const bool push = !(flags & kRecEzero), interior = flags & kRecInterior;
-    const float hx = r2.y, hy = r2.z, hz = r2.w;
-    const uint32_t id = w.idf & kIdMask;
-    float x = w.x, y = w.y, z = w.z, vx = w.vx, vy = w.vy, vz = w.vz;
+__global__ void __launch_bounds__(128, 6) k_seg32(const __grid_constant__ Seg32 a, const __grid_constant__ StepConst c,
+                                                  const __grid_constant__ FieldArgs f) {
+    extern __shared__ __align__(16) unsigned char queue_bytes[];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const unsigned below = (1u << lane) - 1u;
+    WarpQueue &Q = reinterpret_cast<WarpQueue *>(queue_bytes)[wid];
+    unsigned processed = 0, coll = 0, lost = 0, cross = 0, settled = 0, capped = 0;
+    int np = 0, nt = 0;  // waiting for a walk at [0, np), for a test alone at [kWalkQ, kWalkQ + nt)
+    const int64_t stride = int64_t(gridDim.x) * blockDim.x;
+    int64_t base = int64_t(blockIdx.x) * blockDim.x + 32 * wid;
     const float vmin2 = c.vmin_f * c.vmin_f, dt = c.dt_f;
-    float v2 = speed2(vx, vy, vz);  // of the current velocity
-    bool dirty = false;
-    // the candidate steps of the last sixteen-step group tested (cgroup: the
-    // low 32 bits of its count; steps in a segment are consecutive, so the
-    // key changes exactly when the group does)
-    uint32_t cmask = 0u, cgroup = ~0u;
-    const uint32_t step_lo = uint32_t(c.step);
-    auto collide = [&](int j) -> unsigned {
-        const uint32_t sj = step_lo + uint32_t(j);
-        const uint64_t step = uint64_t(c.step) + uint64_t(j);
-        if ((sj >> 4) != cgroup) {
-            cgroup = sj >> 4;
-            cmask = candidate_mask(candidate_block(step, id, c.seed_lo, c.seed_hi));
-        }
-        if (!collide32(c, id, step, (cmask >> (sj & 15u)) & 1u, v2, vx, vy, vz)) return 0u;
-        v2 = speed2(vx, vy, vz);
-        return 1u;
-    };
-    for (int j = j0; j < sq.L; ++j) {
-        processed++;
-        const bool slow = v2 < vmin2;
-        if (slow || (!interior && !in_box32(c, r3.x + x, r3.y + y, r3.z + z))) {
-            processed += unsigned(sq.L - 1 - j);
+    for (;;) {
+        // ---- the next group
+        bool have = false, dirty = false;
+        float x = 0.0f, y = 0.0f, z = 0.0f, vx = 0.0f, vy = 0.0f, vz = 0.0f, nx = 0.0f, ny = 0.0f, nz = 0.0f;
+        float hx = 0.0f, hy = 0.0f, hz = 0.0f;
+        bool push = false, interior = false, have_field = false;
+        int tet = 0, i = 0, j = 0;
+        uint32_t idf = 0;
+        unsigned long long cand = 0ull;
+        const bool fresh = base < a.m.n;
+        if (np >= 32 || nt >= kTestRun || (!fresh && np + nt > 0)) {
+            const bool walks = np >= 32 || (nt < kTestRun && np > 0);
+            const int take = min(walks ? np : nt, 32);
+            const int k = (walks ? np - take : kWalkQ + nt - take) + lane;
+            if (walks)
+                np -= take;
+            else
+                nt -= take;
+            if (lane < take) {
+                x = Q.w[0][k];
+                y = Q.w[1][k];
+                z = Q.w[2][k];
+                nx = Q.w[3][k];
+                ny = Q.w[4][k];
+                nz = Q.w[5][k];
+                vx = Q.w[6][k];
+                vy = Q.w[7][k];
+                vz = Q.w[8][k];
+                tet = __float_as_int(Q.w[9][k]);
+                idf = __float_as_uint(Q.w[10][k]);
+                i = __float_as_int(Q.w[11][k]);
+                const int need = __float_as_int(Q.w[12][k]);
+                cand = (unsigned long long)__float_as_uint(Q.w[13][k]) |
+                       (unsigned long long)__float_as_uint(Q.w[14][k]) << 32;
+                j = need >> kFlagBits;
+                if (need & kNeedTest)
+                    coll += collide32(c, idf & kIdMask, uint64_t(c.step) + uint64_t(j), (cand >> j) & 1ull,
+                                      speed2(vx, vy, vz), vx, vy, vz)
+                                ? 1u
+                                : 0u;
+                int status = W_INSIDE;
+                if (need & kNeedLost) {
+                    status = W_EXIT;
+                    nx = x;
+                    ny = y;
+                    nz = z;
+                } else if (need & kNeedWalk) {
+                    const Walk32 w = walk32(a.m, tet, x, y, z, nx, ny, nz, c.max_cross);
+                    cross += unsigned(w.crossings);
+                    status = w.status;
+                    nx = w.hx;
+                    ny = w.hy;
+                    nz = w.hz;
+                    if (w.status == W_SURFACE) {
+                        atomicAdd(a.tri_count + w.tri, 1u);
+                    } else if (w.status == W_INSIDE && w.tet != tet) {
+                        const uint32_t st = __ldcg(f.stamp + w.tet);
+                        if (!(st >= f.epoch && st < a.seq)) {
+                            const Field32 v = field_values32(f, w.tet);
+                            hx = v.H[0];
+                            hy = v.H[1];
+                            hz = v.H[2];
+                            push = !v.zero;
+                            have_field = true;
+                            if (st < f.epoch && atomicCAS(f.stamp + w.tet, st, a.seq) == st) store_field32(f, w.tet, v);
+                        }
+                    }
+                    tet = w.tet;
+                }
+                x = nx;
+                y = ny;
+                z = nz;
+                dirty = true;
+                if (status == W_INSIDE) {
+                    have = ++j < a.L;
+                } else {
+                    settled += status == W_SURFACE ? 1u : 0u;
+                    lost += status != W_SURFACE ? 1u : 0u;
+                    capped += status == W_CAP ? 1u : 0u;
+                    a.m.p.idf[i] = idf | (status == W_SURFACE ? kSettled : kLost);
+                }
+            }
+            __syncwarp();
+        } else if (fresh) {
+            i = int(base) + lane;
+            base += stride;
+            idf = kDead;
+            if (i < a.m.n) idf = a.m.p.idf[i];
+            if (!(idf & kDead)) {
+                tet = a.m.p.tet[i];
+                x = a.m.p.x[i];
+                y = a.m.p.y[i];
+                z = a.m.p.z[i];
+                vx = a.m.p.vx[i];
+                vy = a.m.p.vy[i];
+                vz = a.m.p.vz[i];
+                if (c.model != SPG_COLL_NONE) cand = segment_candidates(c, idf & kIdMask, a.L);
+                have = true;
+            }
+        } else {
             break;
         }
-        if (push) {
-            vx = (vx + hx) + hx;
-            vy = (vy + hy) + hy;
-            vz = (vz + hz) + hz;
-            v2 = speed2(vx, vy, vz);
-            dirty = true;
+        Geo32 g{};
+        if (have) {
+            load_geo32(a.m.rec, tet, g);
+            // the part that launches write comes from L2: an L1 line may be older
+            const float4 *rp = reinterpret_cast<const float4 *>(a.m.rec + tet);
+            const uint32_t w = __float_as_uint(__ldcg(rp + 3).w);
+            interior = w & kRecInterior;
+            if (!have_field) {
+                const float4 h = __ldcg(rp + 2);
+                hx = h.y;
+                hy = h.z;
+                hz = h.w;
+                push = !(w & kRecEzero);
+            }
         }
-        const float nx = fmaf(vx, dt, x), ny = fmaf(vy, dt, y), nz = fmaf(vz, dt, z);
-        if (nx == x && ny == y && nz == z) continue;
-        if (!(isfinite(nx) && isfinite(ny) && isfinite(nz))) {
-            a.p.idf[i] = w.idf | kLost;
-            lost++;
-            if (c.model != SPG_COLL_NONE) coll += collide(j);
-            a.p.x[i] = x;
-            a.p.y[i] = y;
-            a.p.z[i] = z;
-            a.p.vx[i] = vx;
-            a.p.vy[i] = vy;
-            a.p.vz[i] = vz;
-            return;
+        // ---- its steps
+        int need = 0;
+        float v2 = speed2(vx, vy, vz);
+        while (__any_sync(kFull, have)) {
+            if (have) {
+                ++processed;
+                bool stays = v2 < vmin2;
+                if (!interior) {
+                    const float4 cen = __ldg(reinterpret_cast<const float4 *>(a.m.rec + tet) + 3);
+                    stays = stays || !in_box32(c, cen.x + x, cen.y + y, cen.z + z);
+                }
+                if (stays) {  // nothing moves it any more
+                    processed += unsigned(a.L - 1 - j);
+                    have = false;
+                } else {
+                    if (push) {
+                        vx = (vx + hx) + hx;
+                        vy = (vy + hy) + hy;
+                        vz = (vz + hz) + hz;
+                        v2 = speed2(vx, vy, vz);
+                        dirty = true;
+                    }
+                    nx = fmaf(vx, dt, x);
+                    ny = fmaf(vy, dt, y);
+                    nz = fmaf(vz, dt, z);
+                    if (!(nx == x && ny == y && nz == z)) {
+                        dirty = true;
+                        float l[4];
+                        bary32(g, nx, ny, nz, l);
+                        // inside: all above kNearZero; the smallest of four that sum to 1 is
+                        // at most 1/4, so a larger one comes from a position that is no number
+                        const float mn = fminf(fminf(l[0], l[1]), fminf(l[2], l[3]));
+                        if (!(mn > kNearZero && mn < 0.5f)) need = kNeedWalk;
+                        if (c.model != SPG_COLL_NONE && (((cand >> j) & 1ull) || !(v2 <= c.v2_cand_f)))
+                            need |= kNeedTest;
+                        if (!need) {
+                            x = nx;
+                            y = ny;
+                            z = nz;
+                        }
+                    }
+                    have = !need && ++j < a.L;
+                }
+            }
         }
-        float l[4];
-        bary32(g, nx, ny, nz, l);
-        const float mn = fminf(fminf(l[0], l[1]), fminf(l[2], l[3]));
-        if (!(mn > kNearZero)) {
-            queue_seg32(sq.wq, qn, i, j, x, y, z);
-            if (c.model != SPG_COLL_NONE) coll += collide(j);
-            a.p.x[i] = nx;
-            a.p.y[i] = ny;
-            a.p.z[i] = nz;
-            a.p.vx[i] = vx;
-            a.p.vy[i] = vy;
-            a.p.vz[i] = vz;
-            return;
+        // ---- the waiting ones to the queue, the others to the arrays
+        if (need & kNeedWalk) {
+            if (!(isfinite(nx) && isfinite(ny) && isfinite(nz))) need ^= kNeedWalk | kNeedLost;
         }
-        x = nx;
-        y = ny;
-        z = nz;
-        if (c.model != SPG_COLL_NONE) coll += collide(j);
-        dirty = true;
-    }
-    if (dirty) {
-        a.p.x[i] = x;
-        a.p.y[i] = y;
-        a.p.z[i] = z;
-        a.p.vx[i] = vx;
-        a.p.vy[i] = vy;
-        a.p.vz[i] = vz;
-    }
-}
-
-__device__ __forceinline__ void add_step_counters(DevCounters *ctr, unsigned processed, unsigned coll,
-                                                  unsigned lost) {
-    const unsigned long long s0 = __reduce_add_sync(kFull, processed), s1 = __reduce_add_sync(kFull, coll);
-    const unsigned long long s2 = __reduce_add_sync(kFull, lost);
-    if ((threadIdx.x & 31) == 0) {
-        if (s0) atomicAdd(&ctr->processed, s0);
-        if (s1) atomicAdd(&ctr->collisions, s1);
-        if (s2) atomicAdd(&ctr->lost, s2);
-    }
-}
-
-// The segment's first pass over every particle (grid-stride, the next
-// particle's words loaded before the current one is stepped).
-__global__ void __launch_bounds__(256, 3) k_seg32(MixedArgs a, StepConst c, SegQueues sq, DevCounters *ctr) {
-    const int64_t stride = int64_t(gridDim.x) * blockDim.x;
-    int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    unsigned processed = 0, coll = 0, lost = 0;
-    Words32 cur{};
-    if (i < a.n) cur = load_words32(a.p, i);
-    for (; i < a.n; i += stride) {
-        Words32 nxt{};
-        if (i + stride < a.n) nxt = load_words32(a.p, i + stride);
-        if (!(cur.idf & kDead)) seg_steps32(a, c, i, cur, 0, sq, sq.wq_n, processed, coll, lost);
-        cur = nxt;
-    }
-    add_step_counters(ctr, processed, coll, lost);
-}
-
-// Round r's walks (the queued moves, each of its own step); a particle still
-// inside with steps left is listed for the resume pass of round r.
-__global__ void __launch_bounds__(128) k_seg_walk32(MixedArgs a, int max_cross, SegQueues sq, int r,
-                                                    unsigned int *__restrict__ tri_count, DevCounters *ctr,
-                                                    const __grid_constant__ FieldArgs f) {
-    pdl_sync();
-    const unsigned nq = sq.wq_n[r];
-    unsigned cross = 0, settled = 0, lost = 0, capped = 0;
-    for (unsigned q = blockIdx.x * blockDim.x + threadIdx.x; q < nq; q += gridDim.x * blockDim.x) {
-        const SegItem32 it = sq.wq[q];
-        const int64_t i = it.i;
-        const int t = a.p.tet[i];
-        const Walk32 w = walk32(a, t, it.x0, it.y0, it.z0, a.p.x[i], a.p.y[i], a.p.z[i], max_cross);
-        cross += unsigned(w.crossings);
-        a.p.x[i] = w.hx;
-        a.p.y[i] = w.hy;
-        a.p.z[i] = w.hz;
-        const uint32_t idf = a.p.idf[i];
-        if (w.status == W_SURFACE) {
-            atomicAdd(tri_count + w.tri, 1u);
-            a.p.idf[i] = idf | kSettled;
-            settled++;
-        } else if (w.status != W_INSIDE) {
-            a.p.idf[i] = idf | kLost;
-            lost++;
-            if (w.status == W_CAP) capped++;
+        const unsigned test = __ballot_sync(kFull, need == kNeedTest);
+        const bool side = need == kNeedTest && nt + __popc(test & below) < kTestQ;
+        const unsigned main_q = __ballot_sync(kFull, need != 0 && !side);
+        if (need) {
+            const int k = side ? kWalkQ + nt + __popc(test & below) : np + __popc(main_q & below);
+            Q.w[0][k] = x;
+            Q.w[1][k] = y;
+            Q.w[2][k] = z;
+            Q.w[3][k] = nx;
+            Q.w[4][k] = ny;
+            Q.w[5][k] = nz;
+            Q.w[6][k] = vx;
+            Q.w[7][k] = vy;
+            Q.w[8][k] = vz;
+            Q.w[9][k] = __int_as_float(tet);
+            Q.w[10][k] = __uint_as_float(idf);
+            Q.w[11][k] = __int_as_float(i);
+            Q.w[12][k] = __int_as_float(j << kFlagBits | need);
+            Q.w[13][k] = __uint_as_float(uint32_t(cand));
+            Q.w[14][k] = __uint_as_float(uint32_t(cand >> 32));
+        } else if (dirty) {
+            a.m.p.x[i] = x;
+            a.m.p.y[i] = y;
+            a.m.p.z[i] = z;
+            a.m.p.vx[i] = vx;
+            a.m.p.vy[i] = vy;
+            a.m.p.vz[i] = vz;
+            a.m.p.tet[i] = tet;
         }
-        if (w.tet != t) {
-            a.p.tet[i] = w.tet;
-            if (w.status == W_INSIDE) refresh_tet(f.stamp, f.epoch, w.tet, [&f](int tt) { field_of_tet32(f, tt); });
-        }
-        if (w.status == W_INSIDE && it.step + 1 < sq.L) {
-            const unsigned act = __activemask();
-            const int lane = threadIdx.x & 31;
-            const int leader = __ffs(act) - 1;
-            unsigned base = 0;
-            if (lane == leader) base = atomicAdd(sq.rq_n + r, unsigned(__popc(act)));
-            base = __shfl_sync(act, base, leader);
-            sq.rq[base + __popc(act & ((1u << lane) - 1u))] = make_int2(int(i), it.step + 1);
-        }
+        np += __popc(main_q);
+        nt += min(__popc(test), kTestQ - nt);
+        __syncwarp();
     }
-    const unsigned long long s0 = __reduce_add_sync(kFull, cross), s1 = __reduce_add_sync(kFull, settled);
-    const unsigned long long s2 = __reduce_add_sync(kFull, lost), s3 = __reduce_add_sync(kFull, capped);
-    if ((threadIdx.x & 31) == 0) {
-        if (s0) atomicAdd(&ctr->crossings, s0);
-        if (s1) atomicAdd(&ctr->settled, s1);
-        if (s2) atomicAdd(&ctr->lost, s2);
-        if (s3) atomicAdd(&ctr->capped, s3);
+    // one atomic per counter and warp
+    const unsigned long long n0 = __reduce_add_sync(kFull, processed), n1 = __reduce_add_sync(kFull, coll);
+    const unsigned long long n2 = __reduce_add_sync(kFull, lost), n3 = __reduce_add_sync(kFull, cross);
+    const unsigned long long n4 = __reduce_add_sync(kFull, settled), n5 = __reduce_add_sync(kFull, capped);
+    if (lane == 0) {
+        if (n0) atomicAdd(&a.ctr->processed, n0);
+        if (n1) atomicAdd(&a.ctr->collisions, n1);
+        if (n2) atomicAdd(&a.ctr->lost, n2);
+        if (n3) atomicAdd(&a.ctr->crossings, n3);
+        if (n4) atomicAdd(&a.ctr->settled, n4);
+        if (n5) atomicAdd(&a.ctr->capped, n5);
     }
-}
-
-// Round r's resume pass: the walked particles run on in registers from the
-// step after their walk; their next walk goes to round r + 1. (Ordering each
-// block's items by first step, so that a warp's lanes run the same steps,
-// cost more in block barriers than it saved in idle lanes.)
-__global__ void __launch_bounds__(256, 3) k_seg_resume32(MixedArgs a, StepConst c, SegQueues sq, int r,
-                                                         DevCounters *ctr) {
-    pdl_sync();
-    const unsigned nr = sq.rq_n[r];
-    unsigned processed = 0, coll = 0, lost = 0;
-    for (unsigned q = blockIdx.x * blockDim.x + threadIdx.x; q < nr; q += gridDim.x * blockDim.x) {
-        const int2 it = sq.rq[q];
-        const Words32 w = load_words32(a.p, it.x);
-        seg_steps32(a, c, it.x, w, it.y, sq, sq.wq_n + r + 1, processed, coll, lost);
-    }
-    add_step_counters(ctr, processed, coll, lost);
 }
 
 // round(x * 2^k) of a float (k <= 52), to nearest with ties to even, from the
@@ -1105,43 +1161,20 @@ void launch_step32(const DevParticles32 &p, int64_t n, const MeshDev32 &m, const
                                             land, c.step, f);
 }
 
-int launch_segment32(const DevParticles32 &p, int64_t n, const MeshDev32 &m, const StepConst &c, int L,
-                     unsigned int *tri_count, void *wq, int2 *rq, unsigned int *q_n, DevCounters *ctr,
-                     const FieldArgs &f, cudaStream_t s) {
-    if (n <= 0 || L <= 0 || L > kMaxSegment) return 0;
-    const MixedArgs a = make_args(p, n, m);
-    SegQueues sq;
-    sq.wq = static_cast<SegItem32 *>(wq);
-    sq.rq = rq;
-    sq.wq_n = q_n;
-    sq.rq_n = q_n + L + 1;
-    sq.L = L;
-    cudaMemsetAsync(q_n, 0, sizeof(unsigned int) * size_t(2 * L + 1), s);
-    // one wave of each kernel: SMs x resident blocks (same on every device of this build)
-    static int seg_blocks = 0, walk_blocks = 0, resume_blocks = 0;
-    if (!seg_blocks) {
-        int dev = 0, sms = 0, b0 = 0, b1 = 0, b2 = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b0, k_seg32, 256, 0);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b1, k_seg_walk32, 128, 0);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b2, k_seg_resume32, 256, 0);
-        walk_blocks = std::max(1, sms * std::max(1, b1));
-        resume_blocks = std::max(1, sms * std::max(1, b2));
-        seg_blocks = std::max(1, sms * std::max(1, b0));
-    }
-    const unsigned grid = unsigned(std::min<int64_t>(grid_for(n, 256), seg_blocks));
-    k_seg32<<<grid, 256, 0, s>>>(a, c, sq, ctr);
-    int launches = 1;
-    for (int r = 0; r < L; ++r) {
-        launch_pdl(k_seg_walk32, walk_blocks, 128, s, a, c.max_cross, sq, r, tri_count, ctr, f);
-        ++launches;
-        if (r + 1 < L) {
-            launch_pdl(k_seg_resume32, resume_blocks, 256, s, a, c, sq, r, ctr);
-            ++launches;
-        }
-    }
-    return launches;
+void launch_segment32(const DevParticles32 &p, int64_t n, const MeshDev32 &m, const StepConst &c, int L,
+                      unsigned int *tri_count, DevCounters *ctr, const FieldArgs &f, uint32_t seq, cudaStream_t s) {
+    if (n <= 0 || L <= 0 || L > kMaxSegment) return;
+    const Seg32 a{make_args(p, n, m), tri_count, ctr, L, seq};
+    // one wave: SMs x resident blocks (same on every device of this build);
+    // few particles spread over smaller blocks so that every SM has some
+    static int r = 0;
+    constexpr int kT = 128;
+    constexpr size_t smem = sizeof(WarpQueue) * kT / 32;
+    static_assert(smem <= 48 * 1024, "a block's queues fit the default limit of dynamic shared memory");
+    if (r == 0) r = resident_blocks(k_seg32, kT, smem);
+    const int T = n >= int64_t(r) * kT ? kT : 32;
+    const unsigned grid = unsigned(std::min<int64_t>(grid_for(n, T), int64_t(r) * (kT / T)));
+    k_seg32<<<grid, T, smem * T / kT, s>>>(a, c, f);
 }
 
 void launch_deposit32(const DevParticles32 &p, int64_t n, const MeshDev32 &m, int k, unsigned long long *node_fix,

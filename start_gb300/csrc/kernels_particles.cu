@@ -23,6 +23,7 @@
 #include "field.cuh"
 #include "exact_div.h"
 #include "screen.h"
+#include "segment.cuh"
 #include "sort_block.cuh"
 #include "spg_internal.h"
 
@@ -448,15 +449,7 @@ __device__ __noinline__ int prepare64(const Seg64 &a, const StepConst &c, WarpPo
         const double vx = a.p.vx[i], vy = a.p.vy[i], vz = a.p.vz[i];
         const Push64 h = load_push(a.m.rec, tet);
         unsigned long long cand = 0ull;
-        if (c.model != SPG_COLL_NONE) {
-            const int first = int(uint32_t(c.step) & 15u);
-            for (int g = 0; 16 * g < first + a.L; ++g) {
-                const unsigned long long m = candidate_mask(
-                    candidate_block(uint64_t(c.step) + 16ull * uint64_t(g), idf & kIdMask, c.seed_lo, c.seed_hi));
-                const int at = 16 * g - first;
-                cand |= at >= 0 ? m << at : m >> -at;
-            }
-        }
+        if (c.model != SPG_COLL_NONE) cand = segment_candidates(c, idf & kIdMask, a.L);
         put_ready(P, kPool - 1 - nr - __popc(go & ((1u << lane) - 1u)), x, y, z, h, vx, vy, vz, tet, idf, int(i), kNew,
                   __longlong_as_double((long long)cand));
     }

@@ -342,11 +342,9 @@ void launch_step32(const DevParticles32 &p, int64_t n, const MeshDev32 &m, const
 void launch_refresh32(const DevParticles32 &p, int64_t n, const FieldArgs &f, cudaStream_t s);
 // Steps c.step .. c.step + L - 1 of the mixed form with nothing between them
 // (no solve, re-sort, track record or landing record), bit-identical to L
-// launch_step32 calls: wq holds n items of 20 B, rq n int2, q_n 2 L + 1
-// counters. Returns the number of kernels launched.
-int launch_segment32(const DevParticles32 &p, int64_t n, const MeshDev32 &m, const StepConst &c, int L,
-                     unsigned int *tri_count, void *wq, int2 *rq, unsigned int *q_n, DevCounters *ctr,
-                     const FieldArgs &f, cudaStream_t s);
+// launch_step32 calls. seq as for launch_segment64.
+void launch_segment32(const DevParticles32 &p, int64_t n, const MeshDev32 &m, const StepConst &c, int L,
+                      unsigned int *tri_count, DevCounters *ctr, const FieldArgs &f, uint32_t seq, cudaStream_t s);
 
 // adjoint of the FP32 form (kernels_mixed.cu)
 void launch_copy_alive32(const DevParticles32 &src, const DevParticles32 &dst, int64_t n, cudaStream_t s);
