@@ -7,7 +7,14 @@
 
 #include <cstdint>
 
+#include "spg_internal.h"
+
 namespace spg {
+
+// Sets or clears kRecEzero of a mixed-form record, whose other flags stay.
+__device__ __forceinline__ void set_rec_ezero(TetRec32 &r, bool zero) {
+    *reinterpret_cast<uint8_t *>(&r.ezero) = zero ? uint8_t(kRecEzero) : uint8_t(0);
+}
 
 template <class F>
 __device__ __forceinline__ void refresh_tet(uint32_t *stamp, uint32_t epoch, int t, F compute) {

@@ -450,7 +450,7 @@ __device__ __forceinline__ void store_field32(const FieldArgs &f, int64_t t, con
         f.efield[3 * t + k] = v.E[k];
         f.rec32[t].H[k] = v.H[k];
     }
-    f.rec32[t].ezero = (f.rec32[t].ezero & kRecInterior) | (v.zero ? kRecEzero : 0u);
+    set_rec_ezero(f.rec32[t], v.zero);
 }
 
 __device__ __forceinline__ void field_of_tet32(const FieldArgs &f, int64_t t) {

@@ -275,7 +275,7 @@ int32_t *sort_offsets(int32_t *scratch);
 // the FP32 rounding of centroid + local position, so a particle inside it
 // passes the box test: the test is skipped).
 constexpr uint32_t kRecEzero = 1u;
-constexpr uint32_t kRecInterior = 2u;
+constexpr uint32_t kRecInterior = 0x100u;  // in a byte of its own: kRecEzero is set without reading it
 struct alignas(64) TetRec32 {
     float M[9];
     float H[3];
@@ -321,10 +321,12 @@ struct DevParticles32 {
 // Upload and location in one kernel from device-readable caller arrays of n
 // particles (ids 0..n-1): the FP64 form's state into p (cen == nullptr) or
 // the mixed form's into q (cen: FP64 centroids); lost (zeroed by the caller)
-// receives the count of particles outside the mesh.
+// receives the count of particles outside the mesh. The field of tets
+// [0, zero_tets) is set to zero meanwhile (as launch_zero_field).
 void launch_upload(const double *pos, const double *vel, int64_t n, const MeshDev &m, const int32_t *vox_seed,
                    const double *oi, const int32_t *dims, int max_cross, const DevParticles &p,
-                   const DevParticles32 &q, const double *cen, unsigned long long *lost, cudaStream_t s);
+                   const DevParticles32 &q, const double *cen, unsigned long long *lost, const FieldArgs &f,
+                   int64_t zero_tets, cudaStream_t s);
 
 struct MeshDev32 {
     const TetRec32 *rec;
