@@ -7,16 +7,23 @@
 // in tet-sorted order: a beam puts thousands of particles in a tet) adds the
 // weights to per-lane running sums and reduces them only when its tet
 // changes. In other tiles (the ends of runs, and particles that moved to
-// other tets since the last re-sort) the lanes with equal tets (match_any)
-// are summed by the integer reduce unit. Either way the lowest lane adds the
-// tet's four sums to the block's table of tets in shared memory: one probe,
-// four adds to adjacent words. The table is flushed into the node
-// accumulators at the end of the range (four global atomics per listed tet),
-// and also every kDepCheckTiles tiles if it is more than half full, so a
-// range whose particles are spread over many tets keeps aggregating. While
+// other tets since the last re-sort) every run of equal tets is summed by
+// prefix sums. Either way the first lane adds the tet's four sums to the block's
+// table of tets in shared memory: one probe, four adds. The table is flushed
+// into the node accumulators at the end of the range (four global atomics per
+// listed tet), and also every kDepCheckTiles tiles if it is more than half full,
+// so a range whose particles are spread over many tets keeps aggregating. While
 // the table is over half full a tet it does not hold goes to the node
 // accumulators directly. Integer sums do not depend on order, so the result
 // is the same as one atomic per particle.
+//
+// us per deposit, with a pass per key, 64-bit shared-memory adds (which are
+// compare-and-swap loops) and, in FP64, unfused weights -> now: 6e6 ions of a
+// Thompson source on 1.3e6 tets sorted 224 -> 147, ten and 19 steps after the
+// sort 269 -> 153 and 309 -> 164 (FP64), 54 -> 59, 144 -> 102 and 200 -> 108 (mixed
+// form); 3e6 all over 162,000 tets sorted 140 -> 90 and 65 -> 56, in random order
+// 438 -> 242 and 370 -> 202. FP64 is bound by the issue of the weights' twelve
+// instructions per particle (72 us for 3e6 at the measured rate).
 #ifndef SPG_DEPOSIT_CUH
 #define SPG_DEPOSIT_CUH
 
@@ -34,47 +41,33 @@ constexpr int kDepCheckTiles = 16;       // tiles between checks of the table's 
 
 struct DepositTable {
     int tet[kDepSlots];  // -1: free; a slot's tet does not change until the table is cleared
-    unsigned long long sum[kDepSlots][4];
+    unsigned int lo[kDepSlots][4], hi[kDepSlots][4];  // the sums' halves
     unsigned int held;
 };
 
-// Sums of v[0..3] over the lanes of this lane's group (equal keys); returns
-// the group's lane mask. v[1..3] are split into 21-bit pieces whose sums over
-// at most 32 lanes fit 32 bits (a weight is at most 2^52 in magnitude, so the
-// signed top piece v >> 42 is at most 2^10). When every weight of the warp is
-// below 2^41 in magnitude (one <= 2^41, more than 2e6 particles, and
-// barycentrics in about [-1, 1]) two pieces do: the signed v >> 21 is below
-// 2^20. v[0] = one - v[1] - v[2] - v[3] sums to count * one minus the others.
-__device__ __forceinline__ unsigned group_sums(int key, const long long v[4], long long one, long long sum[4]) {
+// Sums of v[0..3] over the run of equal keys that begins at this lane (heads:
+// the first lanes of the runs; other lanes' results are not used). Prefix sums
+// over the warp (modulo 2^64, exact whenever the run's sum fits 64 bits) and
+// their difference across the run: the same instructions for every warp,
+// where reductions over the lanes of each key (match_any and the integer reduce
+// unit) take a pass per key. v[0] = one - v[1] - v[2] - v[3] sums to count *
+// one minus the others.
+__device__ __forceinline__ void run_sums(unsigned heads, const long long v[4], long long one, long long sum[4]) {
     constexpr unsigned kAll = 0xffffffffu;
-    const unsigned grp = __match_any_sync(kAll, key);
-    bool big = false;
+    const int lane = threadIdx.x & 31;
+    const unsigned after = heads & ~((2u << lane) - 1u);
+    const int last = after ? __ffs(after) - 2 : 31;  // the run's last lane
 #pragma unroll
     for (int q = 1; q < 4; ++q) {
-        const long long t = v[q] >> 41;
-        big = big || (t != 0 && t != -1);
-    }
-    if (!__any_sync(kAll, big)) {
+        unsigned long long p = (unsigned long long)v[q];
 #pragma unroll
-        for (int q = 1; q < 4; ++q) {
-            const unsigned b0 = unsigned(v[q] & 0x1FFFFF);
-            const int b1 = int(v[q] >> 21);
-            const unsigned s0 = __reduce_add_sync(grp, b0);
-            const int s1 = __reduce_add_sync(grp, b1);
-            sum[q] = (long long)s0 + (long long)s1 * (1LL << 21);
+        for (int off = 1; off < 32; off <<= 1) {
+            const unsigned long long t = __shfl_up_sync(kAll, p, off);
+            if (lane >= off) p += t;
         }
-    } else {
-#pragma unroll
-        for (int q = 1; q < 4; ++q) {
-            const unsigned b0 = unsigned(v[q] & 0x1FFFFF), b1 = unsigned((v[q] >> 21) & 0x1FFFFF);
-            const int b2 = int(v[q] >> 42);
-            const unsigned s0 = __reduce_add_sync(grp, b0), s1 = __reduce_add_sync(grp, b1);
-            const int s2 = __reduce_add_sync(grp, b2);
-            sum[q] = (long long)s0 + (long long)s1 * (1LL << 21) + (long long)s2 * (1LL << 42);
-        }
+        sum[q] = (long long)(__shfl_sync(kAll, p, last) - p + (unsigned long long)v[q]);
     }
-    sum[0] = (long long)__popc(grp) * one - sum[1] - sum[2] - sum[3];
-    return grp;
+    sum[0] = (long long)(last - lane + 1) * one - sum[1] - sum[2] - sum[3];
 }
 
 // Appends tet `key` to the list of occupied tets once per deposit (the
@@ -94,6 +87,15 @@ __device__ __forceinline__ void tet_to_nodes(int key, const unsigned long long s
     if (sum[1]) atomicAdd(node_fix + tn.y, sum[1]);
     if (sum[2]) atomicAdd(node_fix + tn.z, sum[2]);
     if (sum[3]) atomicAdd(node_fix + tn.w, sum[3]);
+}
+
+// *(hi, lo) += v by 32-bit shared-memory atomics: the one on the low halves
+// returns whether it carried. (A 64-bit add is a compare-and-swap loop there.)
+__device__ __forceinline__ void add_halves(unsigned int *lo, unsigned int *hi, unsigned long long v) {
+    const unsigned l = unsigned(v), h = unsigned(v >> 32);
+    const unsigned old = atomicAdd(lo, l);
+    const unsigned c = h + (old + l < l ? 1u : 0u);
+    if (c) atomicAdd(hi, c);
 }
 
 // Adds a tet's four sums to its slot (open addressing, linear probing). A
@@ -116,10 +118,8 @@ __device__ __forceinline__ void table_add(DepositTable &s, int key, const long l
             }
         }
         if (cur == key) {
-            atomicAdd(&s.sum[h][0], (unsigned long long)sum[0]);
-            atomicAdd(&s.sum[h][1], (unsigned long long)sum[1]);
-            atomicAdd(&s.sum[h][2], (unsigned long long)sum[2]);
-            atomicAdd(&s.sum[h][3], (unsigned long long)sum[3]);
+#pragma unroll
+            for (int q = 0; q < 4; ++q) add_halves(&s.lo[h][q], &s.hi[h][q], (unsigned long long)sum[q]);
             return;
         }
         h = (h + 1) & (kDepSlots - 1);
@@ -132,7 +132,8 @@ __device__ __forceinline__ void table_add(DepositTable &s, int key, const long l
 __device__ __forceinline__ void table_clear(DepositTable &s) {
     for (int k = threadIdx.x; k < kDepSlots; k += kDepThreads) {
         s.tet[k] = -1;
-        s.sum[k][0] = s.sum[k][1] = s.sum[k][2] = s.sum[k][3] = 0ull;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) s.lo[k][q] = s.hi[k][q] = 0u;
     }
     if (threadIdx.x == 0) s.held = 0u;
 }
@@ -141,7 +142,12 @@ __device__ __forceinline__ void table_clear(DepositTable &s) {
 __device__ __forceinline__ void table_flush(const DepositTable &s, const int4 *__restrict__ tet_nodes,
                                             unsigned long long *__restrict__ node_fix, const OccList &occ) {
     for (int k = threadIdx.x; k < kDepSlots; k += kDepThreads)
-        if (s.tet[k] >= 0) tet_to_nodes(s.tet[k], s.sum[k], tet_nodes, node_fix, occ);
+        if (s.tet[k] >= 0) {
+            unsigned long long sum[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) sum[q] = (unsigned long long)s.hi[k][q] << 32 | s.lo[k][q];
+            tet_to_nodes(s.tet[k], sum, tet_nodes, node_fix, occ);
+        }
 }
 
 // Warp sum of 64-bit values modulo 2^64 (three 21-bit pieces, the top one
@@ -220,8 +226,10 @@ __device__ __forceinline__ void deposit_tiles(const Src &src, int64_t n, const i
             acnt += key >= 0;
         } else {
             long long sum[4];
-            const unsigned grp = group_sums(key, v, src.one, sum);
-            if (key >= 0 && lane == __ffs(grp) - 1) table_add(s, key, sum, tet_nodes, node_fix, occ);
+            const int prev = __shfl_up_sync(kAll, key, 1);
+            const unsigned heads = __ballot_sync(kAll, lane == 0 || prev != key);
+            run_sums(heads, v, src.one, sum);
+            if (key >= 0 && ((heads >> lane) & 1u)) table_add(s, key, sum, tet_nodes, node_fix, occ);
         }
     }
     if (acc_key >= 0) flush_running(s, acc_key, a1, a2, a3, acnt, src.one, tet_nodes, node_fix, occ);
