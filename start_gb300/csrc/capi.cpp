@@ -184,8 +184,11 @@ struct spg_handle {
     // direct host access: the device reads pageable memory through the host
     // page tables (address translation over the C2C link)
     bool ats = false;
-    int32_t *id_slot = nullptr;  // slot of each id for direct downloads
+    int32_t *id_slot = nullptr;  // slot of each id for direct downloads; ranks during a re-sort
     int64_t id_slot_cap = 0;
+    void *sort_rec = nullptr;    // records of a re-sort from no order
+    size_t sort_rec_bytes = 0;
+    bool sorted = false;         // the particles have been re-sorted since they were set
     unsigned long long *io_counter = nullptr;
     double setup_ms[6] = {0, 0, 0, 0, 0, 0};  // spg_setup_times
     int64_t occupied = 0;
@@ -366,6 +369,9 @@ void free_particles(spg_handle *h) {
     }
     cudaFree(h->walkq);
     h->walkq = nullptr;
+    cudaFree(h->sort_rec);
+    h->sort_rec = nullptr;
+    h->sort_rec_bytes = 0;
     h->cap = 0;
 }
 
@@ -815,14 +821,47 @@ int copy_tail(spg_handle *h, T *dst, const T *src, int64_t o, int64_t n) {
     return SPG_OK;
 }
 
+int id_words(spg_handle *h, int64_t n) {
+    if (n <= h->id_slot_cap) return SPG_OK;
+    cudaFree(h->id_slot);
+    h->id_slot = nullptr;
+    h->id_slot_cap = 0;
+    CK(dalloc(&h->id_slot, n));
+    h->id_slot_cap = n;
+    return SPG_OK;
+}
+
+// The records and ranks for a re-sort of a set in no order; nullptr: histogram
+// and scatter. Below 65,536 particles the arrays stay in L2 and the route's
+// other kernel costs more (70,000: 17.6 against 18.7 us, 20,000: 15). Without
+// room for them the sort scatters.
+void *sort_records(spg_handle *h) {
+    if (h->sorted || h->n_active < 65536) return nullptr;
+    const size_t need = size_t(h->n_active) * (h->mixed ? 32 : 64);
+    if (need > h->sort_rec_bytes) {
+        cudaFree(h->sort_rec);
+        h->sort_rec = nullptr;
+        h->sort_rec_bytes = 0;
+        if (cudaMalloc(&h->sort_rec, need) == cudaSuccess)
+            h->sort_rec_bytes = need;
+        else
+            h->sort_rec = nullptr;
+    }
+    if (h->sort_rec && id_words(h, h->np) == SPG_OK) return h->sort_rec;
+    cudaGetLastError();
+    return nullptr;
+}
+
 int do_resort(spg_handle *h) {
     if (!h->have_particles || h->np == 0) return SPG_OK;
+    void *rec = sort_records(h);
+    h->sorted = true;
     ev_begin(h, h->ev_sort);
     const int64_t tail = h->np - h->n_active, o = h->n_active;
     int rc = SPG_OK;
     if (h->mixed) {
         DevParticles32 &src = h->Q[h->cur], &dst = h->Q[1 - h->cur];
-        launch_resort32(src, dst, h->n_active, h->n_tets, h->sort_scratch, h->n_alive_dev, h->stream);
+        launch_resort32(src, dst, h->n_active, h->n_tets, h->sort_scratch, h->id_slot, rec, h->n_alive_dev, h->stream);
         // Particles past n_active are dead already; they keep their slots.
         if (tail > 0)
             for (auto pr : {std::make_pair(dst.x, src.x), std::make_pair(dst.y, src.y), std::make_pair(dst.z, src.z),
@@ -833,7 +872,7 @@ int do_resort(spg_handle *h) {
             return rc;
     } else {
         DevParticles &src = h->P[h->cur], &dst = h->P[1 - h->cur];
-        launch_resort(src, dst, h->n_active, h->n_tets, h->sort_scratch, h->n_alive_dev, h->stream);
+        launch_resort(src, dst, h->n_active, h->n_tets, h->sort_scratch, h->id_slot, rec, h->n_alive_dev, h->stream);
         if (tail > 0)
             for (auto pr : {std::make_pair(dst.x, src.x), std::make_pair(dst.y, src.y), std::make_pair(dst.z, src.z),
                             std::make_pair(dst.vx, src.vx), std::make_pair(dst.vy, src.vy),
@@ -843,7 +882,7 @@ int do_resort(spg_handle *h) {
             return rc;
     }
     ev_end(h, h->ev_sort);
-    h->launches += h->n_active > 0 ? 5 : 3;
+    h->launches += h->n_active > 0 ? (rec ? 6 : 5) : 3;
     CK(cudaGetLastError());
     int64_t na = 0;
     unsigned long long occ = 0;
@@ -1437,6 +1476,7 @@ int reset_run_state(spg_handle *h, bool field_zeroed = false) {
     h->charge_valid = false;
     h->occ_fresh = false;
     h->resorted_at = -1;
+    h->sorted = false;
     CK(cudaMemsetAsync(h->ctr, 0, sizeof(DevCounters), h->stream));
     CK(cudaMemsetAsync(h->tri_count, 0, sizeof(unsigned int) * std::max<int64_t>(h->n_tris, 1), h->stream));
     if (h->vac_valid)  // AMG: a new particle set starts from the electrode field
@@ -2162,13 +2202,8 @@ int spg_get_particles(spg_handle *h, int64_t n, double *pos, double *vel, int32_
         void *wp = pos ? device_writable(pos) : nullptr, *wv = vel ? device_writable(vel) : nullptr;
         void *wt = tet ? device_writable(tet) : nullptr, *wf = flags ? device_writable(flags) : nullptr;
         if ((!pos || wp) && (!vel || wv) && (!tet || wt) && (!flags || wf)) {
-            if (n > h->id_slot_cap) {
-                cudaFree(h->id_slot);
-                h->id_slot = nullptr;
-                h->id_slot_cap = 0;
-                CK(dalloc(&h->id_slot, n));
-                h->id_slot_cap = n;
-            }
+            const int rc = id_words(h, n);
+            if (rc) return rc;
             double *dp = static_cast<double *>(wp), *dv = static_cast<double *>(wv);
             int32_t *dt = static_cast<int32_t *>(wt);
             uint32_t *df = static_cast<uint32_t *>(wf);
@@ -2618,6 +2653,7 @@ int spg_restore(spg_handle *h, const void *buf, size_t bytes) {
     h->have_particles = true;
     h->occ_fresh = false;
     h->resorted_at = -1;
+    h->sorted = false;
     if (h->cg_solves == 0) {
         zero_field(h);
     } else {

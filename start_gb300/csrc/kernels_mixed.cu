@@ -936,6 +936,16 @@ __global__ void __launch_bounds__(kSortBlock) k_sort_scatter32(DevParticles32 sr
     sort_scatter_block(t, src, dst, n, n_tets, kDead, offs);
 }
 
+__global__ void __launch_bounds__(kSortBlock) k_sort_records32(DevParticles32 src, SortRec32 *rec, int64_t n, int n_tets,
+                                                               const int32_t *__restrict__ offs,
+                                                               const int32_t *__restrict__ rank) {
+    sort_to_records(src, rec, n, n_tets, kDead, offs, rank);
+}
+__global__ void __launch_bounds__(kSortBlock) k_sort_unpack32(const SortRec32 *__restrict__ rec, DevParticles32 dst,
+                                                              int64_t n) {
+    sort_unpack(rec, dst, n);
+}
+
 inline unsigned grid_for(int64_t n, int block) { return unsigned((n + block - 1) / block); }
 
 // ------------------------------------------------------------ adjoint (FP32 form)
@@ -1241,11 +1251,17 @@ void launch_gather32(const DevParticles32 &p, int64_t n, int32_t *slot, const do
 }
 
 void launch_resort32(const DevParticles32 &src, DevParticles32 dst, int64_t n, int64_t n_tets, int32_t *scratch,
-                     int64_t *n_alive_dev, cudaStream_t s) {
-    launch_sort_prepare(src.tet, src.idf, n, n_tets, scratch, n_alive_dev, s);
-    if (n > 0)
-        k_sort_scatter32<<<grid_for(n, kSortBlock), kSortBlock, 0, s>>>(src, dst, n, int(n_tets),
-                                                                        sort_offsets(scratch));
+                     int32_t *rank, void *records, int64_t *n_alive_dev, cudaStream_t s) {
+    launch_sort_prepare(src.tet, src.idf, n, n_tets, scratch, records ? rank : nullptr, n_alive_dev, s);
+    if (n <= 0) return;
+    const unsigned grid = grid_for(n, kSortBlock);
+    if (records) {
+        SortRec32 *rec = static_cast<SortRec32 *>(records);
+        k_sort_records32<<<grid, kSortBlock, 0, s>>>(src, rec, n, int(n_tets), sort_offsets(scratch), rank);
+        k_sort_unpack32<<<grid, kSortBlock, 0, s>>>(rec, dst, n);
+    } else {
+        k_sort_scatter32<<<grid, kSortBlock, 0, s>>>(src, dst, n, int(n_tets), sort_offsets(scratch));
+    }
 }
 
 size_t walk_item32_bytes() { return sizeof(WalkItem32); }

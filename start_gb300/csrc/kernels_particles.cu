@@ -1100,6 +1100,16 @@ __global__ void __launch_bounds__(kSortBlock) k_sort_hist(const int32_t *__restr
     sort_hist_block(t, key, cnt);
 }
 
+__global__ void __launch_bounds__(kSortBlock) k_sort_rank(const int32_t *__restrict__ tet,
+                                                          const uint32_t *__restrict__ idf, int64_t n, int n_tets,
+                                                          int32_t *__restrict__ cnt, int32_t *__restrict__ rank) {
+    __shared__ SortTable t;
+    const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+    const int key = i < n ? ((idf[i] & kDead) ? n_tets : tet[i]) : -1;
+    const int r = sort_rank_block(t, key, n_tets, cnt);
+    if (i < n) rank[i] = r;
+}
+
 // Block-local exclusive scan of one tile; tile total to sums[blockIdx.x].
 // Also counts non-empty tet bins (occupied tets).
 __global__ void __launch_bounds__(kScanThreads) k_scan_tile(int32_t *__restrict__ a, int64_t len, int n_tets,
@@ -1199,6 +1209,16 @@ __global__ void __launch_bounds__(kSortBlock) k_sort_scatter(DevParticles src, D
                                                              int32_t *__restrict__ offs) {
     __shared__ SortTable t;
     sort_scatter_block(t, src, dst, n, n_tets, kDead, offs);
+}
+
+__global__ void __launch_bounds__(kSortBlock) k_sort_records(DevParticles src, SortRec64 *rec, int64_t n, int n_tets,
+                                                             const int32_t *__restrict__ offs,
+                                                             const int32_t *__restrict__ rank) {
+    sort_to_records(src, rec, n, n_tets, kDead, offs, rank);
+}
+__global__ void __launch_bounds__(kSortBlock) k_sort_unpack(const SortRec64 *__restrict__ rec, DevParticles dst,
+                                                            int64_t n) {
+    sort_unpack(rec, dst, n);
 }
 
 inline unsigned grid_for(int64_t n, int block) { return unsigned((n + block - 1) / block); }
@@ -1329,7 +1349,7 @@ unsigned long long *sort_occupied_counter(int32_t *scratch) {
 int32_t *sort_offsets(int32_t *scratch) { return scratch + 2; }
 
 void launch_sort_prepare(const int32_t *tet, const uint32_t *idf, int64_t n, int64_t n_tets, int32_t *scratch,
-                         int64_t *n_alive_dev, cudaStream_t s) {
+                         int32_t *rank, int64_t *n_alive_dev, cudaStream_t s) {
     const int64_t len = n_tets + 1;
     const int64_t nb = (len + kScanTile - 1) / kScanTile;
     unsigned long long *occupied = sort_occupied_counter(scratch);
@@ -1337,17 +1357,27 @@ void launch_sort_prepare(const int32_t *tet, const uint32_t *idf, int64_t n, int
     int32_t *sums = cnt + len;
     cudaMemsetAsync(cnt, 0, sizeof(int32_t) * len, s);
     cudaMemsetAsync(occupied, 0, sizeof(unsigned long long), s);
-    if (n > 0) k_sort_hist<<<grid_for(n, kSortBlock), kSortBlock, 0, s>>>(tet, idf, n, int(n_tets), cnt);
+    if (n > 0 && rank)
+        k_sort_rank<<<grid_for(n, kSortBlock), kSortBlock, 0, s>>>(tet, idf, n, int(n_tets), cnt, rank);
+    else if (n > 0)
+        k_sort_hist<<<grid_for(n, kSortBlock), kSortBlock, 0, s>>>(tet, idf, n, int(n_tets), cnt);
     k_scan_tile<<<unsigned(nb), kScanThreads, 0, s>>>(cnt, len, int(n_tets), sums, occupied);
     k_scan_sums<<<1, 1024, 0, s>>>(sums, nb);
     k_scan_add<<<grid_for(len, 256), 256, 0, s>>>(cnt, len, sums, int(n_tets), n_alive_dev);
 }
 
 void launch_resort(const DevParticles &src, DevParticles dst, int64_t n, int64_t n_tets, int32_t *scratch,
-                   int64_t *n_alive_dev, cudaStream_t s) {
-    launch_sort_prepare(src.tet, src.idf, n, n_tets, scratch, n_alive_dev, s);
-    if (n > 0)
-        k_sort_scatter<<<grid_for(n, kSortBlock), kSortBlock, 0, s>>>(src, dst, n, int(n_tets), sort_offsets(scratch));
+                   int32_t *rank, void *records, int64_t *n_alive_dev, cudaStream_t s) {
+    launch_sort_prepare(src.tet, src.idf, n, n_tets, scratch, records ? rank : nullptr, n_alive_dev, s);
+    if (n <= 0) return;
+    const unsigned grid = grid_for(n, kSortBlock);
+    if (records) {
+        SortRec64 *rec = static_cast<SortRec64 *>(records);
+        k_sort_records<<<grid, kSortBlock, 0, s>>>(src, rec, n, int(n_tets), sort_offsets(scratch), rank);
+        k_sort_unpack<<<grid, kSortBlock, 0, s>>>(rec, dst, n);
+    } else {
+        k_sort_scatter<<<grid, kSortBlock, 0, s>>>(src, dst, n, int(n_tets), sort_offsets(scratch));
+    }
 }
 
 }  // namespace spg

@@ -255,16 +255,18 @@ void launch_slot_of_id(const uint32_t *idf, int64_t n, int32_t *slot, cudaStream
 void launch_gather_by_id(const DevParticles &p, int64_t n, int32_t *slot, double *pos, double *vel,
                          int32_t *tet, uint32_t *flags, cudaStream_t s);
 // Re-sort: histogram, exclusive scan, scatter. Writes the number of alive
-// particles to *n_alive_dev. scratch must hold sort_scratch_words(n_tets) ints, 8-byte aligned.
+// particles to *n_alive_dev. scratch must hold sort_scratch_words(n_tets) ints,
+// 8-byte aligned. For particles in no order, with records (n of 64 bytes, 32 in
+// the mixed form) and rank (n ints) given, by way of those (sort_block.cuh).
 int64_t sort_scratch_words(int64_t n_tets);
 // Number of tets holding at least one alive particle at the last re-sort.
 unsigned long long *sort_occupied_counter(int32_t *scratch);
 void launch_resort(const DevParticles &src, DevParticles dst, int64_t n, int64_t n_tets, int32_t *scratch,
-                   int64_t *n_alive_dev, cudaStream_t s);
-// Histogram + exclusive scan of the sort keys; sort_offsets(scratch) then
+                   int32_t *rank, void *records, int64_t *n_alive_dev, cudaStream_t s);
+// Histogram (and ranks, if not nullptr) and exclusive scan of the sort keys; sort_offsets(scratch) then
 // holds the first slot of every key (tets, then n_tets for dead particles).
 void launch_sort_prepare(const int32_t *tet, const uint32_t *idf, int64_t n, int64_t n_tets, int32_t *scratch,
-                         int64_t *n_alive_dev, cudaStream_t s);
+                         int32_t *rank, int64_t *n_alive_dev, cudaStream_t s);
 int32_t *sort_offsets(int32_t *scratch);
 
 // ---------------------------------------------------------- mixed precision
@@ -365,7 +367,7 @@ void launch_to_local(const double *pos, const double *vel, const int32_t *tet, c
 void launch_gather32(const DevParticles32 &p, int64_t n, int32_t *slot, const double *cen, double *pos, double *vel,
                      int32_t *tet, uint32_t *flags, cudaStream_t s);
 void launch_resort32(const DevParticles32 &src, DevParticles32 dst, int64_t n, int64_t n_tets, int32_t *scratch,
-                     int64_t *n_alive_dev, cudaStream_t s);
+                     int32_t *rank, void *records, int64_t *n_alive_dev, cudaStream_t s);
 size_t walk_item32_bytes();
 
 // PCG (kernels_pcg.cu).
