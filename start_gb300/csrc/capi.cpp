@@ -124,7 +124,7 @@ struct spg_handle {
     // Jacobi PCG of a system that fits on the chip, one launch per solve
     // (blocks == 0: it does not fit, or AMG is selected)
     ResidentPlan resident;
-    double2 *res_zp = nullptr;        // two arrays of n_nodes pairs
+    ZpuRec *res_zpu = nullptr;        // two arrays of n_nodes records
     double *res_partials = nullptr;
     unsigned int *res_arrived = nullptr;
     // PCG iterations are replayed as a CUDA graph of kPcgChunk iterations
@@ -1036,8 +1036,8 @@ int launch_resident(spg_handle *h, const double *b, double *x) {
     a.inv_diag = h->inv_diag;
     a.b = b;
     a.x = x;
-    a.zp[0] = h->res_zp;
-    a.zp[1] = h->res_zp + h->n_nodes;
+    a.zpu[0] = h->res_zpu;
+    a.zpu[1] = h->res_zpu + h->n_nodes;
     a.partials = h->res_partials;
     a.arrived = h->res_arrived;
     a.sc = h->sc;
@@ -1747,7 +1747,7 @@ int spg_create(const spg_mesh_desc *mesh, const spg_params *params, spg_handle *
     if (!h->amg && !h->amg32) h->resident = resident_plan(n);
     CK(cudaGetLastError());
     if (h->resident.blocks > 0) {
-        CK(dalloc(&h->res_zp, 2 * size_t(n)));
+        CK(dalloc(&h->res_zpu, 2 * size_t(n)));
         CK(dalloc(&h->res_partials, kResidentPartials));
         CK(dalloc(&h->res_arrived, 1));
     }
@@ -1800,7 +1800,7 @@ int spg_destroy(spg_handle *h) {
                     h->gE,       h->lam,      h->mu,       h->dJdg,    h->sums, h->hist64, h->hist.tet, h->hist.vx,
                     h->hist.vy,  h->hist.vz,  h->tri_scratch, h->ctr_scratch,
                     h->q,        h->partials, h->sc,       h->tri_count, h->ctr,      h->n_alive_dev, h->sort_scratch, h->walkq_n,
-                    h->io,       h->res_zp,  h->res_partials, h->res_arrived};
+                    h->io,       h->res_zpu,  h->res_partials, h->res_arrived};
     for (void *ptr : ptrs) cudaFree(ptr);
     for (EventSeries *s : {&h->ev_step, &h->ev_dep, &h->ev_pcg, &h->ev_ef, &h->ev_sort}) ev_destroy(*s);
     for (void *ptr : h->amg_alloc) cudaFree(ptr);

@@ -2,35 +2,40 @@
 //
 // The system lives on the chip for the whole solve: one thread per row holds
 // x, r, p and the inverse diagonal in registers and its matrix row in shared
-// memory, and the search direction's ingredients {z, p} of every row lie in a
-// pair of small arrays. An iteration is
-//   phase A  p_k = z + beta p (own row, and again at every gathered column, so
-//            that no pass and no barrier is spent on the p update), q = A p_k,
-//            reduction of p.q;
-//   phase B  x += alpha p, r -= alpha q, z = D^-1 r, {z, p} of the row stored
-//            into the other array of the pair, reduction of r.z and r.r.
-// Every value is formed by the operations of the separate kernels (k_spmv_dot,
-// k_update, k_pupdate); only the sums over the rows (and the place of the
-// diagonal in a row's sum) are taken in another fixed order, so a solve is
-// deterministic and differs from those kernels by rounding alone.
+// memory, and what other rows need of a row, its record {z, p, u = D^-1 A p},
+// lies in a pair of small arrays. An iteration has one exchange of sums:
+//   p = z + beta p, q = A p (of a coupled row, z less alpha u and p plus beta
+//   times the published p, so that no pass and no barrier is spent on the
+//   updates), {z, p, u} stored into the other array of the pair;
+//   the sums p.q, z.q, u.q, r.z and r.r over all rows;
+//   alpha = r.z / p.q; x += alpha p, r -= alpha q, z = D^-1 r.
+// The next r.z, which beta needs before the next sums, is predicted from this
+// exchange, r.z - 2 alpha z.q + alpha^2 u.q, and formed from the vectors in the
+// next one, so no rounding of a prediction is carried on ("predict and
+// recompute", Chen and Carson, SIAM J. Sci. Comput. 42, 2020). The stop test
+// sees r.r of an update one exchange later, before anything else is updated.
+// With the values of k_spmv_dot, k_update and k_pupdate it differs by rounding
+// alone (solves of up to 190 iterations: 1e-15 of x), and every sum has a fixed
+// order, so a solve is deterministic.
 //
-// What bounds it is latency: two exchanges of sums per iteration, each a tree
-// over the block, a barrier over the blocks and a tree over their partial
-// sums. On GB300 an FP64 instruction holds its warp's scheduler for 63 cycles
-// (about 1.7 operations per clock and SM in all), a division takes 1,470.
+// What bounds it is latency: the exchange (a tree over the block, a barrier over
+// the blocks, a tree over their partial sums) and the FP64 chains around it. On
+// GB300 an FP64 instruction holds its warp's scheduler for 63 cycles (about 1.7
+// operations per clock and SM in all), a division takes 1,470.
 // Two forms:
-//   * cluster: up to 16 blocks in one cluster, {z, p} in distributed shared
+//   * cluster: up to 16 blocks in one cluster, the records in distributed shared
 //     memory, the hardware barrier (400 to 600 cycles). Its 16 SMs issue few
-//     FP64 operations, so it ends where the grid becomes faster, about 6,000
-//     rows: 5.5 us an iteration at 4,096 rows and 6.0 at 5,832 (cluster),
-//     6.5 at 6,859 (grid), 6.8 at 4,913 in the grid form.
-//   * grid: up to one block per SM, cooperative launch, {z, p} in L2, a counter
+//     FP64 operations, so it ends where the grid becomes faster, at 4,096 rows:
+//     us an iteration, cluster / grid, 1,331 rows 4.1 / 5.3, 3,375 4.9 / 5.3,
+//     4,096 5.2 / 5.3, 4,913 5.8 / 5.4.
+//   * grid: up to one block per SM, cooperative launch, the records in L2, a counter
 //     in global memory as the barrier (1.2 us). It ends at one row per thread,
 //     155,648 rows on 152 SMs.
-// Measured per iteration of the lattice Laplacian, three kernels per iteration
-// in a graph before -> here: 1,331 rows 22 -> 4.4 us, 17,576 rows 22 -> 7.0,
-// 132,651 rows 24 -> 12.4; of a caller's CSR system with 68,921 rows (three
-// launches per iteration, the host asking every eight) 64 -> 9.1.
+// Measured per iteration of the lattice Laplacian: three kernels per iteration in
+// a graph; one launch with two exchanges per iteration ({z, p} published); one
+// exchange: 1,331 rows 22, 4.4, 4.1 us; 5,832 rows -, 6.0, 5.2; 17,576 rows 22, 7.0,
+// 5.6; 68,921 rows -, 9.1, 8.8; 132,651 rows 24, 12.4, 13.5 (there the FP64 pipe is
+// full and the gathers' second multiply-add costs what the exchange saves).
 #include <algorithm>
 #include <cmath>
 #include <cstdint>
@@ -43,7 +48,7 @@ namespace spg {
 namespace {
 
 constexpr unsigned kFull = 0xffffffffu;
-constexpr int kMaxSums = 4;
+constexpr int kSums = kResidentSums;
 constexpr int kMaxCluster = 16;
 // Polls of the grid barrier before a block gives up (each takes most of a
 // microsecond): a few seconds. The cooperative launch makes every block
@@ -90,18 +95,24 @@ __device__ __forceinline__ RowRef row_ref(const ResidentArgs &a, int i) {
     return RowRef{k0, 1, k1 - k0};
 }
 
-struct Zp {
-    double z, p;
+// What a row publishes for the rows coupled to it.
+struct Zpu {
+    double z, p, u;
 };
 
-__device__ __forceinline__ Zp load_zp(const double2 *p) {
-    Zp r;  // not a read-only load: other blocks write the array between the barriers
-    asm volatile("ld.global.v2.f64 {%0, %1}, [%2];" : "=d"(r.z), "=d"(r.p) : "l"(p) : "memory");
+__device__ __forceinline__ Zpu load_zpu(const ZpuRec *p) {
+    Zpu r;  // not a read-only load: other blocks write the array between the barriers
+    double unused;
+    asm volatile("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];"
+                 : "=d"(r.z), "=d"(r.p), "=d"(r.u), "=d"(unused)
+                 : "l"(p)
+                 : "memory");
     return r;
 }
-__device__ __forceinline__ Zp load_zp_cluster(uint32_t addr) {
-    Zp r;
+__device__ __forceinline__ Zpu load_zpu_cluster(uint32_t addr) {
+    Zpu r;
     asm volatile("ld.shared::cluster.v2.f64 {%0, %1}, [%2];" : "=d"(r.z), "=d"(r.p) : "r"(addr) : "memory");
+    asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(r.u) : "r"(addr + 16u) : "memory");
     return r;
 }
 
@@ -116,67 +127,85 @@ __device__ __forceinline__ void cluster_barrier() {
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
-// Sum over the first 2 * FROM lanes of a warp (result in lane 0).
-template <int FROM>
-__device__ __forceinline__ double warp_sum(double v) {
-#pragma unroll
-    for (int off = FROM; off > 0; off >>= 1) v += __shfl_down_sync(kFull, v, off);
-    return v;
-}
-
 struct Shared {
-    double tot[kMaxSums];                   // the totals of the last exchange
-    double part[2][kMaxSums][kMaxCluster];  // cluster form: every block's partial sums
-    double alpha, beta, inv_rz;
+    double tot[kSums];                   // the totals of the last exchange
+    double warp[4][kSums];               // the sums of the first four warps' columns
+    double part[2][kSums][kMaxCluster];  // cluster form: every block's partial sums
+    double alpha, beta;
     int stop, timed_out;
 };
 
-// One exchange: the totals over all rows of the n values per thread in
-// buf[k T + t], into s.tot[k] by warp k modulo the block's warps (other warps
-// read them after the caller's barrier). Everything the block wrote before is
-// visible to every block afterwards. An FP64 instruction holds its warp's
-// scheduler for 63 cycles whatever its lanes and independence, so at most four
-// warps first add the columns of a large block, one per scheduler, and each
-// value then has a warp of its own. target: arrivals after which this
-// exchange is complete (grid form). Out of line: one copy for every phase.
+// v[k] summed over the warp; lane 16 (k & 1) + 8 (k >> 1) gets value k < 4, lane
+// 4 value 4. Lanes hand over the value they do not keep, so the five sums take
+// eight FP64 additions instead of 25.
+__device__ __forceinline__ double warp_sums(const double (&v)[kSums]) {
+    const int lane = threadIdx.x & 31;
+    const bool b4 = lane & 16, b3 = lane & 8, b2 = lane & 4;
+    const double x01 = (b4 ? v[1] : v[0]) + __shfl_xor_sync(kFull, b4 ? v[0] : v[1], 16);
+    const double x23 = (b4 ? v[3] : v[2]) + __shfl_xor_sync(kFull, b4 ? v[2] : v[3], 16);
+    double x4 = v[4] + __shfl_xor_sync(kFull, v[4], 16);
+    const double y = (b3 ? x23 : x01) + __shfl_xor_sync(kFull, b3 ? x01 : x23, 8);
+    x4 += __shfl_xor_sync(kFull, x4, 8);
+    double w = (b2 ? x4 : y) + __shfl_xor_sync(kFull, b2 ? y : x4, 4);
+    w += __shfl_xor_sync(kFull, w, 2);
+    w += __shfl_xor_sync(kFull, w, 1);
+    return w;
+}
+
+// One exchange: the totals over all rows of the five values per thread in
+// buf[k T + t], into s.tot[k] (read after the caller's barrier). Everything the
+// block wrote before is visible to every block afterwards. An FP64 instruction
+// holds its warp's scheduler for 63 cycles whatever its lanes and independence,
+// so four warps, one per scheduler, add the columns of a large block and sum
+// five values together, and half a warp each sums two values over the blocks.
+// target: arrivals after which this exchange is complete (grid form). Out of
+// line: one copy for every call.
 template <bool CLUSTER>
 __device__ __noinline__ void exchange(double *partials, unsigned int *arrived, Shared &s, double *buf, unsigned par,
-                                      unsigned target, int n) {
+                                      unsigned target) {
     const int T = blockDim.x, t = threadIdx.x, lane = t & 31, wid = t >> 5, nw = T >> 5;
+    const int G = int(gridDim.x);
     __syncthreads();
-    if (T > 128) {
-        if (t < 128)
-            for (int k = 0; k < n; ++k) {
-                double w = buf[k * T + t];
-                for (int j = t + 128; j < T; j += 128) w += buf[k * T + j];
-                buf[k * T + t] = w;
-            }
-        __syncthreads();
+    if (t < 128) {
+        double v[kSums];
+#pragma unroll
+        for (int k = 0; k < kSums; ++k) v[k] = buf[k * T + t];
+        for (int j = t + 128; j < T; j += 128)
+#pragma unroll
+            for (int k = 0; k < kSums; ++k) v[k] += buf[k * T + j];
+        const double w = warp_sums(v);
+        if ((lane & 7) == 0) s.warp[wid][(lane >> 4) + 2 * ((lane >> 3) & 1)] = w;
+        if (lane == 4) s.warp[wid][4] = w;
     }
-    for (int k = wid; k < n; k += nw) {
-        const double *b = buf + k * T + lane;
-        double w = b[0] + b[32];
-        if (T > 64) w += b[64];
-        if (T > 96) w += b[96];
-        w = warp_sum<16>(w);
+    __syncthreads();
+    if (wid == 0) {
+        const int k = lane >> 2, w = lane & 3;
+        double q = k < kSums && w < nw ? s.warp[w][k] : 0.0;
+        q += __shfl_xor_sync(kFull, q, 1);
+        q += __shfl_xor_sync(kFull, q, 2);
         if constexpr (CLUSTER) {
-            w = __shfl_sync(kFull, w, 0);
-            if (unsigned(lane) < gridDim.x)
-                asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(
-                                 map_rank(shared_addr(&s.part[par][k][blockIdx.x]), unsigned(lane))),
-                             "d"(w)
-                             : "memory");
-        } else if (lane == 0) {
-            partials[(size_t(par) * kMaxSums + k) * gridDim.x + blockIdx.x] = w;
-            asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(arrived) : "memory");
+            for (int e0 = 0; e0 < kSums * G; e0 += 32) {  // value e % 5 to block e / 5
+                const int e = e0 + lane, rank = e / kSums, v = e - rank * kSums;
+                const double out = __shfl_sync(kFull, q, 4 * v);
+                if (rank < G)
+                    asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(
+                                     map_rank(shared_addr(&s.part[par][v][blockIdx.x]), unsigned(rank))),
+                                 "d"(out)
+                                 : "memory");
+            }
+        } else {
+            if (k < kSums && w == 0) partials[(size_t(par) * kSums + k) * G + blockIdx.x] = q;
+            __syncwarp();
+            if (lane == 0) asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(arrived) : "memory");
         }
     }
     if constexpr (CLUSTER) cluster_barrier();
-    for (int k = wid; k < n; k += nw) {
+    const int hl = lane & 15;
+    for (int k0 = 2 * wid; k0 < kSums; k0 += 2 * nw) {
+        const int k = k0 + (lane >> 4);
         double w = 0.0;
         if constexpr (CLUSTER) {
-            if (unsigned(lane) < gridDim.x) w = s.part[par][k][lane];
-            w = warp_sum<8>(w);
+            if (k < kSums && hl < G) w = s.part[par][k][hl];
         } else {
             unsigned got;
             int polls = 0;
@@ -184,19 +213,21 @@ __device__ __noinline__ void exchange(double *partials, unsigned int *arrived, S
                 asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(got) : "l"(arrived) : "memory");
             } while (got < target && ++polls < kMaxPolls);
             if (got < target) s.timed_out = 1;
-            // the blocks' partial sums, five per lane in flight together
-            const double *p = partials + (size_t(par) * kMaxSums + k) * gridDim.x;
-            for (unsigned b = lane; b - lane < gridDim.x; b += 160) {
-                double u[5];
+            __syncwarp();
+            // the blocks' partial sums, ten per lane in flight together
+            const double *p = partials + (size_t(par) * kSums + (k < kSums ? k : 0)) * G;
+            for (int b0 = 0; b0 < G; b0 += 160) {
+                double u[10];
 #pragma unroll
-                for (int q = 0; q < 5; ++q) u[q] = b + 32 * q < gridDim.x ? __ldcg(p + b + 32 * q) : 0.0;
+                for (int q = 0; q < 10; ++q) u[q] = b0 + 16 * q + hl < G ? __ldcg(p + b0 + 16 * q + hl) : 0.0;
 #pragma unroll
-                for (int q = 0; q < 5; ++q)
-                    if (b - lane + 32 * q < gridDim.x) w += u[q];
+                for (int q = 0; q < 10; ++q)
+                    if (b0 + 16 * q < G) w += u[q];
             }
-            w = warp_sum<16>(w);
         }
-        if (lane == 0) s.tot[k] = w;
+#pragma unroll
+        for (int off = 8; off > 0; off >>= 1) w += __shfl_xor_sync(kFull, w, off);
+        if (hl == 0 && k < kSums) s.tot[k] = w;
         __syncwarp();
     }
 }
@@ -211,30 +242,33 @@ constexpr int kGathers = 6;  // gathers in flight per thread: the off-diagonal e
 
 template <bool CLUSTER, int TMAX>
 __global__ void __launch_bounds__(TMAX, 1) k_pcg_resident(const __grid_constant__ ResidentArgs a) {
-    extern __shared__ double2 dyn[];
+    extern __shared__ __align__(32) unsigned char dyn[];
     __shared__ Shared s;
     const int T = blockDim.x, t = threadIdx.x, wid = t >> 5;
     const int i = blockIdx.x * T + t;
     const bool act = i < a.n;
-    // dynamic shared memory: cluster form's {z, p} pair [2][T], the exchange's
-    // values [kMaxSums][T], the staged matrix entries' values and places [staged][T]
-    double2 *zp_sh = dyn;
-    double *buf = reinterpret_cast<double *>(dyn + (CLUSTER ? 2 * T : 0));
-    double *mval = buf + kMaxSums * T;
+    // dynamic shared memory: cluster form's records [2][T], the exchange's
+    // values [kSums][T], the staged matrix entries' values and places [staged][T]
+    ZpuRec *zp_sh = reinterpret_cast<ZpuRec *>(dyn);
+    double *buf = reinterpret_cast<double *>(zp_sh + (CLUSTER ? 2 * T : 0));
+    double *mval = buf + kSums * T;
     int32_t *mcol = reinterpret_cast<int32_t *>(mval + size_t(a.staged) * T);
     unsigned par = 0, target = 0;
-    auto sums = [&](int n) {
-        target += gridDim.x * unsigned(n);
-        exchange<CLUSTER>(a.partials, a.arrived, s, buf, par, target, n);
+    auto sums = [&] {
+        target += gridDim.x;
+        exchange<CLUSTER>(a.partials, a.arrived, s, buf, par, target);
         par ^= 1u;
     };
-    if (t == 0) {
-        s.timed_out = 0;
-        s.inv_rz = 0.0;
-    }
+    auto publish = [&](int half, double z, double p, double u) {
+        if constexpr (CLUSTER)
+            zp_sh[half * T + t] = ZpuRec{z, p, u, 0.0};
+        else
+            a.zpu[half][i] = ZpuRec{z, p, u, 0.0};
+    };
+    if (t == 0) s.timed_out = 0;
 
     const RowRef row = act ? row_ref(a, i) : RowRef{0, 1, 0};
-    // place of column c's {z, p}: its index, or its shared address in the cluster
+    // place of column c's record: its index, or its shared address in the cluster
     auto place = [&](int32_t c) -> int32_t {
         if constexpr (CLUSTER) {
             const uint32_t rank = uint32_t(c) / uint32_t(T);
@@ -287,10 +321,7 @@ __global__ void __launch_bounds__(TMAX, 1) k_pcg_resident(const __grid_constant_
         rz0 = r * z;
         bb0 = b * b;
         rr0 = r * r;
-        if constexpr (CLUSTER)
-            zp_sh[t] = make_double2(z, 0.0);
-        else
-            a.zp[0][i] = make_double2(z, 0.0);
+        publish(0, z, 0.0, 0.0);
     }
     // the warp's rows filled up to one even count with zero couplings of a row
     // to itself (or, past the last row, of nothing to the last), so that the
@@ -308,8 +339,9 @@ __global__ void __launch_bounds__(TMAX, 1) k_pcg_resident(const __grid_constant_
     buf[T + t] = bb0;
     buf[2 * T + t] = rr0;
     buf[3 * T + t] = bad;
+    buf[4 * T + t] = 0.0;
     if constexpr (CLUSTER) cluster_barrier();  // every block runs before its shared memory is written
-    sums(4);
+    sums();
     __syncthreads();
     double rz = s.tot[0], rr = s.tot[2], pq = 0.0, alpha = 0.0, beta = 0.0;
     const double bb = s.tot[1], tol2 = a.rtol2 * bb;
@@ -320,94 +352,90 @@ __global__ void __launch_bounds__(TMAX, 1) k_pcg_resident(const __grid_constant_
 
     int cur = 0;
     while (stop == 0) {
-        // ---- phase A
+        // ---- p = z + beta p and q = A p: of another row c, z is the z it
+        // published less alpha u, and p that plus beta times the p it published
         p = fma(beta, p, z);
         double q;
         {
             double a0 = diag * p, a1 = 0.0;
-            const uint32_t half = CLUSTER ? uint32_t(cur) * uint32_t(T) * 16u : 0u;
-            const double2 *src = CLUSTER ? nullptr : a.zp[cur];
-            auto get = [&](int32_t at) -> Zp {
+            const uint32_t half = CLUSTER ? uint32_t(cur) * uint32_t(T) * uint32_t(sizeof(ZpuRec)) : 0u;
+            const ZpuRec *src = CLUSTER ? nullptr : a.zpu[cur];
+            auto get = [&](int32_t at) -> Zpu {
                 if constexpr (CLUSTER)
-                    return load_zp_cluster(uint32_t(at) + half);
+                    return load_zpu_cluster(uint32_t(at) + half);
                 else
-                    return load_zp(src + at);
+                    return load_zpu(src + at);
             };
+            auto dir = [&](const Zpu &g) { return fma(beta, g.p, fma(-alpha, g.u, g.z)); };
             int k = 0;
             for (; k + kGathers <= staged; k += kGathers) {
-                Zp g[kGathers];
+                Zpu g[kGathers];
 #pragma unroll
                 for (int u = 0; u < kGathers; ++u) g[u] = get(mcol[(k + u) * T + t]);
 #pragma unroll
                 for (int u = 0; u < kGathers; u += 2) {
-                    a0 = fma(mval[(k + u) * T + t], fma(beta, g[u].p, g[u].z), a0);
-                    a1 = fma(mval[(k + u + 1) * T + t], fma(beta, g[u + 1].p, g[u + 1].z), a1);
+                    a0 = fma(mval[(k + u) * T + t], dir(g[u]), a0);
+                    a1 = fma(mval[(k + u + 1) * T + t], dir(g[u + 1]), a1);
                 }
             }
             for (; k + 2 <= staged; k += 2) {
-                const Zp g0 = get(mcol[k * T + t]), g1 = get(mcol[(k + 1) * T + t]);
-                a0 = fma(mval[k * T + t], fma(beta, g0.p, g0.z), a0);
-                a1 = fma(mval[(k + 1) * T + t], fma(beta, g1.p, g1.z), a1);
+                const Zpu g0 = get(mcol[k * T + t]), g1 = get(mcol[(k + 1) * T + t]);
+                a0 = fma(mval[k * T + t], dir(g0), a0);
+                a1 = fma(mval[(k + 1) * T + t], dir(g1), a1);
             }
-            if (k < staged) {  // an odd capacity
-                const Zp g = get(mcol[k * T + t]);
-                a0 = fma(mval[k * T + t], fma(beta, g.p, g.z), a0);
-            }
+            if (k < staged) a0 = fma(mval[k * T + t], dir(get(mcol[k * T + t])), a0);  // an odd capacity
             for (k = next; k < row.count; ++k) {
                 const int32_t c = __ldg(a.col + row.at(k));
                 const double m = __ldg(a.val + row.at(k));
                 if (c == i || m == 0.0) continue;
-                const Zp g = get(place(c));
-                a0 = fma(m, fma(beta, g.p, g.z), a0);
+                a0 = fma(m, dir(get(place(c))), a0);
             }
             q = a0 + a1;
         }
+        const double u = q * dinv;
+        cur ^= 1;
+        if (act) publish(cur, z, p, u);
         buf[t] = act ? p * q : 0.0;
-        sums(1);
+        buf[T + t] = act ? z * q : 0.0;
+        buf[2 * T + t] = act ? u * q : 0.0;
+        buf[3 * T + t] = act ? r * z : 0.0;
+        buf[4 * T + t] = act ? r * r : 0.0;
+        sums();
+        __syncthreads();
         if (wid == 0) {
             pq = s.tot[0];
-            // not positive: A not SPD on this subspace, or NaN
-            const int why = s.timed_out ? kPcgTimedOut : positive(pq) ? 0 : kPcgBreakdown;
-            alpha = why ? 0.0 : quotient(rz, pq, reciprocal(pq));
+            rz = s.tot[3];
+            // the stop test of the last update, then p.q: not positive if A is not SPD on
+            // this subspace, or NaN
+            const int why = s.timed_out               ? kPcgTimedOut
+                            : s.tot[4] <= tol2        ? 1
+                            : iters > 0 && iters >= a.max_iter ? 2
+                            : positive(pq)            ? 0
+                                                      : kPcgBreakdown;
+            const double y = reciprocal((t & 1) ? rz : pq);  // both at once
+            const double y0 = __shfl_sync(kFull, y, 0), y1 = __shfl_sync(kFull, y, 1);
+            alpha = why ? 0.0 : quotient(rz, pq, y0);
+            const double next_rz = fma(alpha * alpha, s.tot[2], fma(-2.0 * alpha, s.tot[1], rz));
+            beta = positive(next_rz) ? quotient(next_rz, rz, y1) : 0.0;
             if (t == 0) {
                 s.stop = why;
                 s.alpha = alpha;
+                s.beta = beta;
             }
-        } else if (wid == 1) {
-            const double y = reciprocal(rz);  // for beta, off its critical path
-            if (t == 32) s.inv_rz = y;
         }
         __syncthreads();
         stop = s.stop;
-        alpha = s.alpha;
+        rr = s.tot[4];
+        pq = s.tot[0];
+        rz = s.tot[3];
         if (stop) break;
-        // ---- phase B
+        alpha = s.alpha;
+        beta = s.beta;
+        // ---- x, r, z of the row
         r = fma(-alpha, q, r);
         z = r * dinv;
-        cur ^= 1;
-        if (act) {
-            if constexpr (CLUSTER)
-                zp_sh[cur * T + t] = make_double2(z, p);
-            else
-                a.zp[cur][i] = make_double2(z, p);
-        }
-        buf[t] = act ? r * z : 0.0;
-        buf[T + t] = act ? r * r : 0.0;
         x = fma(alpha, p, x);
         ++iters;
-        sums(2);
-        if (wid == 0) {
-            beta = quotient(s.tot[0], rz, s.inv_rz);
-            if (t == 0) s.beta = beta;
-        } else if (wid == 1) {
-            const int why = s.timed_out ? kPcgTimedOut : s.tot[1] <= tol2 ? 1 : iters >= a.max_iter ? 2 : 0;
-            if (t == 32) s.stop = why;
-        }
-        __syncthreads();
-        stop = s.stop;
-        beta = s.beta;
-        rz = s.tot[0];
-        rr = s.tot[1];
     }
     // a refused system keeps the caller's x
     if (act && (iters > 0 || zero_x)) a.x[i] = zero_x ? 0.0 : x;
@@ -436,10 +464,10 @@ Kernel kernel_of(const ResidentPlan &p) {
 }
 
 // Rows up to which one cluster of 16 blocks is used.
-constexpr int64_t kClusterRows = 6144;
+constexpr int64_t kClusterRows = 4096;
 
 size_t smem_of(int threads, int staged, bool cluster) {
-    return size_t(threads) * ((cluster ? 32 : 0) + 8 * kMaxSums + 12 * size_t(staged));
+    return size_t(threads) * ((cluster ? 2 * sizeof(ZpuRec) : 0) + 8 * kSums + 12 * size_t(staged));
 }
 
 cudaLaunchConfig_t config_of(const ResidentPlan &p, cudaLaunchAttribute *attr, cudaStream_t s) {

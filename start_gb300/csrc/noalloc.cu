@@ -9,10 +9,11 @@
 // Such a caller already holds the matrix, the right-hand side and the solution
 // vector in memory it allocated itself; this entry point needs nothing else.
 //
-// The scratch array (r, z, p, q, the Jacobi inverse diagonal, per-block
-// partial sums and the CG scalars) is sized for kNoAllocMaxRows rows:
-// 5 * 131072 doubles + 3 * 512 block partials + scalars, about 5.3 MB, which
-// every GPU that loads the library keeps until the process exits.
+// The scratch array (two records per row of the one-launch solver, or r, z, p, q
+// and the Jacobi inverse diagonal of the separate kernels, with the partial sums
+// and the CG scalars) is sized for kNoAllocMaxRows rows: 8 * 131072 doubles and
+// the sums, 8.4 MB, which every GPU that loads the library keeps until the
+// process exits.
 #include <cmath>
 #include <cstring>
 #include <mutex>
@@ -30,7 +31,10 @@ constexpr int kNaThreads = 256;
 constexpr int kNaMaxBlocks = 512;
 constexpr int kNaChunk = 8;  // iterations launched between convergence checks
 constexpr int64_t kScalarWords = 16;
-constexpr int64_t kScratchWords = 5 * kNoAllocMaxRows + 3 * kNaMaxBlocks + kScalarWords;
+constexpr int64_t kSumsAt = 8 * kNoAllocMaxRows;  // partial sums, the barrier's counter, the scalars
+constexpr int64_t kScalarsAt = kSumsAt + int64_t(kResidentPartials) + 16;
+constexpr int64_t kScratchWords = kScalarsAt + kScalarWords;
+static_assert(kResidentPartials >= 3 * kNaMaxBlocks, "room for either solver's sums");
 static_assert(sizeof(PcgScalars) <= kScalarWords * sizeof(double), "scalar slot too small");
 
 // The one scratch array shared by every call on a device.
@@ -288,7 +292,7 @@ extern "C" int spg_pcg_solve_noalloc(int64_t n, const int32_t *row_ptr, const in
     PcgScalars hs;
     cudaError_t e;
     if (plan.blocks > 0) {
-        // the whole solve in one launch; the working vectors' scratch holds its pairs and partial sums
+        // the whole solve in one launch; the working vectors' scratch holds its records and partial sums
         ResidentArgs r;
         r.n = int(n);
         r.row_ptr = row_ptr;
@@ -296,11 +300,11 @@ extern "C" int spg_pcg_solve_noalloc(int64_t n, const int32_t *row_ptr, const in
         r.val = val;
         r.b = b;
         r.x = x;
-        r.zp[0] = reinterpret_cast<double2 *>(base);
-        r.zp[1] = reinterpret_cast<double2 *>(base + 2 * kNoAllocMaxRows);
-        r.partials = base + 4 * kNoAllocMaxRows;
-        r.arrived = reinterpret_cast<unsigned int *>(base + 4 * kNoAllocMaxRows + kResidentPartials);
-        r.sc = reinterpret_cast<PcgScalars *>(base + 5 * kNoAllocMaxRows + 3 * kNaMaxBlocks);
+        r.zpu[0] = reinterpret_cast<ZpuRec *>(base);
+        r.zpu[1] = reinterpret_cast<ZpuRec *>(base + 4 * kNoAllocMaxRows);
+        r.partials = base + kSumsAt;
+        r.arrived = reinterpret_cast<unsigned int *>(base + kSumsAt + kResidentPartials);
+        r.sc = reinterpret_cast<PcgScalars *>(base + kScalarsAt);
         r.rtol2 = rtol * rtol;
         r.max_iter = max_iter;
         r.breakdown = kPcgBreakdown;
@@ -324,8 +328,8 @@ extern "C" int spg_pcg_solve_noalloc(int64_t n, const int32_t *row_ptr, const in
     a.p = base + 2 * kNoAllocMaxRows;
     a.q = base + 3 * kNoAllocMaxRows;
     a.dinv = base + 4 * kNoAllocMaxRows;
-    a.partials = base + 5 * kNoAllocMaxRows;
-    a.sc = reinterpret_cast<PcgScalars *>(base + 5 * kNoAllocMaxRows + 3 * kNaMaxBlocks);
+    a.partials = base + kSumsAt;
+    a.sc = reinterpret_cast<PcgScalars *>(base + kScalarsAt);
     // The scalars keep the previous call's values: start from a clean block
     // (ticket 0, not converged) every call.
     PcgScalars init;

@@ -29,9 +29,12 @@ struct ResidentPlan {
 
 // The system and its working memory. SELL-32 (slice_ptr) or CSR (row_ptr);
 // inv_diag nullptr: taken from the matrix, and a row without a finite nonzero
-// diagonal entry is refused. zp: two arrays of n {z, p} pairs, 16-byte
-// aligned (grid form only); partials: resident_partials() doubles; arrived:
-// zeroed by the launch.
+// diagonal entry is refused. zpu: two arrays of n records (grid form only);
+// partials: kResidentPartials doubles; arrived: zeroed by the launch.
+struct alignas(32) ZpuRec {
+    double z, p, u, unused;  // D^-1 r, the search direction, D^-1 A p
+};
+constexpr int kResidentSums = 5;
 struct ResidentArgs {
     int n = 0;
     const int64_t *slice_ptr = nullptr;
@@ -39,7 +42,7 @@ struct ResidentArgs {
     const int32_t *col = nullptr;
     const double *val = nullptr, *inv_diag = nullptr, *b = nullptr;
     double *x = nullptr;
-    double2 *zp[2] = {nullptr, nullptr};
+    ZpuRec *zpu[2] = {nullptr, nullptr};
     double *partials = nullptr;
     unsigned int *arrived = nullptr;
     PcgScalars *sc = nullptr;
@@ -48,7 +51,7 @@ struct ResidentArgs {
     bool zero_on_zero_b = false;
 };
 
-constexpr size_t kResidentPartials = 2 * 4 * 512;  // two parities of four sums, at most 512 blocks
+constexpr size_t kResidentPartials = 2 * kResidentSums * 512;  // two parities, at most 512 blocks
 
 ResidentPlan resident_plan(int64_t n);
 cudaError_t launch_pcg_resident(const ResidentPlan &plan, ResidentArgs a, cudaStream_t s);
