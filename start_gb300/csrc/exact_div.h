@@ -44,14 +44,17 @@ SPG_XHD inline double from_bits(long long b) {
 // below is half the ulp above); then the neighbour in the remainder's
 // direction is taken, and an exact half-way remainder keeps the even one.
 // Comparisons and the ulp step are integer operations on the bit patterns.
-// Zero and quotients or thresholds near the subnormal or overflow range take
-// the division itself.
+// Quotients or thresholds near the subnormal or overflow range take the
+// division itself.
 SPG_XHD inline double div_by_known(double x, double m, double r) {
     const long long qb0 = as_bits(x * r);
     const int eq = int((qb0 >> 52) & 0x7ff);
     const long long mb = as_bits(m);
     const int em = int((mb >> 52) & 0x7ff);
-    // (x == 0 is a zero exponent of x r; the tests below are integer operations)
+    // zero over a finite m is the zero of the product's sign (a potential that is
+    // flat over most of the mesh must not cost its warps the division)
+    if ((as_bits(x) << 1) == 0 && em != 0 && em != 0x7ff) return from_bits(qb0);
+    // (the tests below are integer operations)
     if (eq < 64 || eq > 2000 || em + eq < 1140 || em + eq > 3000) return x / m;
     const double q0 = from_bits(qb0);
     const double q1 = std::fma(std::fma(-q0, m, x), r, q0);
