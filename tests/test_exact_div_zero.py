@@ -8,6 +8,7 @@ ROOT = Path(__file__).resolve().parent.parent
 
 SRC = r"""
 #include <cstdio>
+#include <initializer_list>
 #include <limits>
 #include "exact_div.h"
 int main() {
