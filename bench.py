@@ -111,25 +111,24 @@ class ClockSampler:
                 "reasons": sorted(reasons)}
 
 
-# dram__bytes_read.sum + dram__bytes_write.sum of the step kernel and its walk kernel per alive
-# particle, workload 1 geometry, one ncu --set full capture at 4e6 particles (FP64: 229.1 + 151.4
-# MB for k_step64, 71.27 + 1.472 MB for k_walk_queue64; mixed: 128.2 + 40.67 MB for k_step32,
-# 53.52 + 1.419 MB for k_walk_queue32)
+# dram__bytes_read.sum + dram__bytes_write.sum of one launch of the step kernel (a segment of up to
+# 32 steps, here seven) per alive particle, workload 1 geometry, one ncu capture at 4e6 particles
+# (FP64: 224.7 + 159.4 MB; mixed: 128.7 + 81.1 MB)
 STEP_TRAFFIC_B = {
-    "64": (453.2e6 / 4e6, "ncu capture of k_step64 + k_walk_queue64 at 4e6 particles, scaled by particles"),
-    "32": (223.8e6 / 4e6, "ncu capture of k_step32 + k_walk_queue32 at 4e6 particles, scaled by particles"),
+    "64": (384.1e6 / 4e6, "ncu capture of k_seg64 (seven steps) at 4e6 particles, scaled by particles"),
+    "32": (209.8e6 / 4e6, "ncu capture of k_seg32 (seven steps) at 4e6 particles, scaled by particles"),
 }
 # The resource that binds the step kernels is not HBM: the FP64 form's step is
 # FP64-issue-bound (GB300 issues about 2 FP64 thread-ops per clock per SM),
-# the FP32 form's is memory-latency-bound. Pipe utilisation from the same
-# captures (sm__pipe_fp64_cycles_active, % of peak sustained active).
+# the mixed form's by instruction issue. From the same captures
+# (sm__pipe_fp64_cycles_active, smsp__issue_active, % of peak sustained active).
 STEP_BINDING = {
-    "64": {"resource": "fp64 pipe", "k_step64": 0.783, "k_walk_queue64": 0.589,
-           "source": "ncu --set full, k_step64 + k_walk_queue64 at 4e6 particles"},
-    "32": {"resource": "memory latency (long-scoreboard stalls; fp64 pipe 0 in k_step32)",
-           "k_step32_issue_active": 0.434, "k_step32_warps_active": 0.482,
-           "source": "ncu --set full, k_step32 + k_walk_queue32 at 4e6 particles"},
+    "64": {"resource": "fp64 pipe", "k_seg64": 0.736, "source": "ncu, k_seg64 at 4e6 particles"},
+    "32": {"resource": "instruction issue", "k_seg32_issue_active": 0.663, "k_seg32_active_lanes": 24.7,
+           "source": "ncu, k_seg32 at 4e6 particles"},
 }
+STEP_BYTES_NOTE = ("algorithmic bytes of one step per particle-step (the state read and written, the occupied tets' "
+                   "records); a segment moves the state once, so this effective rate exceeds its DRAM traffic")
 
 
 def measured_peak():
@@ -539,7 +538,7 @@ def run_gpu(args):
     peak, peak_src = measured_peak()
     sfx = "32" if args.precision == "mixed" else "64"
     phases = {
-        "step": (f"k_step{sfx} + k_walk_queue{sfx} (push, move, collide, walk, settle)", prof["step_ms"],
+        "step": (f"k_seg{sfx} (push, move, collide, walk, settle)", prof["step_ms"],
                  prof["step_bytes"], prof["step_launches"]),
         "pcg": ("PCG iterations (SELL-32 SpMV + dots, updates"
                 + (", AMG V-cycle)" if args.precond != "jacobi" else ")"), prof["pcg_ms"], prof["pcg_bytes"],
@@ -553,8 +552,8 @@ def run_gpu(args):
     traffic, traffic_src = args.traffic, "--traffic" if args.traffic else None
     binding = None
     if traffic is None and dom == "step" and args.workload == 1:
-        # DRAM bytes (read + write) of the step kernel pair per alive particle from one ncu capture
-        # of the same geometry at 4e6 particles, scaled by the particles one launch processes
+        # DRAM bytes (read + write) of the step kernel per alive particle and launch from one ncu
+        # capture of the same geometry at 4e6 particles, scaled by the particles one launch processes
         per_particle, src = STEP_TRAFFIC_B[sfx]
         traffic, traffic_src = per_particle * ps / max(1, K), src
         binding = STEP_BINDING[sfx]
@@ -563,6 +562,8 @@ def run_gpu(args):
             "peak_source": peak_src, "bytes_per_launch": dbytes / max(1, dl), "ms_per_launch": dms / max(1, dl)}
     if binding:
         roof["binding"] = binding
+    if dom == "step":
+        roof["note"] = STEP_BYTES_NOTE
     for k, (nm, ms_k, b_k, l_k) in phases.items():
         roof[f"{k}_GBps"] = b_k / (ms_k / 1e3) / 1e9 if ms_k > 0 else None
     breakdown = {k: prof[k] for k in ("step_ms", "deposit_ms", "pcg_ms", "efield_ms", "sort_ms")}
@@ -629,10 +630,7 @@ def run_gpu(args):
                  "breakdown_ms": {k: mp[k] for k in ("step_ms", "deposit_ms", "pcg_ms", "efield_ms", "sort_ms")},
                  "pcg_iters": mp["pcg_iters"],
                  "step_GBps": mp["step_bytes"] / (mp["step_ms"] / 1e3) / 1e9 if mp["step_ms"] > 0 else None,
-                 "step_GBps_note": ("algorithmic bytes of one step per particle-step (the state read and "
-                                    "written, the occupied tets' records); the segmented step moves the "
-                                    "state once per segment, so this effective rate exceeds its DRAM "
-                                    "traffic (profiles/k_seg32_w1_4e6ptcl.md)"),
+                 "step_GBps_note": STEP_BYTES_NOTE,
                  "pcg_GBps": mp["pcg_bytes"] / (mp["pcg_ms"] / 1e3) / 1e9 if mp["pcg_ms"] > 0 else None,
                  "gpu_launches": mp["kernel_launches"],
                  "one_launch_per_step": single,

@@ -290,9 +290,9 @@ int spg_resort(spg_handle *h);
 /* No counterpart in the reference (an execution choice, not a result).
  * spg_run and spg_process run the steps between two events of the loop (a
  * solve, a re-sort, the end of the call) as segments of up to max_steps steps:
- * one pass keeps each particle in registers until a move needs the exact tet
- * walk, the walk runs batched, and the walked particles resume from the next
- * step (the FP64 form in one launch, the mixed form in a chain of them).
+ * one launch keeps each particle in registers or shared memory, runs the moves
+ * that need the exact tet walk batched per warp, and steps the walked
+ * particles on.
  * Results are bit-identical to one launch per step (max_steps = 1). Default
  * 32; SPG_E_INVALID outside 1..64. Runs with trajectory sampling always step
  * one launch per step. */
@@ -363,8 +363,8 @@ int spg_profile_reset(spg_handle *h);
  * is all owned by its own pool (a PyTorch caching allocator, a fixed arena),
  * and a loop that must not take the device-wide synchronisation that
  * cudaMalloc/cudaFree can imply. The call itself still synchronises the
- * stream it is given: every 8 iterations it reads the CG scalars back to the
- * host to decide whether to go on.
+ * stream it is given: once, to read the outcome of the solve, which is one
+ * launch (every 8 iterations on a device too small for that).
  *
  * row_ptr [n+1], col [nnz], val [nnz], b [n] and x [n] are DEVICE pointers the
  * caller allocated; x holds the initial guess and receives the solution.
@@ -383,7 +383,7 @@ int spg_profile_reset(spg_handle *h);
  *
  * Limit: n <= 131072 rows. Larger n returns SPG_E_INVALID without touching
  * the GPU. The working vectors live in one static device array of about
- * 5.3 MB that every GPU loading the library keeps until the process exits.
+ * 8.4 MB that every GPU loading the library keeps until the process exits.
  * All calls on a device share it. Calls that overlap on the GPU (several
  * streams, several host threads) race on it and must be serialised by the
  * caller. Each call resets the parts that must start at zero.

@@ -2654,7 +2654,7 @@ int spg_restore(spg_handle *h, const void *buf, size_t bytes) {
     h->have_particles = true;
     h->occ_fresh = false;
     h->resorted_at = -1;
-    h->sorted = false;
+    h->sorted = hd.occupied > 0;  // saved after a re-sort: near its order
     if (h->cg_solves == 0) {
         zero_field(h);
     } else {
