@@ -331,7 +331,10 @@ int spg_set_dirichlet(spg_handle *h, const double *g);
  * (no deposit or solve), keeping the particle state every checkpoint_every
  * steps and where each particle lands, and returns
  *   J = (1/N) sum over the N particles that landed of exp(-|r - target|^2 / (2 sigma^2)).
- * spg_grad_backward recomputes each checkpoint window, runs the adjoint of
+ * (FP64 form: where 32 bytes per particle and step fit into 32 GB and a quarter
+ * of the free device memory, it records every step instead and takes no
+ * checkpoints; the record stays with the handle until it is destroyed).
+ * spg_grad_backward reads the record or recomputes each checkpoint window, runs the adjoint of
  * push, move and frozen collisions, one adjoint CG on the stiffness matrix,
  * and returns dJ/dg at the Dirichlet nodes (0 elsewhere) and, if non-NULL,
  * dJ/d(initial position) and dJ/d(initial velocity) per particle [3n, id order].

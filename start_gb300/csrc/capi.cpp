@@ -2806,7 +2806,7 @@ int spg_grad_field_gradient(spg_handle *h, int32_t on) {
 namespace {
 // Whether the forward pass records every step (32 bytes per particle and step,
 // and room for the results behind them) for the backward pass, in the record
-// kept or a new one of at most a quarter of the free memory. Else, and in the
+// kept or a new one of at most 32 GB and a quarter of the free memory. Else, and in the
 // mixed form, it keeps checkpoints and the backward pass repeats the steps of
 // each window: 1e6 particles, 300 steps take 9.7 GB and 13.4 -> 9.05 ms for
 // forward and backward together; the record of a step adds 6 % to it.
@@ -2819,7 +2819,8 @@ bool whole_history(spg_handle *h, int64_t steps, int64_t n) {
         cudaGetLastError();
         return false;
     }
-    if (size_t(need) > (free + sizeof(HistRec) * size_t(h->hist_cap)) / 4 / sizeof(HistRec)) return false;
+    const size_t room = std::min<size_t>((free + sizeof(HistRec) * size_t(h->hist_cap)) / 4, size_t(32) << 30);
+    if (size_t(need) > room / sizeof(HistRec)) return false;
     cudaFree(h->hist64);
     h->hist64 = nullptr;
     h->hist_cap = 0;

@@ -3,7 +3,7 @@ that are repeated from checkpoints when the record does not fit.
 
 Without collisions the particles are independent and alike, so a set of 400
 (recorded) and the same 400 repeated 2,500 times (1e6 particles, 2,400 steps: 77
-GB, more than a quarter of the device) have the same J and dJ/dg, and 2,500 times
+GB, more than the record may take) have the same J and dJ/dg, and 2,500 times
 the derivative of each particle. The sums over particles are of 1e6 FP64 terms in
 another order: 1e-10 of the largest component covers them; a second backward pass
 of the record returns what the first did, up to the order of the same sums.
