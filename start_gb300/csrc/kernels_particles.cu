@@ -381,10 +381,13 @@ __device__ __forceinline__ void field_of_tet64(const FieldArgs &f, int64_t t) {
 constexpr int kPool = 96, kSide = 24, kPoolWords = 12;
 constexpr int kRefill = 2;   // idle lanes that make a warp look for work (8: 343 us per step of 1e7, 4: 331, 2: 328)
 constexpr int kDrain = 16;   // idle lanes that make it run a part-filled batch when nothing else is left
-struct WarpPool {
-    double w[kPoolWords][kPool + kSide];
+template <int ITEMS>
+struct PoolOf {
+    double w[kPoolWords][ITEMS];
     unsigned int cross, settled, lost, capped, coll;
 };
+using WarpPool = PoolOf<kPool + kSide>;
+using StepPool = PoolOf<64>;  // single steps: waiting items only
 // Waiting items: the walk; the collision test; a position that is no number.
 constexpr int kNeedWalk = 1, kNeedTest = 2, kNeedLost = 4;
 // Ready items: the field is not zero; the tet lies inside the modelling box; a
@@ -419,7 +422,8 @@ __device__ __forceinline__ Push64 load_push(const TetRec *__restrict__ rec, int 
     return Push64{a.x, a.y, b.x, ((w & 0xffffffffull) == 0ull ? kPush : 0) | ((w >> 32) != 0ull ? kInterior : 0)};
 }
 
-__device__ __forceinline__ void put_ready(WarpPool &P, int k, double x, double y, double z, const Push64 &h, double vx,
+template <class Pool>
+__device__ __forceinline__ void put_ready(Pool &P, int k, double x, double y, double z, const Push64 &h, double vx,
                                           double vy, double vz, int tet, uint32_t idf, int i, int word, double cand) {
     P.w[0][k] = x;
     P.w[1][k] = y;
@@ -461,7 +465,8 @@ __device__ __noinline__ int prepare64(const Seg64 &a, const StepConst &c, WarpPo
 // The waiting items [first, first + take) of the warp's pool, one per lane:
 // collision, walk, landing. An item that goes on becomes a ready one, the
 // others are written to the particle arrays. Returns the new count of ready items.
-__device__ __noinline__ int run_pool64(const Seg64 &a, const StepConst &c, const FieldArgs &f, WarpPool &P, int first,
+template <class Pool>
+__device__ __noinline__ int run_pool64(const Seg64 &a, const StepConst &c, const FieldArgs &f, Pool &P, int first,
                                        int take, int nr) {
     const int lane = threadIdx.x & 31;
     const bool mine = lane < take;
@@ -760,6 +765,127 @@ __global__ void __launch_bounds__(128, 4) k_seg64(const __grid_constant__ Seg64 
         }
     }
     // one atomic per counter and warp
+    const unsigned long long n0 = warp_sum(processed);
+    if (lane == 0) {
+        const unsigned long long n1 = P.coll, n3 = P.cross, n4 = P.settled, n5 = P.capped, n6 = P.lost;
+        if (n0) atomicAdd(&a.ctr->processed, n0);
+        if (n1) atomicAdd(&a.ctr->collisions, n1);
+        if (n3) atomicAdd(&a.ctr->crossings, n3);
+        if (n4) atomicAdd(&a.ctr->settled, n4);
+        if (n5) atomicAdd(&a.ctr->capped, n5);
+        if (n6) atomicAdd(&a.ctr->lost, n6);
+    }
+}
+
+// A single step (a call of one step, or steps between which the trajectories are
+// sampled). Nothing is gained there by a lane that takes another particle at
+// once: a warp steps 32 particles straight from the arrays, writes those that stay
+// in their tet, and pools the others; 32 of these are walked and decided in a
+// full warp and written. No state lives across the pool, so the kernel holds 80
+// registers and 24 warps per SM instead of 128 and 16, which hides the loads that
+// a step of its own needs. The operations are those of k_seg64's step. us per
+// step, a step and a walk kernel with a queue in memory / k_seg64 with L = 1 /
+// here: 1e7 ions on 6.0e6 tets 417, 523, 390; 1e6 of a Thompson source 58, 62, 48,
+// all over the mesh 71, 78, 60; 1e5 27, 20, 17. (Blocks per SM 5 / 6 / 8: 408, 390,
+// 495 at 1e7.)
+__global__ void __launch_bounds__(128, 6) k_step64(const __grid_constant__ Seg64 a, const __grid_constant__ StepConst c,
+                                                   const __grid_constant__ FieldArgs f) {
+    extern __shared__ __align__(16) unsigned char pool_bytes[];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const unsigned below = (1u << lane) - 1u;
+    StepPool &P = reinterpret_cast<StepPool *>(pool_bytes)[wid];
+    if (lane == 0) P.cross = P.settled = P.lost = P.capped = P.coll = 0u;
+    __syncwarp();
+    unsigned processed = 0;
+    int np = 0;
+    const int64_t stride = int64_t(gridDim.x) * blockDim.x;
+    for (int64_t base = int64_t(blockIdx.x) * blockDim.x + 32 * wid; base < a.n; base += stride) {
+        const int64_t i = base + lane;
+        uint32_t idf = kDead;
+        if (i < a.n) idf = a.p.idf[i];
+        int need = 0, tet = 0;
+        double x = 0.0, y = 0.0, z = 0.0, vx = 0.0, vy = 0.0, vz = 0.0, nx = 0.0, ny = 0.0, nz = 0.0;
+        uint32_t is_cand = 0u;
+        if (!(idf & kDead)) {
+            ++processed;
+            tet = a.p.tet[i];
+            x = a.p.x[i];
+            y = a.p.y[i];
+            z = a.p.z[i];
+            vx = a.p.vx[i];
+            vy = a.p.vy[i];
+            vz = a.p.vz[i];
+            const ScreenRegs scr = load_screen(a.m.screen + tet);
+            const Push64 h = load_push(a.m.rec, tet);
+            // the tests of k_seg64's step, in its order
+            const long long ax = __double_as_longlong(vx) & 0x7fffffffffffffffLL;
+            const long long ay = __double_as_longlong(vy) & 0x7fffffffffffffffLL;
+            const long long az = __double_as_longlong(vz) & 0x7fffffffffffffffLL;
+            bool stays = false;
+            if (ax < c.two_vmin_bits && ay < c.two_vmin_bits && az < c.two_vmin_bits)
+                stays = sqrt(vx * vx + vy * vy + vz * vz) < c.vmin;
+            const long long kx = order_key(x), ky = order_key(y), kz = order_key(z);
+            stays = stays || !(kx >= c.lo_key[0] && kx <= c.hi_key[0] && ky >= c.lo_key[1] && ky <= c.hi_key[1] &&
+                               kz >= c.lo_key[2] && kz <= c.hi_key[2]);
+            if (!stays) {
+                if (h.flags & kPush) {
+                    vx = (vx + h.hx) + h.hx;
+                    vy = (vy + h.hy) + h.hy;
+                    vz = (vz + h.hz) + h.hz;
+                }
+                nx = x + vx * c.dt;
+                ny = y + vy * c.dt;
+                nz = z + vz * c.dt;
+                if (!(same_value(nx, x) && same_value(ny, y) && same_value(nz, z))) {
+                    if (c.model != SPG_COLL_NONE) {
+                        const uint32_t id = idf & kIdMask;
+                        is_cand = candidate_byte(candidate_block(uint64_t(c.step), id, c.seed_lo, c.seed_hi),
+                                                 uint64_t(c.step)) == 0u;
+                        const float fx = hi_float(vx), fy = hi_float(vy), fz = hi_float(vz);
+                        const float v2 = fmaf(fz, fz, fmaf(fy, fy, fx * fx));
+                        if ((is_cand || !(v2 <= c.v2_cand_f)) &&
+                            !no_collision_sure(c, id, uint64_t(c.step), is_cand, v2))
+                            need = kNeedTest;
+                    }
+                    if (!(finite_bits(nx) && finite_bits(ny) && finite_bits(nz)))
+                        need |= kNeedLost;
+                    else if (!inside_sure(scr, nx, ny, nz))
+                        need |= kNeedWalk;
+                }
+                if (!need) {
+                    a.p.x[i] = nx;
+                    a.p.y[i] = ny;
+                    a.p.z[i] = nz;
+                    a.p.vx[i] = vx;
+                    a.p.vy[i] = vy;
+                    a.p.vz[i] = vz;
+                }
+            }
+        }
+        const unsigned out = __ballot_sync(kFull, need != 0);
+        if (need) {
+            const int k = np + __popc(out & below);
+            P.w[0][k] = x;
+            P.w[1][k] = y;
+            P.w[2][k] = z;
+            P.w[3][k] = nx;
+            P.w[4][k] = ny;
+            P.w[5][k] = nz;
+            P.w[6][k] = vx;
+            P.w[7][k] = vy;
+            P.w[8][k] = vz;
+            P.w[9][k] = __hiloint2double(int(idf), tet);
+            P.w[10][k] = __hiloint2double(need, int(i));
+            P.w[11][k] = __longlong_as_double((long long)is_cand);
+        }
+        np += __popc(out);  // at most 31 + 32
+        __syncwarp();
+        if (np >= 32) {
+            np -= 32;
+            run_pool64(a, c, f, P, np, 32, 0);
+        }
+    }
+    if (np > 0) run_pool64(a, c, f, P, 0, np, 0);
     const unsigned long long n0 = warp_sum(processed);
     if (lane == 0) {
         const unsigned long long n1 = P.coll, n3 = P.cross, n4 = P.settled, n5 = P.capped, n6 = P.lost;
@@ -1246,6 +1372,15 @@ void launch_segment64(const DevParticles &p, int64_t n, const MeshDev &m, const 
     a.hist_n = hist_n;
     a.L = L;
     a.seq = seq;
+    if (L == 1 && !hist) {
+        static int blocks = 0;
+        constexpr size_t bytes = sizeof(StepPool) * 4;
+        if (blocks == 0) blocks = resident_blocks(k_step64, 128, bytes);
+        const int T = n >= int64_t(blocks) * 128 ? 128 : 32;
+        const unsigned grid = unsigned(std::min<int64_t>(grid_for(n, T), int64_t(blocks) * (128 / T)));
+        k_step64<<<grid, T, bytes * T / 128, s>>>(a, c, f);
+        return;
+    }
     // one wave: SMs x resident blocks (same on every device of this build);
     // few particles spread over smaller blocks so that every SM has some
     static int resident[2] = {0, 0};
