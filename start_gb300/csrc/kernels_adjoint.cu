@@ -93,8 +93,8 @@ __device__ __forceinline__ float reach(double v, double h) {
     return fmaf(fabsf(hi_float(v)) + 2.0f * fabsf(hi_float(h)), 1.0f + 2e-6f, 1e-30f);
 }
 
-// Backward recursion over steps [k0, k1) of one checkpoint window, one
-// particle per thread; the adjoint state (abar_x, abar_v) carries between
+// Backward recursion over steps [k0, k1) of one checkpoint window or of the
+// whole record, one particle per thread; the adjoint state (abar_x, abar_v) carries between
 // windows in ax/av. Contributions to dJ/dE of consecutive steps in one tet
 // are summed in registers and added once (k_gE_to_nodes scales them).
 // FP64 issue bounds it (1.7 thread-operations per clock and SM), so a step takes
@@ -104,8 +104,9 @@ __device__ __forceinline__ float reach(double v, double h) {
 // pushed speed; only a step that these leave open forms the pushed velocity and
 // decides as the forward did (collide64.cuh). With a square root, a Philox block
 // and the FP64 probability in every step the ten windows of 1e6 ions, 300 steps
-// took 11.5 ms; now 3.1 (FP64 pipe 80 % active; the rest of its instructions are
-// the tet changes and collisions of single lanes). The next step's record is
+// took 11.5 ms; now 3.1, and 2.8 as one launch over the forward's whole record
+// (FP64 pipe 78 % active; the rest of its instructions are the tet changes and
+// collisions of single lanes). The next step's record is
 // loaded before the current one is used.
 __global__ void __launch_bounds__(128) k_backward(const DevParticles p, int64_t n, const HistRec *__restrict__ h, int k0, int k1,
                                                   const TetRec *__restrict__ rec, const LandRec *__restrict__ land,
