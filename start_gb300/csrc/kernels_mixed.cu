@@ -519,9 +519,10 @@ __global__ void __launch_bounds__(128) k_walk_queue32(const __grid_constant__ Mi
 // full warp and they step on from where they left. So no particle passes
 // through memory between its load and its last store, and the branches of few
 // lanes cost a warp once per group instead of in 60 % of its steps.
-// A field that an earlier launch wrote (epoch <= stamp < seq, as in the FP64
-// form) is read, any other is formed in registers and stored by the lane that
-// swaps the stamp. Every particle goes through the same FP32 operations in the
+// A field that an earlier launch wrote (stored_before, as in the FP64 form) is
+// read, any other is formed in registers and stored by the lane that swaps the
+// stamp; a particle from the queue looks at the stamp also where its tet stays the
+// same, since it may have entered it in this launch. Every particle goes through the same FP32 operations in the
 // same order as in single steps, so the result is bit-identical to stepping one
 // step per launch.
 //
@@ -605,6 +606,7 @@ __global__ void __launch_bounds__(128, 6) k_seg32(const __grid_constant__ Seg32 
                                 ? 1u
                                 : 0u;
                 int status = W_INSIDE;
+                bool entered = false;
                 if (need & kNeedLost) {
                     status = W_EXIT;
                     nx = x;
@@ -619,18 +621,8 @@ __global__ void __launch_bounds__(128, 6) k_seg32(const __grid_constant__ Seg32 
                     nz = w.hz;
                     if (w.status == W_SURFACE) {
                         atomicAdd(a.tri_count + w.tri, 1u);
-                    } else if (w.status == W_INSIDE && w.tet != tet) {
-                        const uint32_t st = __ldcg(f.stamp + w.tet);
-                        if (!(st >= f.epoch && st < a.seq)) {
-                            const Field32 v = field_values32(f, w.tet);
-                            hx = v.H[0];
-                            hy = v.H[1];
-                            hz = v.H[2];
-                            push = !v.zero;
-                            have_field = true;
-                            if (st < f.epoch && atomicCAS(f.stamp + w.tet, st, a.seq) == st) store_field32(f, w.tet, v);
-                        }
                     }
+                    entered = w.status == W_INSIDE && w.tet != tet;
                     tet = w.tet;
                 }
                 x = nx;
@@ -639,6 +631,20 @@ __global__ void __launch_bounds__(128, 6) k_seg32(const __grid_constant__ Seg32 
                 dirty = true;
                 if (status == W_INSIDE) {
                     have = ++j < a.L;
+                    if (have || entered) {
+                        // Also where the tet stays the same: the particle may have entered it
+                        // earlier in this launch, and then its field is being stored by another lane.
+                        const uint32_t st = __ldcg(f.stamp + tet);
+                        if (!stored_before(st, f.epoch, a.seq)) {
+                            const Field32 v = field_values32(f, tet);
+                            hx = v.H[0];
+                            hy = v.H[1];
+                            hz = v.H[2];
+                            push = !v.zero;
+                            have_field = true;
+                            if (st < f.epoch && atomicCAS(f.stamp + tet, st, a.seq) == st) store_field32(f, tet, v);
+                        }
+                    }
                 } else {
                     settled += status == W_SURFACE ? 1u : 0u;
                     lost += status != W_SURFACE ? 1u : 0u;

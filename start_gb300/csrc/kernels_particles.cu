@@ -361,10 +361,12 @@ __device__ __forceinline__ void field_of_tet64(const FieldArgs &f, int64_t t) {
 // so the segment length changes no result.
 //
 // A walk may enter a tet whose field is of an older potential. Stamps count up
-// with every launch that can write fields: epoch <= stamp < seq says the field
-// was computed by an earlier launch and is read; otherwise the lane forms it in
-// registers, and the lane whose compare-and-swap sets the stamp to seq also
-// stores it for later launches. No lane reads a field written in its launch.
+// with every launch that can write fields: a field that an earlier launch computed
+// (stored_before) is read; otherwise the lane forms it in registers, and the lane
+// whose compare-and-swap sets the stamp to seq also stores it for later launches.
+// Nothing orders these stores with a read in the same launch, and no lane makes
+// one: a new particle's tet was entered in an earlier launch, and an item that
+// leaves the pool looks at the stamp, whether its walk entered a tet or not.
 
 // Items of a warp's pool: those waiting for their walk at [0, np), those ready
 // to step at [kPool - nr, kPool), those with a collision to decide at
@@ -505,7 +507,7 @@ __device__ __noinline__ int run_pool64(const Seg64 &a, const StepConst &c, const
                 scatter64(c, u01_from(r.v[0], r.v[1]), u01_from(r.v[2], r.v[3]), vx, vy, vz);
             }
         }
-        bool have_field = false;
+        bool entered = false;
         if (need & kNeedLost) {
             idf |= kLost;
             status = W_EXIT;
@@ -534,17 +536,8 @@ __device__ __noinline__ int run_pool64(const Seg64 &a, const StepConst &c, const
             }
             if (w.status != W_INSIDE) {
                 a.p.idf[i] = idf;
-            } else if (w.tet != tet) {
-                const uint32_t st = __ldcg(f.stamp + w.tet);
-                if (!(st >= f.epoch && st < a.seq)) {
-                    const Field64 v = field_values64(f, w.tet);
-                    h.hx = v.H[0];
-                    h.hy = v.H[1];
-                    h.hz = v.H[2];
-                    h.flags = (v.ezero == 0u ? kPush : 0) | (__ldcg(&a.m.rec[w.tet].interior) != 0u ? kInterior : 0);
-                    have_field = true;
-                    if (st < f.epoch && atomicCAS(f.stamp + w.tet, st, a.seq) == st) store_field64(f, w.tet, v);
-                }
+            } else {
+                entered = w.tet != tet;
             }
             tet = w.tet;
         }
@@ -552,6 +545,21 @@ __device__ __noinline__ int run_pool64(const Seg64 &a, const StepConst &c, const
         y = ny;
         z = nz;
         on = status == W_INSIDE && j + 1 < a.L;
+        if (on || entered) {
+            // Also where the tet stays the same: the particle may have entered it earlier
+            // in this launch, and then its field is being stored by another lane.
+            const uint32_t st = __ldcg(f.stamp + tet);
+            if (!stored_before(st, f.epoch, a.seq)) {
+                const Field64 v = field_values64(f, tet);
+                h.hx = v.H[0];
+                h.hy = v.H[1];
+                h.hz = v.H[2];
+                h.flags = (v.ezero == 0u ? kPush : 0) | (__ldcg(&a.m.rec[tet].interior) != 0u ? kInterior : 0);
+                if (st < f.epoch && atomicCAS(f.stamp + tet, st, a.seq) == st) store_field64(f, tet, v);
+            } else if (on) {
+                h = load_push(a.m.rec, tet);
+            }
+        }
         if (!on) {
             a.p.x[i] = x;
             a.p.y[i] = y;
@@ -560,8 +568,6 @@ __device__ __noinline__ int run_pool64(const Seg64 &a, const StepConst &c, const
             a.p.vy[i] = vy;
             a.p.vz[i] = vz;
             a.p.tet[i] = tet;
-        } else if (!have_field) {
-            h = load_push(a.m.rec, tet);
         }
     }
     __syncwarp();
