@@ -489,10 +489,16 @@ cudaLaunchConfig_t config_of(const ResidentPlan &p, cudaLaunchAttribute *attr, c
     return cfg;
 }
 
-// Whether the device runs this plan (opt-in shared memory, cluster size, all blocks resident).
-bool fits(const ResidentPlan &p, int sms) {
+// Whether the device runs this plan (opt-in shared memory, cluster size, all
+// blocks resident). A kernel's limit of dynamic shared memory is one value per
+// device that all its plans share, and plans outlive this call: it is set to all
+// that the kernel's own arrays leave of the opt-in size, whatever this plan needs.
+bool fits(const ResidentPlan &p, int sms, int optin) {
     const Kernel k = kernel_of(p);
-    if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(p.smem)) != cudaSuccess ||
+    cudaFuncAttributes fa;
+    if (cudaFuncGetAttributes(&fa, k) != cudaSuccess || p.smem + fa.sharedSizeBytes > size_t(optin) ||
+        cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - int(fa.sharedSizeBytes)) !=
+            cudaSuccess ||
         (p.cluster &&
          cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess)) {
         cudaGetLastError();
@@ -526,7 +532,7 @@ ResidentPlan resident_plan(int64_t n) {
         const int64_t room = int64_t(optin) - 4096 - int64_t(smem_of(threads, 0, cluster));
         p.staged = int(std::min<int64_t>(32, std::max<int64_t>(0, room / (12 * int64_t(threads)))));
         p.smem = smem_of(threads, p.staged, cluster);
-        return fits(p, sms);
+        return fits(p, sms, optin);
     };
     if (n <= kClusterRows) {
         const int threads = int(std::max<int64_t>(64, ((n + kMaxCluster - 1) / kMaxCluster + 31) / 32 * 32));
