@@ -221,7 +221,10 @@ struct spg_handle {
     std::vector<DevParticles> ckpt;   // particle state at steps 0, ce, 2 ce, ...
     int32_t grad_steps = 0, grad_every = 0;
     int64_t grad_step0 = 0;
+    // landings and adjoints in the slots of the forward pass, and the particles'
+    // id words there: later steps may re-sort the live arrays
     LandRec *land = nullptr;
+    uint32_t *grad_idf = nullptr;
     double *gr = nullptr, *adj_x = nullptr, *adj_v = nullptr, *gE = nullptr, *lam = nullptr, *mu = nullptr,
            *dJdg = nullptr, *sums = nullptr;
     bool grad_whole = false;     // hist64 holds every step of the last forward pass
@@ -1797,7 +1800,7 @@ int spg_destroy(spg_handle *h) {
                     h->stag,     h->sref,
                     h->rec32,    h->cen,      h->cen_lo,   h->sval32,   h->inv_diag32, h->e32,     h->r32,       h->z32,
                     h->p32,      h->q32,      h->partials32, h->sc32,
-                    h->elim_rp,  h->elim_row, h->elim_col, h->elim_val, h->land, h->gr, h->adj_x, h->adj_v,
+                    h->elim_rp,  h->elim_row, h->elim_col, h->elim_val, h->land, h->grad_idf, h->gr, h->adj_x, h->adj_v,
                     h->gE,       h->lam,      h->mu,       h->dJdg,    h->sums, h->hist64, h->hist.tet, h->hist.vx,
                     h->hist.vy,  h->hist.vz,  h->tri_scratch, h->ctr_scratch,
                     h->q,        h->partials, h->sc,       h->tri_count, h->ctr,      h->n_alive_dev, h->sort_scratch, h->walkq_n,
@@ -2867,12 +2870,15 @@ int spg_grad_forward(spg_handle *h, int32_t nsteps, int32_t checkpoint_every, co
         h->ckpt_cap = std::max<int64_t>(n, 1);
     }
     if (n > h->land_cap) {
-        for (void *q : {(void *)h->land, (void *)h->gr, (void *)h->adj_x, (void *)h->adj_v}) cudaFree(q);
+        for (void *q : {(void *)h->land, (void *)h->grad_idf, (void *)h->gr, (void *)h->adj_x, (void *)h->adj_v})
+            cudaFree(q);
         h->land = nullptr;
+        h->grad_idf = nullptr;
         h->gr = h->adj_x = h->adj_v = nullptr;
         h->land_cap = 0;
         const int64_t m = std::max<int64_t>(n, 1);
         CK(dalloc(&h->land, m));
+        CK(dalloc(&h->grad_idf, m));
         CK(dalloc(&h->gr, 3 * m));
         CK(dalloc(&h->adj_x, 3 * m));
         CK(dalloc(&h->adj_v, 3 * m));
@@ -2884,6 +2890,9 @@ int spg_grad_forward(spg_handle *h, int32_t nsteps, int32_t checkpoint_every, co
         (rc = ensure(h, &h->ctr_scratch, 1)))
         return rc;
     CK(cudaMemsetAsync(h->land, 0xff, sizeof(LandRec) * std::max<int64_t>(n, 1), h->stream));
+    if (n > 0)
+        CK(cudaMemcpyAsync(h->grad_idf, h->mixed ? h->Q[h->cur].idf : h->P[h->cur].idf, sizeof(uint32_t) * size_t(n),
+                           cudaMemcpyDeviceToDevice, h->stream));
     h->grad_steps = nsteps;
     h->grad_every = checkpoint_every;
     h->grad_step0 = h->step;
@@ -2983,7 +2992,7 @@ int spg_grad_backward(spg_handle *h, double *dJ_dg, double *dJ_dx0, double *dJ_d
     if (h->grad_whole) {  // the forward's own record of every step
         StepConst c = step_const(h);
         c.step = h->grad_step0;
-        launch_backward(h->P[h->cur], n, h->hist64, 0, h->grad_steps, h->rec, h->land, h->gr, h->grad_inv_n, h->adj_x,
+        launch_backward(h->grad_idf, n, h->hist64, 0, h->grad_steps, h->rec, h->land, h->gr, h->grad_inv_n, h->adj_x,
                         h->adj_v, h->gE, c, s, G);
         CK(cudaGetLastError());
     }
@@ -3016,8 +3025,8 @@ int spg_grad_backward(spg_handle *h, double *dJ_dg, double *dJ_dx0, double *dJ_d
             launch_backward32(work32, n, mesh_dev32(h), h->hist, k0, k1, h->land, h->gr, h->grad_inv_n, h->adj_x,
                               h->adj_v, h->gE, c, s, G);
         else
-            launch_backward(work, n, h->hist64, k0, k1, h->rec, h->land, h->gr, h->grad_inv_n, h->adj_x, h->adj_v,
-                            h->gE, c, s, G);
+            launch_backward(h->grad_idf, n, h->hist64, k0, k1, h->rec, h->land, h->gr, h->grad_inv_n, h->adj_x,
+                            h->adj_v, h->gE, c, s, G);
         CK(cudaGetLastError());
     }
     // the results' pages while the GPU runs the windows
@@ -3049,10 +3058,7 @@ int spg_grad_backward(spg_handle *h, double *dJ_dg, double *dJ_dx0, double *dJ_d
         double *dv = dx + 3 * n;
         if (!dJ_dx0) dx = nullptr;
         if (!dJ_dv0) dv = nullptr;
-        if (h->mixed)
-            launch_gather_adj32(h->Q[h->cur], n, h->adj_x, h->adj_v, dx, dv, s);
-        else
-            launch_gather_adj(h->P[h->cur], n, h->adj_x, h->adj_v, dx, dv, s);
+        launch_gather_adj(h->grad_idf, n, h->adj_x, h->adj_v, dx, dv, s);
         if (dJ_dx0) CK(cudaMemcpyAsync(dJ_dx0, dx, sizeof(double) * 3 * n, cudaMemcpyDeviceToHost, s));
         if (dJ_dv0) CK(cudaMemcpyAsync(dJ_dv0, dv, sizeof(double) * 3 * n, cudaMemcpyDeviceToHost, s));
         CK(cudaStreamSynchronize(s));

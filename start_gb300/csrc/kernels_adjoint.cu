@@ -108,7 +108,7 @@ __device__ __forceinline__ float reach(double v, double h) {
 // (FP64 pipe 78 % active; the rest of its instructions are the tet changes and
 // collisions of single lanes). The next step's record is
 // loaded before the current one is used.
-__global__ void __launch_bounds__(128) k_backward(const DevParticles p, int64_t n, const HistRec *__restrict__ h, int k0, int k1,
+__global__ void __launch_bounds__(128) k_backward(const uint32_t *__restrict__ idf, int64_t n, const HistRec *__restrict__ h, int k0, int k1,
                                                   const TetRec *__restrict__ rec, const LandRec *__restrict__ land,
                                                   const double *__restrict__ gr, double gscale, double *__restrict__ ax,
                                                   double *__restrict__ av, double *__restrict__ gE,
@@ -120,7 +120,7 @@ __global__ void __launch_bounds__(128) k_backward(const DevParticles p, int64_t 
     // c.step is the absolute step of k = 0; landing steps are absolute
     const int N = L.step < 0 ? -1 : int(int64_t(L.step) - c.step);
     if (N < k0) return;
-    const uint32_t id = p.idf[i] & kIdMask;
+    const uint32_t id = idf[i] & kIdMask;
     double Ax = ax[3 * i], Ay = ax[3 * i + 1], Az = ax[3 * i + 2];
     double Vx = av[3 * i], Vy = av[3 * i + 1], Vz = av[3 * i + 2];
     int run = -1;
@@ -360,11 +360,11 @@ __global__ void k_copy_alive(const DevParticles src, DevParticles dst, int64_t n
     dst.tet[i] = src.tet[i];
 }
 
-__global__ void k_gather_adj(const DevParticles p, int64_t n, const double *__restrict__ ax,
+__global__ void k_gather_adj(const uint32_t *__restrict__ idf, int64_t n, const double *__restrict__ ax,
                              const double *__restrict__ av, double *dx, double *dv) {
     const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    const int64_t id = p.idf[i] & kIdMask;
+    const int64_t id = idf[i] & kIdMask;
     for (int k = 0; k < 3; ++k) {
         if (dx) dx[3 * id + k] = ax[3 * i + k];
         if (dv) dv[3 * id + k] = av[3 * i + k];
@@ -385,11 +385,11 @@ void launch_objective(const DevParticles &p, int64_t n, const LandRec *land, con
         k_objective<<<grid_for(n, 256), 256, 0, s>>>(p, n, land, target[0], target[1], target[2],
                                                       1.0 / (2.0 * sigma * sigma), gr, sums);
 }
-void launch_backward(const DevParticles &p, int64_t n, const HistRec *h, int k0, int k1, const TetRec *rec,
+void launch_backward(const uint32_t *idf, int64_t n, const HistRec *h, int k0, int k1, const TetRec *rec,
                      const LandRec *land, const double *gr, double gscale, double *ax, double *av, double *gE,
                      const StepConst &c, cudaStream_t s, const double *G) {
     if (n > 0)
-        k_backward<<<grid_for(n, 128), 128, 0, s>>>(p, n, h, k0, k1, rec, land, gr, gscale, ax, av, gE, c,
+        k_backward<<<grid_for(n, 128), 128, 0, s>>>(idf, n, h, k0, k1, rec, land, gr, gscale, ax, av, gE, c,
                                                      c.charge / c.mass * c.dt, G);
 }
 void launch_gE_to_nodes(const int4 *tet_nodes, const TetRec *rec, const double *gE, double cq, int64_t nt, double *lam,
@@ -412,9 +412,9 @@ void launch_set_dirichlet(const uint8_t *is_dir, const double *g, double *dir_va
                           cudaStream_t s) {
     k_set_dirichlet<<<grid_for(nn, 256), 256, 0, s>>>(is_dir, g, dir_value, phi, nn);
 }
-void launch_gather_adj(const DevParticles &p, int64_t n, const double *ax, const double *av, double *dx, double *dv,
+void launch_gather_adj(const uint32_t *idf, int64_t n, const double *ax, const double *av, double *dx, double *dv,
                        cudaStream_t s) {
-    if (n > 0) k_gather_adj<<<grid_for(n, 256), 256, 0, s>>>(p, n, ax, av, dx, dv);
+    if (n > 0) k_gather_adj<<<grid_for(n, 256), 256, 0, s>>>(idf, n, ax, av, dx, dv);
 }
 
 void launch_field_gradient(const int4 *tet_nodes, const TetRec *rec, const double *E, int64_t nt, int64_t nn,

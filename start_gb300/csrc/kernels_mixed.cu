@@ -1129,17 +1129,6 @@ __global__ void k_copy_alive32(DevParticles32 src, DevParticles32 dst, int64_t n
     dst.tet[i] = src.tet[i];
 }
 
-__global__ void k_gather_adj32(DevParticles32 p, int64_t n, const double *__restrict__ ax,
-                               const double *__restrict__ av, double *dx, double *dv) {
-    const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const int64_t id = p.idf[i] & kIdMask;
-    for (int k = 0; k < 3; ++k) {
-        if (dx) dx[3 * id + k] = ax[3 * i + k];
-        if (dv) dv[3 * id + k] = av[3 * i + k];
-    }
-}
-
 MixedArgs make_args(const DevParticles32 &p, int64_t n, const MeshDev32 &m) {
     MixedArgs a;
     a.p = p;
@@ -1224,11 +1213,6 @@ void launch_backward32(const DevParticles32 &p, int64_t n, const MeshDev32 &m, c
     if (n > 0)
         k_backward32<<<grid_for(n, 128), 128, 0, s>>>(make_args(p, n, m), h, k0, k1, land, gr, gscale, ax, av, gE, c,
                                                        c.charge / c.mass * c.dt, G);
-}
-
-void launch_gather_adj32(const DevParticles32 &p, int64_t n, const double *ax, const double *av, double *dx,
-                         double *dv, cudaStream_t s) {
-    if (n > 0) k_gather_adj32<<<grid_for(n, 256), 256, 0, s>>>(p, n, ax, av, dx, dv);
 }
 
 void launch_field32_full(const FieldArgs &f, int64_t n_tets, cudaStream_t s) {

@@ -188,10 +188,10 @@ struct AdjHist {
 void launch_copy_alive(const DevParticles &src, const DevParticles &dst, int64_t n, cudaStream_t s);
 void launch_objective(const DevParticles &p, int64_t n, const LandRec *land, const double *target, double sigma,
                       double *gr, double *sums, cudaStream_t s);
-// G (nullable): per-tet gradient of the recovered field (launch_field_gradient);
-// with it the position adjoint also carries the push's dependence on the
-// particle's position.
-void launch_backward(const DevParticles &p, int64_t n, const HistRec *h, int k0, int k1, const TetRec *rec,
+// idf: the particles' id words in the slots of the record. G (nullable): per-tet
+// gradient of the recovered field (launch_field_gradient); with it the position
+// adjoint also carries the push's dependence on the particle's position.
+void launch_backward(const uint32_t *idf, int64_t n, const HistRec *h, int k0, int k1, const TetRec *rec,
                      const LandRec *land, const double *gr, double gscale, double *ax, double *av, double *gE,
                      const StepConst &c, cudaStream_t s, const double *G = nullptr);
 // G[9 t + 3 d + c] = dE_d/dx_c of the continuous field whose nodal values are
@@ -209,7 +209,8 @@ void launch_lift(const int64_t *erp, const int32_t *ec, const double *ev, const 
                  cudaStream_t s);
 void launch_set_dirichlet(const uint8_t *is_dir, const double *g, double *dir_value, double *phi, int64_t nn,
                           cudaStream_t s);
-void launch_gather_adj(const DevParticles &p, int64_t n, const double *ax, const double *av, double *dx, double *dv,
+// The particles' adjoints in id order (both forms).
+void launch_gather_adj(const uint32_t *idf, int64_t n, const double *ax, const double *av, double *dx, double *dv,
                        cudaStream_t s);
 
 struct FieldArgs;
@@ -358,8 +359,6 @@ void launch_objective32(const DevParticles32 &p, int64_t n, const MeshDev32 &m, 
 void launch_backward32(const DevParticles32 &p, int64_t n, const MeshDev32 &m, const AdjHist &h, int k0, int k1,
                        const LandRec *land, const double *gr, double gscale, double *ax, double *av, double *gE,
                        const StepConst &c, cudaStream_t s, const double *G = nullptr);
-void launch_gather_adj32(const DevParticles32 &p, int64_t n, const double *ax, const double *av, double *dx,
-                         double *dv, cudaStream_t s);
 void launch_deposit32(const DevParticles32 &p, int64_t n, const MeshDev32 &m, int k, unsigned long long *node_fix,
                       const OccList &occ, cudaStream_t s);
 void launch_to_local(const double *pos, const double *vel, const int32_t *tet, const double *cen, int64_t n,
