@@ -338,7 +338,9 @@ int spg_set_dirichlet(spg_handle *h, const double *g);
  * push, move and frozen collisions, one adjoint CG on the stiffness matrix,
  * and returns dJ/dg at the Dirichlet nodes (0 elsewhere) and, if non-NULL,
  * dJ/d(initial position) and dJ/d(initial velocity) per particle [3n, id order].
- * N is held constant. Tet crossings are piecewise constant and carry no gradient. */
+ * N is held constant. Tet crossings are piecewise constant and carry no gradient.
+ * Steps and re-sorts between the two passes do not matter; after a particle set
+ * of another size, or injected particles, spg_grad_backward returns SPG_E_STATE. */
 int spg_grad_forward(spg_handle *h, int32_t nsteps, int32_t checkpoint_every, const double target[3], double sigma,
                      double *J, int64_t *n_landed);
 int spg_grad_backward(spg_handle *h, double *dJ_dg, double *dJ_dx0, double *dJ_dv0, int32_t *adj_cg_iters);

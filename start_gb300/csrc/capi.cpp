@@ -220,6 +220,7 @@ struct spg_handle {
     // gradient state (spg_grad_forward / spg_grad_backward)
     std::vector<DevParticles> ckpt;   // particle state at steps 0, ce, 2 ce, ...
     int32_t grad_steps = 0, grad_every = 0;
+    int64_t grad_n = 0;          // particles of the last forward pass
     int64_t grad_step0 = 0;
     // landings and adjoints in the slots of the forward pass, and the particles'
     // id words there: later steps may re-sort the live arrays
@@ -2893,6 +2894,7 @@ int spg_grad_forward(spg_handle *h, int32_t nsteps, int32_t checkpoint_every, co
     if (n > 0)
         CK(cudaMemcpyAsync(h->grad_idf, h->mixed ? h->Q[h->cur].idf : h->P[h->cur].idf, sizeof(uint32_t) * size_t(n),
                            cudaMemcpyDeviceToDevice, h->stream));
+    h->grad_n = n;
     h->grad_steps = nsteps;
     h->grad_every = checkpoint_every;
     h->grad_step0 = h->step;
@@ -2939,6 +2941,9 @@ int spg_grad_forward(spg_handle *h, int32_t nsteps, int32_t checkpoint_every, co
 int spg_grad_backward(spg_handle *h, double *dJ_dg, double *dJ_dx0, double *dJ_dv0, int32_t *adj_iters) {
     if (!h || !dJ_dg) return fail(h, SPG_E_INVALID, "grad_backward: dJ_dg is required");
     if (!h->grad_ready) return fail(h, SPG_E_STATE, "grad_backward: run spg_grad_forward first (with landings)");
+    // landings, records and the caller's results are sized for those particles
+    if (h->np != h->grad_n)
+        return fail(h, SPG_E_STATE, "grad_backward: the number of particles changed since spg_grad_forward");
     CK(cudaSetDevice(h->device));
     const int64_t n = h->np;
     const int W = h->grad_every;
