@@ -383,7 +383,8 @@ int spg_profile_reset(spg_handle *h);
  *                        matrix is not SPD, or the data hold NaN); the
  *                        message says which; x keeps the last iterate.
  *   SPG_E_INVALID        bad sizes or null arrays, or a row with no stored
- *                        diagonal entry or a zero or non-finite one.
+ *                        diagonal entry or a zero or non-finite one (of
+ *                        several, the last one stored; A has their sum).
  * stream is a cudaStream_t, or NULL for the default stream.
  *
  * Limit: n <= 131072 rows. Larger n returns SPG_E_INVALID without touching

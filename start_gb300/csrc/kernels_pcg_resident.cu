@@ -281,7 +281,7 @@ __global__ void __launch_bounds__(TMAX, 1) k_pcg_resident(const __grid_constant_
     // ---- r = b - A x, z = D^-1 r. The row's couplings to other rows go to
     // shared memory while they fit (entries from `next` on are read again in
     // every iteration); exact zeros are left out, the diagonal stays apart.
-    double x = 0.0, r = 0.0, z = 0.0, p = 0.0, dinv = 1.0, diag = 0.0;
+    double x = 0.0, r = 0.0, z = 0.0, p = 0.0, dinv = 1.0, diag = 0.0, last = 0.0;
     int staged = 0, next = row.count;
     double rz0 = 0.0, bb0 = 0.0, rr0 = 0.0, bad = 0.0;
     if (act) {
@@ -292,6 +292,7 @@ __global__ void __launch_bounds__(TMAX, 1) k_pcg_resident(const __grid_constant_
             const double m = __ldg(a.val + row.at(k));
             if (c == i) {
                 diag += m;
+                last = m;
                 found = true;
             } else if (m != 0.0) {
                 if (staged < a.staged) {
@@ -311,8 +312,9 @@ __global__ void __launch_bounds__(TMAX, 1) k_pcg_resident(const __grid_constant_
         if (a.inv_diag) {
             dinv = __ldg(a.inv_diag + i);
         } else {
-            if (!found || !(fabs(diag) > 0.0) || !isfinite(diag)) bad = 1.0;
-            dinv = bad != 0.0 ? 1.0 : 1.0 / diag;
+            // (of several entries on the diagonal, the last one, as in k_na_setup)
+            if (!found || !(fabs(last) > 0.0) || !isfinite(last)) bad = 1.0;
+            dinv = bad != 0.0 ? 1.0 : 1.0 / last;
         }
         x = a.x[i];
         const double b = a.b[i];
