@@ -26,20 +26,21 @@
 //   * cluster: up to 16 blocks in one cluster, the records in distributed shared
 //     memory, the hardware barrier (400 to 600 cycles). Its 16 SMs issue few
 //     FP64 operations, so it ends where the grid becomes faster, at 4,096 rows:
-//     us an iteration, cluster / grid, 1,331 rows 4.1 / 5.3, 3,375 4.9 / 5.3,
-//     4,096 5.2 / 5.3, 4,913 5.8 / 5.4.
+//     us an iteration, cluster / grid, 1,331 rows 4.2 / 5.5, 3,375 5.0 / 5.4,
+//     4,096 5.5 / 5.5, 4,913 6.0 / 5.4.
 //   * grid: up to one block per SM, cooperative launch, the records in L2, a counter
 //     in global memory as the barrier (1.2 us). It ends at one row per thread,
 //     155,648 rows on 152 SMs.
 // Measured per iteration of the lattice Laplacian: three kernels per iteration in
 // a graph; one launch with two exchanges per iteration ({z, p} published); one
-// exchange: 1,331 rows 22, 4.4, 4.1 us; 5,832 rows -, 6.0, 5.2; 17,576 rows 22, 7.0,
-// 5.6; 68,921 rows -, 9.1, 8.8; 132,651 rows 24, 12.4, 13.5 (there the FP64 pipe is
+// exchange: 1,331 rows 22, 4.4, 4.2 us; 5,832 rows -, 6.0, 5.3; 17,576 rows 22, 7.0,
+// 5.6; 68,921 rows -, 9.1, 8.9; 132,651 rows 24, 12.4, 13.6 (there the FP64 pipe is
 // full and the gathers' second multiply-add costs what the exchange saves).
 #include <algorithm>
 #include <cmath>
 #include <cstdint>
 
+#include "newton_div.h"
 #include "pcg_resident.h"
 #include "spg_internal.h"
 
@@ -55,26 +56,12 @@ constexpr int kMaxCluster = 16;
 // resident, so the limit is never met in a healthy run.
 constexpr int kMaxPolls = 1 << 22;
 
-// Quotients on the critical path of every iteration, without the 1,470 cycles
-// of the division sequence: reciprocal() is a seed and one third-order Newton
-// step (y' = y + y (h + h^2), h = 1 - b y); quotient() corrects a y with its
-// exact remainder. Operands whose steps could leave the normal range take the
-// division, out of line so that it is not computed beside the fast form.
-__device__ __forceinline__ double reciprocal(double b) {
-    double y;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
-    const double h = fma(-b, y, 1.0);
-    return fma(y, fma(h, h, h), y);
-}
-__device__ __forceinline__ bool mid_range(double a) {
-    const int e = (__double2hiint(a) >> 20) & 0x7ff;
-    return e >= 300 && e <= 1700;
-}
+// Quotients on the critical path of every iteration (newton_div.h); operands
+// beyond its range take the division, out of line so that it is not computed
+// beside the fast form.
 __device__ __noinline__ double divide(double a, double b) { return a / b; }
 __device__ __forceinline__ double quotient(double a, double b, double y) {
-    if (!(mid_range(a) && mid_range(b))) return divide(a, b);
-    const double q = a * y;
-    return fma(fma(-b, q, a), y, q);
+    return newton_range(a) && newton_range(b) ? newton_quotient(a, b, y) : divide(a, b);
 }
 
 // Row access of the two matrix formats: entry k of the row is col[at(k)],
@@ -414,7 +401,7 @@ __global__ void __launch_bounds__(TMAX, 1) k_pcg_resident(const __grid_constant_
                             : iters > 0 && iters >= a.max_iter ? 2
                             : positive(pq)            ? 0
                                                       : kPcgBreakdown;
-            const double y = reciprocal((t & 1) ? rz : pq);  // both at once
+            const double y = newton_reciprocal((t & 1) ? rz : pq);  // both at once
             const double y0 = __shfl_sync(kFull, y, 0), y1 = __shfl_sync(kFull, y, 1);
             alpha = why ? 0.0 : quotient(rz, pq, y0);
             const double next_rz = fma(alpha * alpha, s.tot[2], fma(-2.0 * alpha, s.tot[1], rz));
