@@ -331,9 +331,10 @@ int spg_set_dirichlet(spg_handle *h, const double *g);
  * (no deposit or solve), keeping the particle state every checkpoint_every
  * steps and where each particle lands, and returns
  *   J = (1/N) sum over the N particles that landed of exp(-|r - target|^2 / (2 sigma^2)).
- * (FP64 form: where 32 bytes per particle and step fit into 32 GB and a quarter
- * of the free device memory, it records every step instead and takes no
- * checkpoints; the record stays with the handle until it is destroyed).
+ * (FP64 form: where 32 bytes per particle and step fit into the limit of
+ * spg_set_grad_record, 32 GB by default, and a quarter of the free device memory,
+ * it records every step instead and takes no checkpoints; the record stays with
+ * the handle).
  * spg_grad_backward reads the record or recomputes each checkpoint window, runs the adjoint of
  * push, move and frozen collisions, one adjoint CG on the stiffness matrix,
  * and returns dJ/dg at the Dirichlet nodes (0 elsewhere) and, if non-NULL,
@@ -344,6 +345,11 @@ int spg_set_dirichlet(spg_handle *h, const double *g);
 int spg_grad_forward(spg_handle *h, int32_t nsteps, int32_t checkpoint_every, const double target[3], double sigma,
                      double *J, int64_t *n_landed);
 int spg_grad_backward(spg_handle *h, double *dJ_dg, double *dJ_dx0, double *dJ_dv0, int32_t *adj_cg_iters);
+/* No counterpart in the reference (an execution choice, not a result). Largest
+ * record of every step that spg_grad_forward may keep, in bytes; 0: checkpoints
+ * and windows always. A kept record above the limit is given back at once, and a
+ * backward pass that would read it needs another forward pass (SPG_E_STATE). */
+int spg_set_grad_record(spg_handle *h, size_t max_bytes);
 /* No counterpart in the reference. on != 0: spg_grad_backward also carries the
  * push's dependence on the particle's position, through the gradient of a
  * continuous field recovered from the per-tet E (nodal volume averages,

@@ -230,6 +230,7 @@ struct spg_handle {
            *dJdg = nullptr, *sums = nullptr;
     bool grad_whole = false;     // hist64 holds every step of the last forward pass
     HistRec *hist64 = nullptr;           // FP64 form
+    size_t hist_limit = size_t(32) << 30;  // bytes of a whole record (spg_set_grad_record)
     AdjHist hist{};                      // mixed form
     unsigned int *tri_scratch = nullptr;
     DevCounters *ctr_scratch = nullptr;
@@ -2799,6 +2800,18 @@ int spg_set_step_segments(spg_handle *h, int32_t max_steps) {
     return SPG_OK;
 }
 
+int spg_set_grad_record(spg_handle *h, size_t max_bytes) {
+    if (!h) return SPG_E_INVALID;
+    CK(cudaSetDevice(h->device));
+    h->hist_limit = max_bytes;
+    if (!h->hist64 || sizeof(HistRec) * size_t(h->hist_cap) <= max_bytes) return SPG_OK;
+    cudaFree(h->hist64);
+    h->hist64 = nullptr;
+    h->hist_cap = 0;
+    if (h->grad_whole) h->grad_ready = false;
+    return SPG_OK;
+}
+
 int spg_grad_field_gradient(spg_handle *h, int32_t on) {
     if (!h) return SPG_E_INVALID;
     h->grad_fg = on != 0;
@@ -2810,20 +2823,21 @@ int spg_grad_field_gradient(spg_handle *h, int32_t on) {
 namespace {
 // Whether the forward pass records every step (32 bytes per particle and step,
 // and room for the results behind them) for the backward pass, in the record
-// kept or a new one of at most 32 GB and a quarter of the free memory. Else, and in the
-// mixed form, it keeps checkpoints and the backward pass repeats the steps of
+// kept or a new one of at most hist_limit bytes and a quarter of the free memory. Else,
+// and in the mixed form, it keeps checkpoints and the backward pass repeats the steps of
 // each window: 1e6 particles, 300 steps take 9.7 GB and 13.4 -> 9.05 ms for
 // forward and backward together; the record of a step adds 6 % to it.
 bool whole_history(spg_handle *h, int64_t steps, int64_t n) {
     if (h->mixed || n < 1) return false;
     const int64_t need = (steps + 2) * n;
+    if (size_t(need) > h->hist_limit / sizeof(HistRec)) return false;
     if (need <= h->hist_cap) return true;
     size_t free = 0, total = 0;
     if (cudaMemGetInfo(&free, &total) != cudaSuccess) {
         cudaGetLastError();
         return false;
     }
-    const size_t room = std::min<size_t>((free + sizeof(HistRec) * size_t(h->hist_cap)) / 4, size_t(32) << 30);
+    const size_t room = (free + sizeof(HistRec) * size_t(h->hist_cap)) / 4;
     if (size_t(need) > room / sizeof(HistRec)) return false;
     cudaFree(h->hist64);
     h->hist64 = nullptr;

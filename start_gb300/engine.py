@@ -356,6 +356,11 @@ class StartPIC:
                                                N.as_ptr(dv, C.c_double) if particles else None, C.byref(it)))
         return g, dx, dv, it.value
 
+    def set_grad_record(self, max_bytes):
+        """Largest record of every step that grad_forward may keep (0: checkpoints
+        and windows always); a larger one is given back (spg_set_grad_record)."""
+        self._check(self.lib.spg_set_grad_record(self.h, int(max_bytes)))
+
     def grad_field_gradient(self, on=True):
         """Whether grad_backward also carries the push's dependence on the
         position through the recovered field's gradient (spg_grad_field_gradient)."""
