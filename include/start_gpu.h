@@ -285,7 +285,10 @@ int spg_process(spg_handle *h, int32_t nsteps, spg_stats *stats);
  * reference's loop does: src/FiniteElementMethod/Solvers/
  * MatrixEquationSolver.cpp:405-412 logs the failure and returns). */
 int spg_run(spg_handle *h, int32_t nsteps, spg_stats *stats);
-/* Re-sorts particles by tet now (settled/lost particles move to the end). */
+/* Re-sorts particles by tet now (settled/lost particles move to the end). The
+ * first sort of a set of 65,536 particles or more takes 64 bytes a particle of
+ * device memory in the FP64 form (where they are free), which stay with the
+ * particle arrays for the next set. */
 int spg_resort(spg_handle *h);
 /* No counterpart in the reference (an execution choice, not a result).
  * spg_run and spg_process run the steps between two events of the loop (a

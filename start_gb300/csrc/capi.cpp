@@ -169,7 +169,7 @@ struct spg_handle {
     int64_t cap = 0, np = 0, n_active = 0, init_lost = 0;
     unsigned int *tri_count = nullptr;
     DevCounters *ctr = nullptr;
-    WalkItem *walkq = nullptr;       // mixed form's walk queue, capacity cap (particles)
+    WalkItem *walkq = nullptr;       // mixed form: walk queue, or records of a re-sort, capacity cap (particles)
     unsigned int *walkq_n = nullptr;
     // segmented steps: at most seg_max steps per segment (1: one launch per
     // step)
@@ -186,7 +186,7 @@ struct spg_handle {
     bool ats = false;
     int32_t *id_slot = nullptr;  // slot of each id for direct downloads; ranks during a re-sort
     int64_t id_slot_cap = 0;
-    void *sort_rec = nullptr;    // records of a re-sort from no order
+    void *sort_rec = nullptr;    // records of a re-sort from no order (FP64 form)
     size_t sort_rec_bytes = 0;
     bool sorted = false;         // the particles have been re-sorted since they were set
     unsigned long long *io_counter = nullptr;
@@ -840,10 +840,18 @@ int id_words(spg_handle *h, int64_t n) {
 // The records and ranks for a re-sort of a set in no order; nullptr: histogram
 // and scatter. Below 65,536 particles the arrays stay in L2 and the route's
 // other kernel costs more (70,000: 17.6 against 18.7 us, 20,000: 15). Without
-// room for them the sort scatters.
+// room for them the sort scatters. The mixed form's records take the memory of
+// its walk queue, which only the gradient's steps use; the FP64 form's own
+// (64 bytes a particle) go with the particle arrays.
 void *sort_records(spg_handle *h) {
     if (h->sorted || h->n_active < 65536) return nullptr;
-    const size_t need = size_t(h->n_active) * (h->mixed ? 32 : 64);
+    static_assert(sizeof(WalkItem) == 32, "a record of the mixed form");
+    if (h->mixed) {
+        if (id_words(h, h->np) == SPG_OK) return h->walkq;
+        cudaGetLastError();
+        return nullptr;
+    }
+    const size_t need = size_t(h->n_active) * 64;
     if (need > h->sort_rec_bytes) {
         cudaFree(h->sort_rec);
         h->sort_rec = nullptr;
