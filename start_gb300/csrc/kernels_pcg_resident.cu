@@ -446,14 +446,14 @@ __global__ void __launch_bounds__(TMAX, 1) k_pcg_resident(const __grid_constant_
     if constexpr (CLUSTER) cluster_barrier();  // no block leaves while its shared memory may be read
 }
 
-using Kernel = void (*)(ResidentArgs);
-Kernel kernel_of(const ResidentPlan &p) {
-    if (p.cluster) return k_pcg_resident<true, 384>;
-    return p.threads <= 512 ? k_pcg_resident<false, 512> : k_pcg_resident<false, 1024>;
-}
-
 // Rows up to which one cluster of 16 blocks is used.
 constexpr int64_t kClusterRows = 4096;
+
+using Kernel = void (*)(ResidentArgs);
+Kernel kernel_of(const ResidentPlan &p) {
+    if (p.cluster) return k_pcg_resident<true, int(kClusterRows) / kMaxCluster>;
+    return p.threads <= 512 ? k_pcg_resident<false, 512> : k_pcg_resident<false, 1024>;
+}
 
 size_t smem_of(int threads, int staged, bool cluster) {
     return size_t(threads) * ((cluster ? 2 * sizeof(ZpuRec) : 0) + 8 * kSums + 12 * size_t(staged));
