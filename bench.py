@@ -113,18 +113,18 @@ class ClockSampler:
 
 # dram__bytes_read.sum + dram__bytes_write.sum of one launch of the step kernel (a segment of up to
 # 32 steps, here seven) per alive particle, workload 1 geometry, one ncu capture at 4e6 particles
-# (FP64: 224.7 + 159.4 MB; mixed: 128.7 + 81.1 MB)
+# (FP64: 224.7 + 158.7 MB; mixed: 128.8 + 80.7 MB)
 STEP_TRAFFIC_B = {
-    "64": (384.1e6 / 4e6, "ncu capture of k_seg64 (seven steps) at 4e6 particles, scaled by particles"),
-    "32": (209.8e6 / 4e6, "ncu capture of k_seg32 (seven steps) at 4e6 particles, scaled by particles"),
+    "64": (383.4e6 / 4e6, "ncu capture of k_seg64 (seven steps) at 4e6 particles, scaled by particles"),
+    "32": (209.5e6 / 4e6, "ncu capture of k_seg32 (seven steps) at 4e6 particles, scaled by particles"),
 }
 # The resource that binds the step kernels is not HBM: the FP64 form's step is
 # FP64-issue-bound (GB300 issues about 2 FP64 thread-ops per clock per SM),
 # the mixed form's by instruction issue. From the same captures
 # (sm__pipe_fp64_cycles_active, smsp__issue_active, % of peak sustained active).
 STEP_BINDING = {
-    "64": {"resource": "fp64 pipe", "k_seg64": 0.736, "source": "ncu, k_seg64 at 4e6 particles"},
-    "32": {"resource": "instruction issue", "k_seg32_issue_active": 0.663, "k_seg32_active_lanes": 24.7,
+    "64": {"resource": "fp64 pipe", "k_seg64": 0.739, "source": "ncu, k_seg64 at 4e6 particles"},
+    "32": {"resource": "instruction issue", "k_seg32_issue_active": 0.657, "k_seg32_active_lanes": 24.7,
            "source": "ncu, k_seg32 at 4e6 particles"},
 }
 STEP_BYTES_NOTE = ("algorithmic bytes of one step per particle-step (the state read and written, the occupied tets' "
@@ -288,7 +288,9 @@ def grad_leg(args, local):
     """Gradient of the smoothed landing objective (the 100 mm electrode cube at
     h = 4 mm, 1e6 Ti+, 300 steps, argon 1 Pa HS with collision events frozen,
     checkpoints every 32 steps): cost of forward + backward against one plain
-    forward pass (set particles, electrode solve, 300 particle steps).
+    forward pass (set particles, electrode solve, 300 particle steps), with the
+    ions drawn on the host in every pass (cost_ratio: most of both times) and
+    from ions drawn beforehand (cost_ratio_given_ions).
 
     Two configurations: the one the gradient is timed on (top electrode at
     +500 V turning the ions back onto z = 0, target the centre of the bottom
@@ -307,13 +309,20 @@ def grad_leg(args, local):
     lp = LandingProblem(n_particles=args.grad_particles, steps=300, collisions=True)
     e = lp.engine
 
-    def plain_forward(Vx):
+    def start(Vx, ions):
         e.set_dirichlet(lp.dirichlet_values(Vx))
-        x0, v0, _, _ = lp.initial_state(a0)
-        e.set_particles(x0, v0)
+        e.set_particles(*(ions or lp.initial_state(a0)[:2]))
         e.solve(np.zeros(lp.mesh.n_nodes))
+
+    def plain_forward(Vx, ions=None):
+        start(Vx, ions)
         e.process(lp.steps)
         e.synchronize()
+
+    def gradient(Vx, ions):
+        start(Vx, ions)
+        e.grad_forward(lp.steps, lp.target, lp.sigma, lp.every)
+        e.grad_backward()
 
     def timed(f, reps=3):
         ts = []
@@ -338,10 +347,14 @@ def grad_leg(args, local):
             return {"electrodes_V": np.asarray(Vx).tolist(), "target": lp.target.tolist(), "J": J,
                     "n_landed": 0, "plain_forward_ms": t_plain, "grad_forward_ms": t_fwd}
         t_bwd, (dV, da, iters) = timed(lp.backward)
+        ions = lp.initial_state(a0)[:2]
+        t_plain_given, _ = timed(lambda: plain_forward(Vx, ions))
+        t_grad_given, _ = timed(lambda: gradient(Vx, ions))
         return {"electrodes_V": np.asarray(Vx).tolist(), "target": lp.target.tolist(), "J": J,
                 "n_landed": n_landed, "dJ_dV": dV.tolist(), "dJ_dalpha": da, "adjoint_cg_iters": iters,
                 "plain_forward_ms": t_plain, "grad_forward_ms": t_fwd, "backward_ms": t_bwd,
-                "cost_ratio": (t_fwd + t_bwd) / t_plain}
+                "cost_ratio": (t_fwd + t_bwd) / t_plain, "plain_forward_given_ions_ms": t_plain_given,
+                "gradient_given_ions_ms": t_grad_given, "cost_ratio_given_ions": t_grad_given / t_plain_given}
 
     out = {"workload": "cube100mm_h4mm_1e6ptcl_grad", "n_particles": int(args.grad_particles), "steps": 300,
            "checkpoint_every": lp.every, "half_angle_deg": 30.0, "sigma_m": lp.sigma,
@@ -351,7 +364,8 @@ def grad_leg(args, local):
     e.grad_field_gradient(True)
     fg = measure(V, (0.05, 0.05, 0.0))
     e.grad_field_gradient(False)
-    out["field_gradient"] = {k: fg[k] for k in ("dJ_dV", "dJ_dalpha", "grad_forward_ms", "backward_ms", "cost_ratio")}
+    out["field_gradient"] = {k: fg[k] for k in ("dJ_dV", "dJ_dalpha", "grad_forward_ms", "backward_ms", "cost_ratio",
+                                                "cost_ratio_given_ions")}
     if not args.no_grad_fd:
         grads = {"pathwise": (out["dJ_dV"], out["dJ_dalpha"]), "field_gradient": (fg["dJ_dV"], fg["dJ_dalpha"])}
         out["live_fd"] = live_fd_gaps(lp, V, a0, grads, ((1e-3, 1e-4), (1.0, 1e-2)))
