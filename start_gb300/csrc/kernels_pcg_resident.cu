@@ -26,14 +26,14 @@
 //   * cluster: up to 16 blocks in one cluster, the records in distributed shared
 //     memory, the hardware barrier (400 to 600 cycles). Its 16 SMs issue few
 //     FP64 operations, so it ends where the grid becomes faster, at 4,096 rows:
-//     us an iteration, cluster / grid, 1,331 rows 4.2 / 5.5, 3,375 5.0 / 5.4,
-//     4,096 5.5 / 5.5, 4,913 6.0 / 5.4.
+//     us an iteration, cluster / grid, 1,331 rows 4.1 / 5.1, 3,375 5.0 / 5.3,
+//     4,096 5.4 / 5.3, 4,913 5.9 / 5.4 (3 % between cards).
 //   * grid: up to one block per SM, cooperative launch, the records in L2, a counter
 //     in global memory as the barrier (1.2 us). It ends at one row per thread,
 //     155,648 rows on 152 SMs.
 // Measured per iteration of the lattice Laplacian: three kernels per iteration in
 // a graph; one launch with two exchanges per iteration ({z, p} published); one
-// exchange: 1,331 rows 22, 4.4, 4.2 us; 5,832 rows -, 6.0, 5.3; 17,576 rows 22, 7.0,
+// exchange: 1,331 rows 22, 4.4, 4.1 us; 5,832 rows -, 6.0, 5.2; 17,576 rows 22, 7.0,
 // 5.6; 68,921 rows -, 9.1, 8.9; 132,651 rows 24, 12.4, 13.6 (there the FP64 pipe is
 // full and the gathers' second multiply-add costs what the exchange saves).
 #include <algorithm>

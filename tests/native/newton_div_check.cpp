@@ -2,8 +2,9 @@
 // against the division: random operands of both signs over the whole accepted
 // range, quotients next to midpoints between doubles, powers of two and their
 // neighbours, both ends of the range, and values that must be turned away.
-// Prints the largest difference in ulp (of the reciprocal, of the quotient) and
-// the share of quotients that are not the rounded one.
+// Prints the largest relative error of the reciprocal, the largest difference of
+// the quotient in ulp, and of those that are not the rounded quotient the largest
+// distance, in ulp, of a / b from the midpoint between the two.
 #include <cstdio>
 #include <cstdlib>
 #include <initializer_list>
@@ -24,13 +25,23 @@ int main(int argc, char **argv) {
     std::mt19937_64 g(2025);
     std::uniform_real_distribution<double> u(0.0, 1.0);
     const double lo = std::ldexp(1.0, -423), hi = std::nextafter(std::ldexp(1.0, 424), 0.0);
-    long long worst_r = 0, worst_q = 0, off = 0, tested = 0, wrong_range = 0;
+    double worst_r = 0.0;
+    double from_mid = 0.0;
+    long long worst_q = 0, tested = 0, wrong_range = 0;
     auto check = [&](double a, double b) {
         const double y = spg::newton_reciprocal(b), q = spg::newton_quotient(a, b, y);
-        const long long dr = ulps(y, 1.0 / b), dq = ulps(q, a / b);
+        const double dr = std::fabs(std::fma(-b, y, 1.0));
+        const long long dq = ulps(q, a / b);
         worst_r = dr > worst_r ? dr : worst_r;
         worst_q = dq > worst_q ? dq : worst_q;
-        off += dq != 0;
+        if (dq == 1) {
+            // a/b lies next to the midpoint of q and c: the nearer to zero plus half an ulp.
+            // The remainder and its difference from b ulp / 2 are exact.
+            const double c = a / b, lo2 = std::fabs(q) < std::fabs(c) ? q : c;
+            const double ulp = (std::fabs(q) < std::fabs(c) ? c : q) - lo2;
+            const double d = std::fabs((std::fma(-b, lo2, a) - 0.5 * ulp * b) / (ulp * b));
+            from_mid = d > from_mid ? d : from_mid;
+        }
         ++tested;
         wrong_range += !spg::newton_range(a) || !spg::newton_range(b);
     };
@@ -58,6 +69,6 @@ int main(int argc, char **argv) {
     for (double v : {0.0, -0.0, inf, -inf, std::numeric_limits<double>::quiet_NaN(), std::nextafter(lo, 0.0),
                      std::nextafter(hi, inf), 5e-324, 2.2e-308, 1.7e308, -1.7e308})
         wrong_range += spg::newton_range(v);
-    std::printf("%lld %lld %lld %.3e %lld\n", tested, worst_r, worst_q, double(off) / double(tested), wrong_range);
+    std::printf("%lld %.3e %lld %.3e %lld\n", tested, worst_r, worst_q, from_mid, wrong_range);
     return 0;
 }
